@@ -225,3 +225,88 @@ def test_qwen3_next_engine_on_gpu_graphs_match_eager():
         torch.cuda.empty_cache()
     assert outs[0] == outs[1]
     assert all(len(t) == 12 for t in outs[0])
+
+
+def _gdn_f64(q, k, v, g, beta, lens, state, idx, has, l2norm=True):
+    qf, kf, vf = q.double(), k.double(), v.double()
+    if l2norm:
+        qf = qf * torch.rsqrt(qf.pow(2).sum(-1, keepdim=True) + 1e-6)
+        kf = kf * torch.rsqrt(kf.pow(2).sum(-1, keepdim=True) + 1e-6)
+    rep = v.shape[1] // q.shape[1]
+    qf, kf = qf.repeat_interleave(rep, 1) * 128 ** -0.5, kf.repeat_interleave(rep, 1)
+    out, state, t = torch.zeros_like(vf), state.double(), 0
+    for b, n in enumerate(lens):
+        S = state[idx[b]].clone() if has[b] else torch.zeros_like(state[0])
+        for t in range(t, t + n):
+            S = S * torch.exp(g[t].double())[:, None, None]
+            u = beta[t].double()[:, None] * (vf[t] - torch.einsum("hkv,hk->hv", S, kf[t]))
+            S = S + torch.einsum("hk,hv->hkv", kf[t], u)
+            out[t] = torch.einsum("hkv,hk->hv", S, qf[t])
+        t = t + 1 if n else t
+        if n:
+            state[idx[b]] = S
+    return out, state
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("lens", [(1, 1, 1), (4, 16, 1), (3, 0, 17), (33, 5, 64), (31, 2, 100)])
+@pytest.mark.parametrize("pitch", [0, 8, 3])               # rows behind one another, on 16 bytes, on 2 bytes only
+def test_gdn_groups_of_tokens(dtype, lens, pitch):
+    """Steps of one token and groups of four: sequences that end inside a group or a stage, empty ones, strided rows, strong decay.
+    Outputs are rounded once (half a unit of 2^-8 or 2^-11) behind sums of 128 fp32 products: fp32 state within 1e-5."""
+    from vllm_metax_b200.ops.gdn import gated_delta_rule
+
+    q, k, v, g, beta, qsl, state, idx, has = _gdn_case(dtype, seed=7, lens=lens)
+    g[::3] *= 60                                            # e^-30 in one token
+    want, s_want = _gdn_f64(q, k, v, g, beta, lens, state, idx, has)
+    wide = lambda x: torch.cat([x.flatten(1), x.new_zeros(x.shape[0], pitch)], 1).cuda()[:, : x[0].numel()].unflatten(1, x.shape[1:])
+    s_got = state.cuda()
+    got = gated_delta_rule(wide(q), wide(k), wide(v), g.cuda(), beta.cuda(), qsl.cuda(), s_got, idx.cuda(), has.cuda())
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    torch.testing.assert_close(got.cpu().double(), want, rtol=eps, atol=1e-5)
+    torch.testing.assert_close(s_got.cpu().double(), s_want, rtol=1e-5, atol=1e-5)
+
+
+@gpu
+def test_gdn_gates_and_norm_in_the_kernels():
+    """``ba`` of a projection instead of decays and betas, the grouped projection as the convolution's input, and the gated
+    norm of a view, against the same from plain tensors."""
+    from vllm_metax_b200.ops import gdn
+
+    gen = torch.Generator().manual_seed(3)
+    for lens in ((1, 1, 1), (40, 3, 9)):
+        T, nk, rep, d = sum(lens), 2, 2, 128
+        qkvz = torch.randn(T, nk * 6 * d, generator=gen).bfloat16().cuda()
+        ba = torch.randn(T, nk * 2 * rep, generator=gen).bfloat16().cuda()
+        a_log, dt = torch.rand(4, generator=gen).cuda(), torch.randn(4, generator=gen).cuda()
+        w = torch.randn(nk * 4 * d, 4, generator=gen).bfloat16().cuda()
+        qsl = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32).cuda()
+        idx, has = torch.tensor([2, 0, 3], dtype=torch.int32).cuda(), torch.tensor([1, 0, 1], dtype=torch.int32).cuda()
+        conv = torch.randn(4, 3, nk * 4 * d, generator=gen).bfloat16().cuda()
+        flat = torch.cat([t.flatten(1) for t in qkvz.view(T, nk, -1).split([d, d, rep * d, rep * d], -1)[:3]], -1)
+        c1, c2 = conv.clone(), conv.clone()
+        got = gdn.causal_conv1d(qkvz, w, None, c1, qsl, idx, has, heads=(nk, d, rep * d))
+        assert torch.equal(got, gdn.causal_conv1d(flat, w, None, c2, qsl, idx, has)) and torch.equal(c1, c2)
+        ref = gdn.causal_conv1d_ref(flat.cpu(), w.cpu(), None, conv.cpu().clone(), qsl.cpu(), idx.cpu(), has.cpu())
+        torch.testing.assert_close(got.cpu(), ref, rtol=2.0 ** -7, atol=1e-3)
+        q, k, v = (t.unflatten(1, (-1, d)) for t in got.split([nk * d, nk * d, nk * rep * d], -1))
+        b, a = ba.view(T, nk, 2 * rep).chunk(2, -1)
+        beta = torch.sigmoid(b.reshape(T, -1).float())
+        g = -torch.exp(a_log) * torch.nn.functional.softplus(a.reshape(T, -1).float() + dt)
+        s0 = torch.randn(4, 4, d, d, generator=gen).cuda() * 0.1
+        s1, s2 = s0.clone(), s0.clone()
+        o1 = gdn.gated_delta_rule_ba(q, k, v, ba, a_log, dt, qsl, s1, idx, has)
+        o2 = gdn.gated_delta_rule(q, k, v, g, beta, qsl, s2, idx, has)
+        torch.testing.assert_close(o1, o2, rtol=2.0 ** -7, atol=1e-5)
+        torch.testing.assert_close(s1, s2, rtol=1e-5, atol=1e-5)
+        z = qkvz.view(T, nk, -1)[..., 4 * d:]
+        nw = torch.randn(d, generator=gen).bfloat16().cuda()
+        y = gdn.gated_head_norm(o1.reshape(T, -1), z, nw, d, 1e-6)
+        n = o1.float() * torch.rsqrt(o1.float().pow(2).mean(-1, keepdim=True) + 1e-6) * nw.float()
+        want = n.bfloat16().float() * torch.nn.functional.silu(z.reshape(T, -1, d).float())
+        # the normed value may round to the next bf16 (2^-7 at most of it), the product rounds once more (2^-8)
+        torch.testing.assert_close(y.view(T, -1, d).float(), want, rtol=2.0 ** -7 + 2.0 ** -8, atol=1e-5)
+        y = gdn.gated_head_norm(o1.reshape(T, -1), z, None, d)
+        want = o1.float() * torch.sigmoid(z.reshape(T, -1, d).float())
+        torch.testing.assert_close(y.view(T, -1, d).float(), want, rtol=2.0 ** -7, atol=1e-6)

@@ -44,7 +44,7 @@ UNIT_SETS = {
 UNIT_GROUPS = {"gqa": ("gqa",), "hybrid": ("latent", "hybrid", "recurrent"), "parallel": ("gqa", "recurrent"),
                "streams": ("gqa", "latent", "streams")}
 # units that compute in true 32-bit (recurrences, norms, angles, fp32 products): no fast-math substitutions
-PRECISE_UNITS = ("channel_delta", "gemm_simt", "gla", "head_norm_rope", "latent_attn", "paged_attn_simt", "prenorm",
+PRECISE_UNITS = ("channel_delta", "gdn", "gemm_simt", "gla", "head_norm_rope", "latent_attn", "paged_attn_simt", "prenorm",
                  "residual_conv", "residual_norm", "rglru", "rope_angles", "stream_norm")
 
 NVCC_FLAGS = [

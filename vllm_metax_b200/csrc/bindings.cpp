@@ -644,27 +644,34 @@ void v4_gather_dequant(Tensor& dst, const Tensor& cache, const Tensor& slots, in
 }
 
 // q, k [T, Hq, 128], v [T, Hv, 128], g / beta f32 [T, Hv], state f32 [slots, Hv, 128, 128] (in / out)
-void gdn_recurrent(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g,
-                   const Tensor& beta, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
-                   const optional<Tensor>& has_initial, double scale, bool l2norm) {
+void gdn_run(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& query_start_loc,
+             const optional<Tensor>& state_idx, const optional<Tensor>& has_initial, double scale, bool l2norm,
+             b200::GdnParams& p) {
   TORCH_CHECK(q.dim() == 3 && k.dim() == 3 && v.dim() == 3 && q.stride(2) == 1 && k.stride(2) == 1 && v.stride(2) == 1);
   TORCH_CHECK(q.stride(1) == q.size(2) && k.stride(1) == k.size(2) && v.stride(1) == v.size(2) && k.sizes() == q.sizes());
   const int64_t T = q.size(0), hq = q.size(1), hv = v.size(1);
-  TORCH_CHECK(v.size(0) == T && out.is_contiguous() && out.sizes() == v.sizes() && out.scalar_type() == q.scalar_type());
-  TORCH_CHECK(g.is_contiguous() && beta.is_contiguous() && g.scalar_type() == at::kFloat && beta.scalar_type() == at::kFloat &&
-              g.numel() == T * hv && beta.numel() == T * hv);
+  TORCH_CHECK(v.size(0) == T && out.is_contiguous() && out.sizes() == v.sizes() && out.scalar_type() == q.scalar_type() &&
+              k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type());
   TORCH_CHECK(state.is_contiguous() && state.scalar_type() == at::kFloat && state.dim() == 4 && state.size(1) == hv);
   TORCH_CHECK(query_start_loc.scalar_type() == at::kInt && query_start_loc.is_contiguous());
   const int64_t B = query_start_loc.numel() - 1;
   if (state_idx.has_value()) TORCH_CHECK(state_idx->scalar_type() == at::kInt && state_idx->numel() >= B);
   if (has_initial.has_value()) TORCH_CHECK(has_initial->scalar_type() == at::kInt && has_initial->numel() >= B);
   const c10::cuda::CUDAGuard guard(q.device());
-  const int rc = b200::gdn_recurrent(out.data_ptr(), state.data_ptr<float>(), q.data_ptr(), k.data_ptr(), v.data_ptr(),
-                                     g.data_ptr<float>(), beta.data_ptr<float>(), query_start_loc.data_ptr<int>(),
-                                     state_idx.has_value() ? state_idx->data_ptr<int>() : nullptr, (int)B, (int)hq, (int)hv,
-                                     (int)q.size(2), (int)v.size(2), q.stride(0), k.stride(0), v.stride(0), (float)scale,
-                                     l2norm, has_initial.has_value() ? has_initial->data_ptr<int>() : nullptr,
-                                     dtype16(q), cur_stream());
+  p.out = out.data_ptr(); p.state = state.data_ptr<float>();
+  p.q = q.data_ptr(); p.k = k.data_ptr(); p.v = v.data_ptr();
+  p.query_start_loc = query_start_loc.data_ptr<int>();
+  p.state_idx = state_idx.has_value() ? state_idx->data_ptr<int>() : nullptr;
+  p.has_initial = has_initial.has_value() ? has_initial->data_ptr<int>() : nullptr;
+  p.tokens = T; p.q_stride = q.stride(0); p.k_stride = k.stride(0); p.v_stride = v.stride(0);
+  p.batch = (int)B; p.hq = (int)hq; p.hv = (int)hv; p.l2norm = l2norm; p.scale = (float)scale;
+  Tensor lengths;                                     // (a step of decode rows only has no groups of tokens)
+  p.lengths = nullptr;
+  if (T > B) {
+    lengths = at::empty({b200::gdn_lengths_bytes(T, (int)hq)}, q.options().dtype(at::kByte));
+    p.lengths = reinterpret_cast<const b200::GdnLengths*>(lengths.data_ptr());
+  }
+  const int rc = b200::gdn_recurrent(p, (int)q.size(2), (int)v.size(2), dtype16(q), cur_stream());
   TORCH_CHECK(rc == 0, "gdn_recurrent: head sizes must be 128 and value heads a multiple of q/k heads");
 }
 
@@ -722,6 +729,43 @@ void tq_decode(Tensor& out, const Tensor& q, const Tensor& cache, const Tensor& 
                                  seq_lens.data_ptr<int>(), (int)B, (int)hq, (int)hkv, (int)cache.size(1), cache.size(0),
                                  (int)splits, (float)scale, (int)kbits, (int)vbits, nc, dtype16(q), cur_stream());
   TORCH_CHECK(rc == 0, "tq_decode: unsupported format or GQA group (1, 2, 4, 8)");
+}
+void gdn_recurrent(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g,
+                   const Tensor& beta, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
+                   const optional<Tensor>& has_initial, double scale, bool l2norm) {
+  const int64_t n = v.numel() / (v.dim() == 3 && v.size(2) > 0 ? v.size(2) : 1);
+  TORCH_CHECK(g.is_contiguous() && beta.is_contiguous() && g.scalar_type() == at::kFloat && beta.scalar_type() == at::kFloat &&
+              g.numel() == n && beta.numel() == n);
+  b200::GdnParams p{};
+  p.g = g.data_ptr<float>(); p.beta = beta.data_ptr<float>();
+  gdn_run(out, state, q, k, v, query_start_loc, state_idx, has_initial, scale, l2norm, p);
+}
+// the same with g = -exp(a_log) softplus(a + dt_bias) and beta = sigmoid(b) of ba [T, Hq, 2 Hv / Hq] = (b.., a..) per key head
+void gdn_recurrent_ba(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& ba,
+                      const Tensor& a_log, const Tensor& dt_bias, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
+                      const optional<Tensor>& has_initial, double scale, bool l2norm) {
+  TORCH_CHECK(v.dim() == 3 && ba.dim() == 2 && ba.stride(1) == 1 && ba.size(0) == v.size(0) && ba.size(1) == 2 * v.size(1) &&
+              ba.scalar_type() == v.scalar_type());
+  TORCH_CHECK(a_log.is_contiguous() && dt_bias.is_contiguous() && a_log.scalar_type() == at::kFloat &&
+              dt_bias.scalar_type() == at::kFloat && a_log.numel() == v.size(1) && dt_bias.numel() == v.size(1));
+  b200::GdnParams p{};
+  p.ba = ba.data_ptr(); p.ba_stride = ba.stride(0);
+  p.a_log = a_log.data_ptr<float>(); p.dt_bias = dt_bias.data_ptr<float>();
+  gdn_run(out, state, q, k, v, query_start_loc, state_idx, has_initial, scale, l2norm, p);
+}
+// out [T, H * D] = norm(o) * silu(z), or o * sigmoid(z) without w; z [T, groups, at least rep * D]: head h in group h / rep
+void gated_head_norm(Tensor& out, const Tensor& o, const Tensor& z, const optional<Tensor>& w, int64_t dim, double eps) {
+  TORCH_CHECK(o.dim() == 2 && out.is_contiguous() && o.is_contiguous() && out.sizes() == o.sizes() && dim > 0 &&
+              o.size(1) % dim == 0);
+  TORCH_CHECK(z.dim() == 3 && z.stride(2) == 1 && z.size(0) == o.size(0) && z.size(1) * z.size(2) == o.size(1) &&
+              z.size(2) % dim == 0);
+  TORCH_CHECK(out.scalar_type() == o.scalar_type() && z.scalar_type() == o.scalar_type());
+  if (w.has_value()) TORCH_CHECK(w->is_contiguous() && w->numel() == dim && w->scalar_type() == o.scalar_type());
+  const c10::cuda::CUDAGuard guard(o.device());
+  const int rc = b200::gated_head_norm(out.data_ptr(), o.data_ptr(), z.data_ptr(), w.has_value() ? w->data_ptr() : nullptr,
+                                       o.size(0), (int)(o.size(1) / dim), (int)dim, (int)(z.size(2) / dim), z.stride(0),
+                                       z.stride(1), (float)eps, dtype16(o), cur_stream());
+  TORCH_CHECK(rc == 0, "gated_head_norm: heads of 64, 128 or 256 entries, rows on 16 bytes");
 }
 
 // o [T, H, 512] -> out [G, T, (H / G) * 512] with the rope dims rotated back
@@ -973,6 +1017,8 @@ TORCH_LIBRARY_FRAGMENT(b200, m) {
   m.def("rms_norm(Tensor(a!) out, Tensor x, Tensor weight, float eps, bool gemma) -> ()", &rms_norm);
   m.def("fused_add_rms_norm(Tensor(a!) x, Tensor(b!) residual, Tensor weight, float eps, bool gemma) -> ()",
         &fused_add_rms_norm);
+  m.def("gdn_recurrent_ba(Tensor(a!) out, Tensor(b!) state, Tensor q, Tensor k, Tensor v, Tensor ba, Tensor a_log, Tensor dt_bias, Tensor query_start_loc, Tensor? state_idx, Tensor? has_initial, float scale, bool l2norm) -> ()", &gdn_recurrent_ba);
+  m.def("gated_head_norm(Tensor(a!) out, Tensor o, Tensor z, Tensor? w, int dim, float eps) -> ()", &gated_head_norm);
   m.def("head_rms_norm(Tensor(a!) x, Tensor weight, float eps, int heads, int head_dim) -> ()", &head_rms_norm);
   m.def(
       "rms_norm_quant(Tensor(a!) out_q, Tensor(b!)? scale_out, Tensor? scale_in, Tensor x, Tensor(c!)? residual, "

@@ -6,14 +6,18 @@ namespace {
 
 using namespace b200_bind;
 
-// x [T, C] (row pitch free), w [C, K], state [slots, K-1, C] (in / out), all of one dtype (bf16 / fp16 / fp32)
-void causal_conv1d(Tensor& out, const Tensor& x, const Tensor& w, const optional<Tensor>& bias,
-                   const optional<Tensor>& state, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
-                   const optional<Tensor>& has_initial, bool silu) {
+// x [T, C] (row pitch free), w [C, K], state [slots, K-1, C] (in / out), all of one dtype (bf16 / fp16 / fp32).
+// heads > 0: x holds heads groups of equal width that start with dk of q, dk of k and dv of v; channels are all q, all k, all v
+void causal_conv1d_run(Tensor& out, const Tensor& x, const Tensor& w, const optional<Tensor>& bias,
+                       const optional<Tensor>& state, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
+                       const optional<Tensor>& has_initial, bool silu, int64_t heads, int64_t dk, int64_t dv) {
   on_device_of(x, {&out, &w, &query_start_loc}, {&bias, &state, &state_idx, &has_initial});
-  TORCH_CHECK(x.dim() == 2 && x.stride(1) == 1 && out.is_contiguous() && out.sizes() == x.sizes() &&
+  TORCH_CHECK(x.dim() == 2 && x.stride(1) == 1 && out.is_contiguous() && out.dim() == 2 && out.size(0) == x.size(0) &&
               out.scalar_type() == x.scalar_type());
-  const int64_t T = x.size(0), C = x.size(1), K = w.size(1);
+  const int64_t T = x.size(0), C = out.size(1), K = w.size(1);
+  const int64_t group = heads > 0 ? x.size(1) / heads : 0;
+  TORCH_CHECK(heads > 0 ? dk > 0 && dv > 0 && x.size(1) % heads == 0 && group >= 2 * dk + dv && C == heads * (2 * dk + dv)
+                        : heads == 0 && dk == 0 && dv == 0 && C == x.size(1));
   TORCH_CHECK(w.dim() == 2 && w.size(0) == C && w.is_contiguous() && w.scalar_type() == x.scalar_type());
   if (bias.has_value()) TORCH_CHECK(bias->is_contiguous() && bias->numel() == C && bias->scalar_type() == x.scalar_type());
   TORCH_CHECK(query_start_loc.scalar_type() == at::kInt && query_start_loc.is_contiguous());
@@ -31,8 +35,14 @@ void causal_conv1d(Tensor& out, const Tensor& x, const Tensor& w, const optional
                                      state.has_value() ? state->data_ptr() : nullptr, query_start_loc.data_ptr<int>(),
                                      state_idx.has_value() ? state_idx->data_ptr<int>() : nullptr,
                                      has_initial.has_value() ? has_initial->data_ptr<int>() : nullptr, (int)B, (int)T,
-                                     (int)C, (int)K, silu ? 1 : 0, dtype_code(x), cur_stream());
+                                     (int)C, (int)K, silu ? 1 : 0, (int)heads, (int)dk, (int)dv, (int)group, dtype_code(x),
+                                     cur_stream());
   TORCH_CHECK(rc == 0, "causal_conv1d: kernel width must be 1..8");
+}
+void causal_conv1d(Tensor& out, const Tensor& x, const Tensor& w, const optional<Tensor>& bias,
+                   const optional<Tensor>& state, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
+                   const optional<Tensor>& has_initial, bool silu) {
+  causal_conv1d_run(out, x, w, bias, state, query_start_loc, state_idx, has_initial, silu, 0, 0, 0);
 }
 
 // ------------------------------------------------------------------ linear attention
@@ -228,6 +238,7 @@ void prenorm(Tensor& h, const optional<Tensor>& x_out, const Tensor& y, const op
 }  // namespace
 
 TORCH_LIBRARY_FRAGMENT(b200, m) {
+  m.def("causal_conv1d_heads(Tensor(a!) out, Tensor x, Tensor w, Tensor? bias, Tensor(b!)? state, Tensor query_start_loc, Tensor? state_idx, Tensor? has_initial, bool silu, int heads, int dk, int dv) -> ()", &causal_conv1d_run);
   m.def("causal_conv1d(Tensor(a!) out, Tensor x, Tensor w, Tensor? bias, Tensor(b!)? state, Tensor query_start_loc, Tensor? state_idx, Tensor? has_initial, bool silu) -> ()", &causal_conv1d);
   m.def("gla_scratch_floats(Tensor like, int batch, int heads, int dim, int vdim, int max_query_len, bool whole_row=False) -> int", &gla_scratch_floats);
   m.def(

@@ -326,14 +326,29 @@ void v4_indexer_q(void* q8, float* w_out, const void* q, int64_t q_stride_t, int
                   int64_t w_stride, const int64_t* positions, const float* cos_sin, int tokens, int heads, int rot,
                   float softmax_scale, float head_scale, int dtype, cudaStream_t stream);
 // ---- gdn.cu
-int gdn_recurrent(void* out, float* state, const void* q, const void* k, const void* v, const float* g, const float* beta,
-                  const int* query_start_loc, const int* state_idx, int batch, int hq, int hv, int dk, int dv,
-                  int64_t q_stride, int64_t k_stride, int64_t v_stride, float scale, int l2norm,
-                  const int* has_initial, int dtype, cudaStream_t stream);
+struct GdnLengths;
+struct GdnParams {
+  void* out;                 // [tokens, hv, 128]
+  float* state;              // [slots, hv, 128, 128]
+  const void *q, *k, *v;     // [tokens, hq | hv, 128] with token strides in elements
+  const float *g, *beta;     // [tokens, hv] log decay and beta, or null: from
+  const void* ba;            // [tokens, hq, (b of the group's heads, a of them)] with a token stride,
+  const float *a_log, *dt_bias;   // [hv]
+  const int *query_start_loc, *state_idx, *has_initial;
+  const GdnLengths* lengths; // gdn_lengths_bytes() of scratch, or null: a token at a time
+  int64_t tokens, q_stride, k_stride, v_stride, ba_stride;
+  int batch, hq, hv, l2norm;
+  float scale;
+};
+int64_t gdn_lengths_bytes(int64_t tokens, int hq);
+int gdn_recurrent(const GdnParams& p, int dk, int dv, int dtype, cudaStream_t stream);
+// out[t, h] = (unit_rms(o[t, h]) * w) * silu(z[t, h / rep, h % rep]), or o * sigmoid(z) without w; 0, 1: head size, 2: alignment
+int gated_head_norm(void* out, const void* o, const void* z, const void* w, int64_t tokens, int heads, int dim, int rep,
+                    int64_t z_stride, int64_t z_group, float eps, int dtype, cudaStream_t stream);
 // ---- causal_conv1d.cu (depthwise causal convolution over ragged batches with a per-sequence carry)
 int causal_conv1d(void* out, const void* x, int64_t x_stride, const void* w, const void* bias, void* state,
                   const int* query_start_loc, const int* state_idx, const int* has_init, int batch, int tokens,
-                  int channels, int K, int silu, int dtype, cudaStream_t stream);
+                  int channels, int K, int silu, int heads, int dk, int dv, int group, int dtype, cudaStream_t stream);
 // ---- residual_conv.cu (post-norm residual add + short input convolution, fp32 residual stream)
 struct ResidualConvParams {
   const void* y;           // [tokens, D] sublayer output (or the embedding rows when x is null)

@@ -25,7 +25,6 @@ from typing import Optional
 
 import torch
 import torch.nn as nn
-import torch.nn.functional as F
 
 from .. import _custom_ops as ops
 from ..attention.metadata import get_forward_context
@@ -108,20 +107,16 @@ class GatedDeltaNet(nn.Module):
         md = get_forward_context().attn_metadata
         T = h.shape[0]
         idx, init, qsl = md.extra["state_indices"], md.extra["state_has_init"], md.query_start_loc
-        qkvz = self.in_proj_qkvz(h).reshape(T, self.nk_l, 2 * self.dk + 2 * self.rep * self.dv)
-        ba = self.in_proj_ba(h).reshape(T, self.nk_l, 2 * self.rep)
-        q, k, v, z = qkvz.split([self.dk, self.dk, self.rep * self.dv, self.rep * self.dv], -1)
-        b, a = ba.split([self.rep, self.rep], -1)
-        mixed = torch.cat([q.reshape(T, self.key_l), k.reshape(T, self.key_l), v.reshape(T, self.val_l)], -1)
-        mixed = gdn.causal_conv1d(mixed, self.conv1d.weight, None, self.conv_state, qsl, idx, init, silu=True)
+        qkvz = self.in_proj_qkvz(h)                       # per k head: q, k, its v heads, their gates z
+        ba = self.in_proj_ba(h)
+        mixed = gdn.causal_conv1d(qkvz, self.conv1d.weight, None, self.conv_state, qsl, idx, init, silu=True,
+                                  heads=(self.nk_l, self.dk, self.rep * self.dv))
         q, k, v = mixed.split([self.key_l, self.key_l, self.val_l], -1)
-        beta = torch.sigmoid(b.reshape(T, self.nv_l).float())
-        g = -torch.exp(self.A_log) * F.softplus(a.reshape(T, self.nv_l).float() + self.dt_bias)
-        o = gdn.gated_delta_rule(q.reshape(T, self.nk_l, self.dk).contiguous(), k.reshape(T, self.nk_l, self.dk).contiguous(),
-                                 v.reshape(T, self.nv_l, self.dv).contiguous(), g, beta, qsl, self.ssm_state, idx, init)
-        o = ops.rms_norm(o.reshape(T * self.nv_l, self.dv), self.norm.weight, self.norm.eps)
-        o = (o.float() * F.silu(z.reshape(T * self.nv_l, self.dv).float())).to(h.dtype)
-        return self.out_proj(o.reshape(T, self.val_l))
+        o = gdn.gated_delta_rule_ba(q.view(T, self.nk_l, self.dk), k.view(T, self.nk_l, self.dk), v.view(T, self.nv_l, self.dv),
+                                    ba, self.A_log, self.dt_bias, qsl, self.ssm_state, idx, init)
+        z = qkvz.view(T, self.nk_l, -1)[..., 2 * self.dk + self.rep * self.dv:]
+        o = gdn.gated_head_norm(o.reshape(T, self.val_l), z, self.norm.weight, self.dv, self.norm.eps)
+        return self.out_proj(o)
 
 
 class GatedAttention(nn.Module):
@@ -145,15 +140,13 @@ class GatedAttention(nn.Module):
         T, D, H, Hkv = h.shape[0], self.head_dim, self.num_heads, self.num_kv_heads
         qkv = self.qkv_proj(h)
         qg = qkv[:, : 2 * H * D].reshape(T, H, 2, D)
-        q = qg[:, :, 0].reshape(T, H * D)                 # contiguous copies: the kernels want dense head rows
-        gate = qg[:, :, 1].reshape(T, H * D)
+        q = qg[:, :, 0].reshape(T, H * D)                 # a contiguous copy: the kernels want dense head rows
         k = qkv[:, 2 * H * D: (2 * H + Hkv) * D]
         v = qkv[:, (2 * H + Hkv) * D:]
         ops.head_rms_norm(q, self.q_norm.weight, self.q_norm.eps, H, D)
         ops.head_rms_norm(k, self.k_norm.weight, self.k_norm.eps, Hkv, D)
         o = self.attn(q, k, v, positions, self.rope)
-        o = (o.float() * torch.sigmoid(gate.float())).to(h.dtype)
-        return self.o_proj(o)
+        return self.o_proj(gdn.gated_head_norm(o, qg[:, :, 1], None, D))
 
 
 class Qwen3NextDecoderLayer(nn.Module):

@@ -142,13 +142,58 @@ def gated_delta_rule(q, k, v, g, beta, query_start_loc, state=None, state_indice
         state = torch.zeros(1, Hv, 128, 128, dtype=torch.float32, device=q.device)
         state_indices = None
     out = torch.empty_like(v)
-    ops._launches += 1
+    ops._launches += 2 if q.shape[0] > query_start_loc.numel() - 1 else 1
     torch.ops.b200.gdn_recurrent(
         out, state, q, k, v, g.float().contiguous(), beta.float().contiguous(), query_start_loc.int().contiguous(),
         None if state_indices is None else state_indices.int().contiguous(),
         None if has_initial_state is None else has_initial_state.int().contiguous(),
         q.shape[-1] ** -0.5 if scale is None else scale, l2norm)
     return out
+
+
+def gated_delta_rule_ba(q, k, v, ba, a_log, dt_bias, query_start_loc, state=None, state_indices=None, has_initial_state=None,
+                        scale: Optional[float] = None, l2norm: bool = True):
+    """:func:`gated_delta_rule` with ``g = -exp(a_log) softplus(a + dt_bias)`` and ``beta = sigmoid(b)`` of the projection
+    ``ba [T, Hq * 2 rep]``, which holds per key head ``rep = Hv / Hq`` numbers b and as many a; formed in the kernel."""
+    from .. import envs
+
+    T, Hq, Hv = q.shape[0], q.shape[1], v.shape[1]
+    if not q.is_cuda or envs.B200_GDN_CHUNKED or state is None:
+        b, a = ba.reshape(T, Hq, 2 * (Hv // Hq)).chunk(2, -1)
+        beta = torch.sigmoid(b.reshape(T, Hv).float())
+        g = -torch.exp(a_log) * torch.nn.functional.softplus(a.reshape(T, Hv).float() + dt_bias)
+        return gated_delta_rule(q, k, v, g, beta, query_start_loc, state, state_indices, has_initial_state, scale, l2norm)
+    from .. import _custom_ops as ops
+
+    ops.load_native()
+    out = torch.empty(v.shape, dtype=v.dtype, device=v.device)
+    ops._launches += 2 if T > query_start_loc.numel() - 1 else 1
+    torch.ops.b200.gdn_recurrent_ba(
+        out, state, q, k, v, ba, a_log, dt_bias, query_start_loc.int().contiguous(),
+        None if state_indices is None else state_indices.int().contiguous(),
+        None if has_initial_state is None else has_initial_state.int().contiguous(),
+        q.shape[-1] ** -0.5 if scale is None else scale, l2norm)
+    return out
+
+
+def gated_head_norm(o, z, weight, dim: int, eps: float = 0.0):
+    """``o [T, H * dim]``: unit RMS per head times ``weight [dim]`` times ``silu(z)``, or without a weight ``o * sigmoid(z)``.
+    ``z [T, groups, H / groups * dim]`` may be a view into a wider product."""
+    if o.is_cuda and o.dtype in (torch.bfloat16, torch.float16) and dim in (64, 128, 256) and z.stride(0) % 8 == 0 \
+            and z.stride(1) % 8 == 0 and z.data_ptr() % 16 == 0:
+        from .. import _custom_ops as ops
+
+        ops.load_native()
+        out = torch.empty_like(o)
+        ops._launches += 1
+        torch.ops.b200.gated_head_norm(out, o, z, weight, dim, eps)
+        return out
+    if weight is None:
+        return (o.float() * torch.sigmoid(z.reshape(o.shape).float())).to(o.dtype)
+    from .. import _custom_ops as ops
+
+    y = ops.rms_norm(o.reshape(-1, dim), weight, eps)
+    return (y.float() * torch.nn.functional.silu(z.reshape(y.shape).float())).to(o.dtype).reshape(o.shape)
 
 
 # ------------------------------------------------------------------------------------------ short causal convolution
@@ -180,18 +225,27 @@ def causal_conv1d_ref(x, w, bias=None, state=None, query_start_loc=None, state_i
 
 
 def causal_conv1d(x, w, bias=None, state=None, query_start_loc=None, state_indices=None, has_initial_state=None,
-                  silu: bool = True):
+                  silu: bool = True, heads: Optional[tuple] = None):
     """Depthwise causal convolution (+ SiLU) over a ragged batch; the last ``K-1`` inputs of every sequence are carried
-    in ``state`` between steps.  Parity: the ``causal_conv1d_fn`` / ``causal_conv1d_update`` pair the reference's GDN
+    in ``state`` between steps.  ``heads = (n, dk, dv)``: ``x`` is a projection of ``n`` groups of equal width that start with
+    ``dk`` entries of q, ``dk`` of k and ``dv`` of v; channels (and the result) are all q, all k, all v.
+    Parity: the ``causal_conv1d_fn`` / ``causal_conv1d_update`` pair the reference's GDN
     layer calls (vllm_metax/registry/custom_ops/layers/mamba/qwen_gdn_linear_attn.py:8-10)."""
     if not x.is_cuda:
+        if heads is not None:
+            n, dk, dv = heads
+            x = x.reshape(x.shape[0], n, -1)
+            x = torch.cat([t.flatten(1) for t in x[..., : 2 * dk + dv].split([dk, dk, dv], -1)], -1)
         return causal_conv1d_ref(x, w, bias, state, query_start_loc, state_indices, has_initial_state, silu)
     from .. import _custom_ops as ops
 
     ops.load_native(units="core")
-    out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+    out = torch.empty(x.shape if heads is None else (x.shape[0], w.shape[0]), dtype=x.dtype, device=x.device)
     ops._launches += 2 if state is not None else 1
-    torch.ops.b200.causal_conv1d(out, x, w.contiguous(), bias, state, query_start_loc.int().contiguous(),
-                                 None if state_indices is None else state_indices.int().contiguous(),
-                                 None if has_initial_state is None else has_initial_state.int().contiguous(), silu)
+    rest = (query_start_loc.int().contiguous(), None if state_indices is None else state_indices.int().contiguous(),
+            None if has_initial_state is None else has_initial_state.int().contiguous(), silu)
+    if heads is None:
+        torch.ops.b200.causal_conv1d(out, x, w.contiguous(), bias, state, *rest)
+    else:
+        torch.ops.b200.causal_conv1d_heads(out, x, w.contiguous(), bias, state, *rest, *heads)
     return out
