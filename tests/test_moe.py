@@ -148,3 +148,60 @@ def test_moe_chunked_over_tokens_equals_one_pass(monkeypatch):
     torch.testing.assert_close(moe.forward(x, logits, shared), want, rtol=1e-5, atol=1e-5)
     monkeypatch.setenv("B200_FUSED_MOE_CHUNK_SIZE", "0")
     torch.testing.assert_close(moe.forward(x, logits, None), moe.forward(x, logits, shared) - shared, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("numel,experts,block", [(4096, 128, 128), (4104, 3, 16), (9000, 64, 128), (70001, 128, 128),
+                                                 (200003, 1024, 64)])
+@pytest.mark.parametrize("mapped", [False, True])
+def test_moe_align_by_several_ctas(numel, experts, block, mapped):
+    """The order of one CTA's placement and of many's against the stable sort: around the size where they part, segments that
+    end early, experts without pairs, pairs routed elsewhere."""
+    from vllm_metax_b200 import _custom_ops as ops
+
+    g = torch.Generator().manual_seed(numel)
+    ids = (torch.rand(numel, generator=g).pow(3) * experts).to(torch.int32)      # the first experts get most
+    emap = None
+    if mapped:
+        emap = torch.arange(experts, dtype=torch.int32)
+        emap[::3] = -1
+    want = ops.moe_align_block_size(ids, block, experts, emap, want_inverse=True)
+    got = ops.moe_align_block_size(ids.cuda(), block, experts, None if emap is None else emap.cuda(), want_inverse=True)
+    for a, b in zip(got, want):
+        assert torch.equal(a.cpu().reshape(-1), b.reshape(-1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens,topk,hidden,experts", [(1, 8, 2048, 16), (37, 3, 2176, 8), (300, 10, 7168, 64), (5, 1, 264, 4)])
+def test_moe_rows_from_the_pairs(dtype, tokens, topk, hidden, experts):
+    """Scattered rows equal gathered ones (padding apart), as they are, weighted and quantised; combined rows equal the sum in
+    fp32 in the order of the pairs, rounded once."""
+    from vllm_metax_b200 import _custom_ops as ops
+
+    g = torch.Generator().manual_seed(tokens)
+    x = torch.randn(tokens, hidden, generator=g).to(dtype).cuda()
+    ids = torch.stack([torch.randperm(experts, generator=g)[:topk] if topk <= experts else
+                       torch.randint(0, experts, (topk,), generator=g) for _ in range(tokens)]).to(torch.int32).cuda()
+    emap = torch.arange(experts, dtype=torch.int32).cuda()
+    emap[0] = -1                                            # one expert is elsewhere
+    w = torch.rand(tokens, topk, generator=g).cuda()
+    sorted_ids, be, total, inv = ops.moe_align_block_size(ids, 128, experts, emap, want_inverse=True)
+    real = sorted_ids < ids.numel()
+    for weights in (None, w):
+        got, want = ops.moe_scatter(x, inv, sorted_ids, total, topk, weights), ops.moe_gather(x, sorted_ids, total, topk, weights)
+        assert torch.equal(got[real], want[real])
+    if hidden % 128 == 0:
+        q, s = ops.moe_scatter_fp8(x, inv, sorted_ids, total, topk)
+        wq, ws = ops.per_token_group_quant_fp8(ops.moe_gather(x, sorted_ids, total, topk), 128)
+        assert torch.equal(q[real].view(torch.uint8), wq[real].view(torch.uint8)) and torch.equal(s[real], ws[real])
+        h = torch.cat([want, want.flip(1)], 1)
+        a, b = ops.silu_and_mul_per_block_quant(h, 128), ops.silu_and_mul_per_block_quant(h, 128, sorted_ids=sorted_ids, numel=ids.numel())
+        assert torch.equal(a[0][real].view(torch.uint8), b[0][real].view(torch.uint8)) and torch.equal(a[1][real], b[1][real])
+    shared = torch.randn(tokens, hidden, generator=g).to(dtype).cuda()
+    y = torch.randn(sorted_ids.numel(), hidden, generator=g).to(dtype).cuda()
+    out = ops.moe_combine(y, w, inv, tokens, shared)
+    acc, iv = shared.float(), inv.view(tokens, topk).long()
+    for k in range(topk):
+        acc = torch.where((iv[:, k] >= 0)[:, None], acc + w[:, k: k + 1] * y[iv[:, k].clamp_min(0)].float(), acc)
+    torch.testing.assert_close(out.float(), acc, rtol=2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10, atol=1e-5)

@@ -206,3 +206,48 @@ def test_scaled_mm_grouped_gpu(kernel_status_ok):
     n = int(total_padded.item())
     valid = torch.repeat_interleave(block_expert[: n // 128].cpu() >= 0, 128)
     assert cos_diff(out[:n].cpu()[valid], want[:n][valid]) < 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (64, 2112, 7168), (64, 576, 512), (37, 4096, 2048), (130, 24576, 1536),
+                                   (129, 18944, 256), (300, 7168, 2048), (2100, 2560, 1024), (1836, 2112, 1536)])
+def test_fp8_block_scaled_mm_shapes(M, N, K):
+    """Tiles of both widths, ranges of the (tile, k block) space that cut tiles, groups of row blocks with a short last one, ragged
+    rows and columns.  Products of e4m3 are exact in fp32 and their sums over 128 nearly so; one rounding to bf16 at the end."""
+    g = torch.Generator().manual_seed(M + N)
+    a = torch.randn(M, K, generator=g).to(torch.float8_e4m3fn).cuda()
+    w = torch.randn(N, K, generator=g).to(torch.float8_e4m3fn).cuda()
+    a_s = (torch.rand(M, K // 128, generator=g) + 0.5).cuda()
+    w_s = (torch.rand(-(-N // 128), K // 128, generator=g) + 0.5).cuda()
+    out = ops.fp8_block_scaled_mm(a, a_s, w, w_s)
+    ad = a.double() * a_s.double().repeat_interleave(128, 1)
+    wd = w.double() * w_s.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)
+    want = ad @ wd.T
+    torch.testing.assert_close(out.double(), want, rtol=2.0 ** -8 * 1.01, atol=1e-5 * float(want.abs().max()))
+    ops.check_kernel_status(0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,topk,E,N,K", [(5, 2, 4, 256, 256), (64, 8, 64, 512, 1024), (700, 3, 5, 2304, 512)])
+def test_fp8_grouped_mm_without_padding(T, topk, E, N, K):
+    """Experts' rows at the start of their blocks: one, a few, all of a block; padding rows hold NaN and touch nothing."""
+    g = torch.Generator().manual_seed(T)
+    ids = torch.stack([torch.randperm(E, generator=g)[:topk] for _ in range(T)]).to(torch.int32).cuda()
+    sorted_ids, be, total, inv = ops.moe_align_block_size(ids, 128, E, want_inverse=True)
+    real = sorted_ids < ids.numel()
+    x = torch.randn(T, K, generator=g).bfloat16().cuda()
+    a, a_s = ops.moe_scatter_fp8(x, inv, sorted_ids, total, topk)
+    a.view(torch.uint8)[~real] = 0x7F
+    a_s[~real] = float("nan")
+    w = torch.randn(E, N, K, generator=g).to(torch.float8_e4m3fn).cuda()
+    w_s = (torch.rand(E, -(-N // 128), K // 128, generator=g) + 0.5).cuda()
+    out = ops.fp8_block_scaled_mm(a, a_s, w, w_s, torch.bfloat16, be, total, sorted_ids, ids.numel())
+    whole = ops.fp8_block_scaled_mm(a, a_s, w, w_s, torch.bfloat16, be, total)
+    assert torch.equal(out[real], whole[real])
+    rows, e = real.nonzero()[:, 0], be.long().repeat_interleave(128)[real]
+    ad = a[rows].double() * a_s[rows].double().repeat_interleave(128, 1)
+    for i in e.unique().tolist():
+        wd = w[i].double() * w_s[i].double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)
+        want = ad[e == i] @ wd.T
+        torch.testing.assert_close(out[rows[e == i]].double(), want, rtol=2.0 ** -8 * 1.01, atol=1e-5 * float(want.abs().max()))
+    ops.check_kernel_status(0)

@@ -389,12 +389,14 @@ def silu_and_mul_quant(x, scale):
     return ref.silu_and_mul_quant(x, scale)
 
 
-def silu_and_mul_per_block_quant(x, group_size=128, ue8m0=False, act: str = "silu"):
+def silu_and_mul_per_block_quant(x, group_size=128, ue8m0=False, act: str = "silu", sorted_ids=None, numel: int = 0):
+    """``sorted_ids`` (an id per row of ``x``): rows with ids from ``numel`` on are padding, whose results nobody reads."""
     if _use_cuda(x):
         d = x.shape[-1] // 2
         out = torch.empty(*x.shape[:-1], d, dtype=torch.float8_e4m3fn, device=x.device)
         scales = torch.empty(*x.shape[:-1], d // group_size, dtype=torch.float32, device=x.device)
-        torch.ops.b200.act_and_mul_quant(out, scales, None, x.contiguous(), ACT_CODES[act], 0.0, 7.0, group_size, ue8m0)
+        torch.ops.b200.act_and_mul_quant(out, scales, None, x.contiguous(), ACT_CODES[act], 0.0, 7.0, group_size, ue8m0,
+                                         sorted_ids, numel)
         return out, scales
     y = ref.swiglustep_and_mul(x) if act == "swiglustep" else ref.silu_and_mul(x)
     return ref.per_token_group_quant_fp8(y, group_size, ue8m0=ue8m0)
@@ -740,6 +742,26 @@ def moe_align_block_size(topk_ids, block_size: int, num_experts: int, expert_map
     return (sorted_ids, block_expert, total, inv) if want_inverse else (sorted_ids, block_expert, total)
 
 
+def moe_scatter(x, inv, sorted_ids, total_padded, topk: int, weights=None):
+    """:func:`moe_gather` for a consumer that does not look at rows of padding: these stay unwritten."""
+    if _use_cuda(x) and x.dtype != torch.float32 and x.shape[1] % 8 == 0:
+        out = torch.empty(sorted_ids.numel(), x.shape[1], dtype=x.dtype, device=x.device)
+        if torch.ops.b200.moe_scatter(out, None, x.contiguous(), inv, topk, weights):
+            return out
+    return moe_gather(x, sorted_ids, total_padded, topk, weights)
+
+
+def moe_scatter_fp8(x, inv, sorted_ids, total_padded, topk: int):
+    """Expert-sorted rows of ``x`` as e4m3 with a scale per 128 entries: ``([max_padded, H], [max_padded, H / 128])``; rows of
+    padding stay unwritten."""
+    if _use_cuda(x):
+        out = torch.empty(sorted_ids.numel(), x.shape[1], dtype=torch.float8_e4m3fn, device=x.device)
+        scales = torch.empty(sorted_ids.numel(), x.shape[1] // 128, dtype=torch.float32, device=x.device)
+        if torch.ops.b200.moe_scatter(out, scales, x.contiguous(), inv, topk, None):
+            return out, scales
+    return per_token_group_quant_fp8(moe_gather(x, sorted_ids, total_padded, topk), 128)
+
+
 def moe_gather(x, sorted_ids, total_padded, topk: int, weights=None):
     """Rows of ``x [T,H]`` in expert-sorted order, zero rows for padding: ``[max_padded, H]``.  ``weights [T, topk]`` (fp32):
     each pair's row is multiplied by its weight."""
@@ -893,13 +915,15 @@ def merge_attn_states(prefix_out, prefix_lse, suffix_out, suffix_lse, want_lse: 
     return (out, lse) if want_lse else out
 
 
-def fp8_block_scaled_mm(aq, a_scale, wq, w_scale, out_dtype=torch.bfloat16, block_expert=None, total_padded=None):
-    """Block-scaled fp8 GEMM (1x128 activation scales, 128x128 weight scales); grouped when ``wq`` is 3-D."""
+def fp8_block_scaled_mm(aq, a_scale, wq, w_scale, out_dtype=torch.bfloat16, block_expert=None, total_padded=None,
+                        sorted_ids=None, numel: int = 0):
+    """Block-scaled fp8 GEMM (1x128 activation scales, 128x128 weight scales); grouped when ``wq`` is 3-D.  ``sorted_ids``: rows
+    with ids from ``numel`` on are padding at the end of an expert's rows; what they become nobody reads."""
     if _use_cuda(aq):
         n = wq.shape[-2]
         out = torch.empty(aq.shape[0], n, dtype=out_dtype, device=aq.device)
         torch.ops.b200.gemm_fp8_blockscale(out, aq, a_scale.contiguous(), wq, w_scale.contiguous(), block_expert,
-                                           total_padded)
+                                           total_padded, sorted_ids, numel)
         return out
     if wq.dim() == 2:
         return ref.fp8_block_scaled_mm(aq, a_scale, wq, w_scale, out_dtype)
@@ -1029,6 +1053,25 @@ def mla_decode(q, mla_cache, block_table, seq_lens, scale, *, query_start_loc=No
         out.copy_(res)
         return out
     return res
+
+
+def mla_rope_insert(q, qa, kv_c, k_pe, cache, kv, norm_weight, positions, cos_sin, slots, eps: float) -> bool:
+    """See :meth:`layers.mla.MLAAttention.rope_insert`; False: not done (there is no statement of it in plain tensors)."""
+    if not _use_cuda(q):
+        return False
+    torch.ops.b200.mla_rope_insert(q, qa, kv_c, k_pe, cache, kv, norm_weight, positions, cos_sin, slots, eps)
+    return True
+
+
+def mla_expand_keys(kv, k_pe, nope: int):
+    """``[T, H, nope + 64]``: every head's own key part beside the shared rotated one."""
+    T, H, _ = kv.shape
+    if _use_cuda(kv) and kv.dtype != torch.float32 and nope % 8 == 0 and kv.shape[2] % 8 == 0 and kv.is_contiguous() \
+            and k_pe.shape[1] == 64 and k_pe.is_contiguous() and kv.data_ptr() % 16 == 0 and k_pe.data_ptr() % 16 == 0:
+        out = torch.empty(T, H, nope + 64, dtype=kv.dtype, device=kv.device)
+        torch.ops.b200.mla_expand_keys(out, kv, k_pe, nope)
+        return out
+    return torch.cat([kv[..., :nope], k_pe[:, None, :].expand(-1, H, -1)], dim=-1)
 
 
 def rope_angles(positions, inv_freq, tokens: int):

@@ -91,6 +91,41 @@ void concat_and_cache_mla(const Tensor& kv_c, const Tensor& k_pe, Tensor& cache,
                              kv_c.size(0), rank, rope, kv_c.stride(0), k_pe.stride(0), num_slots, rec, dtype16(kv_c),
                              status_ptr(kv_c), cur_stream());
 }
+// q [T, H, D] in place (its last 64 entries), kv [T, 576] with a row pitch; kv_c, k_pe, the cache rows and qa [n, H, 576] are written
+void mla_rope_insert(Tensor& q, Tensor& qa, Tensor& kv_c, Tensor& k_pe, Tensor& cache, const Tensor& kv, const Tensor& norm_w,
+                     const Tensor& positions, const Tensor& cos_sin, const Tensor& slots, double eps) {
+  const int64_t T = q.size(0);
+  TORCH_CHECK(q.dim() == 3 && q.is_contiguous() && q.size(2) % 8 == 0 && q.size(2) >= 64 && kv.dim() == 2 && kv.size(0) == T &&
+              kv.size(1) == 576 && kv.stride(1) == 1 && kv.stride(0) % 8 == 0);
+  TORCH_CHECK(qa.dim() == 3 && qa.is_contiguous() && qa.size(0) <= T && qa.size(1) == q.size(1) && qa.size(2) == 576);
+  TORCH_CHECK(kv_c.is_contiguous() && kv_c.numel() == T * 512 && k_pe.is_contiguous() && k_pe.numel() == T * 64 &&
+              norm_w.is_contiguous() && norm_w.numel() == 512 && cache.is_contiguous() && cache.size(-1) == 576);
+  TORCH_CHECK(positions.scalar_type() == at::kLong && positions.is_contiguous() && positions.numel() >= T &&
+              slots.scalar_type() == at::kLong && slots.is_contiguous() && slots.numel() >= T);
+  TORCH_CHECK(cos_sin.scalar_type() == at::kFloat && cos_sin.is_contiguous() && cos_sin.size(-1) == 64);
+  for (const Tensor* x : {&kv, (const Tensor*)&qa, (const Tensor*)&kv_c, (const Tensor*)&k_pe, (const Tensor*)&cache, &norm_w})
+    TORCH_CHECK(x->scalar_type() == q.scalar_type() && reinterpret_cast<uintptr_t>(x->data_ptr()) % 16 == 0);
+  const c10::cuda::CUDAGuard guard(q.device());
+  b200::MlaRopeInsertParams p{};
+  p.q = q.data_ptr(); p.qa = qa.data_ptr(); p.kv = kv.data_ptr(); p.norm_w = norm_w.data_ptr();
+  p.kv_c = kv_c.data_ptr(); p.k_pe = k_pe.data_ptr(); p.cache = cache.data_ptr(); p.cos_sin = cos_sin.data_ptr<float>();
+  p.positions = positions.data_ptr<int64_t>(); p.slots = slots.data_ptr<int64_t>();
+  p.kv_stride = kv.stride(0); p.num_slots = cache.numel() / 576; p.tokens = T; p.absorbed = qa.size(0);
+  p.heads = (int)q.size(1); p.q_dim = (int)q.size(2); p.eps = (float)eps;
+  p.status = reinterpret_cast<b200::StatusWord*>(status_ptr(q));
+  b200::mla_rope_insert(p, dtype16(q), cur_stream());
+}
+// out [T, H, nope + 64] = (kv [T, H, D][..., :nope] | k_pe [T, 64])
+void mla_expand_keys(Tensor& out, const Tensor& kv, const Tensor& k_pe, int64_t nope) {
+  TORCH_CHECK(kv.dim() == 3 && kv.is_contiguous() && out.is_contiguous() && k_pe.is_contiguous() && out.dim() == 3);
+  TORCH_CHECK(nope % 8 == 0 && kv.size(2) % 8 == 0 && nope <= kv.size(2) && out.size(0) == kv.size(0) && out.size(1) == kv.size(1) &&
+              out.size(2) == nope + 64 && k_pe.numel() == kv.size(0) * 64);
+  for (const Tensor* x : {&kv, (const Tensor*)&out, &k_pe})
+    TORCH_CHECK(x->element_size() == 2 && reinterpret_cast<uintptr_t>(x->data_ptr()) % 16 == 0);
+  const c10::cuda::CUDAGuard guard(kv.device());
+  b200::mla_expand_keys(out.data_ptr(), kv.data_ptr(), k_pe.data_ptr(), kv.size(0), (int)kv.size(1), (int)nope, (int)kv.size(2),
+                        cur_stream());
+}
 void indexer_k_quant_and_cache(const Tensor& k, Tensor& cache, const Tensor& slot_mapping, int64_t block_size,
                                bool ue8m0, bool int8) {
   const int hd = k.size(-1);
@@ -115,13 +150,18 @@ void activation(Tensor& out, const Tensor& x, int64_t act, double p0) {
   b200::activation(out.data_ptr(), x.data_ptr(), x.numel(), act, (float)p0, dtype16(x), cur_stream());
 }
 void act_and_mul_quant(Tensor& out_q, const optional<Tensor>& scale_out, const optional<Tensor>& scale_in,
-                       const Tensor& x, int64_t act, double p0, double p1, int64_t group, bool ue8m0) {
+                       const Tensor& x, int64_t act, double p0, double p1, int64_t group, bool ue8m0,
+                       const optional<Tensor>& sorted_ids, int64_t numel) {
   TORCH_CHECK(x.is_contiguous() && out_q.is_contiguous());
+  if (sorted_ids.has_value())
+    TORCH_CHECK(sorted_ids->is_contiguous() && sorted_ids->scalar_type() == at::kInt &&
+                sorted_ids->numel() == x.numel() / x.size(-1));
   const int d = x.size(-1) / 2;
   const int tokens = x.numel() / x.size(-1);
   const c10::cuda::CUDAGuard guard(x.device());
   b200::act_and_mul_quant(out_q.data_ptr(), ptr<float>(scale_out), ptr<float>(scale_in), x.data_ptr(), tokens, d, act,
-                          (float)p0, (float)p1, group, ue8m0, dtype16(x), cur_stream());
+                          (float)p0, (float)p1, group, ue8m0, sorted_ids.has_value() ? sorted_ids->data_ptr<int>() : nullptr, (int)numel,
+                          dtype16(x), cur_stream());
 }
 
 // ------------------------------------------------------------------ quantisation
@@ -158,7 +198,8 @@ void merge_attn_states(Tensor& out, const optional<Tensor>& out_lse, const Tenso
                           dtype16(p_out), cur_stream());
 }
 void gemm_fp8_blockscale(Tensor& out, const Tensor& a, const Tensor& a_scale, const Tensor& w, const Tensor& w_scale,
-                         const optional<Tensor>& block_expert, const optional<Tensor>& total_padded) {
+                         const optional<Tensor>& block_expert, const optional<Tensor>& total_padded,
+                         const optional<Tensor>& sorted_ids, int64_t numel) {
   const bool grouped = w.dim() == 3;
   TORCH_CHECK(a.dim() == 2 && a.stride(1) == 1 && w.is_contiguous() && a_scale.is_contiguous() && w_scale.is_contiguous());
   TORCH_CHECK(a.element_size() == 1 && w.element_size() == 1 && a.size(1) % 128 == 0 && a.stride(0) % 16 == 0);
@@ -167,10 +208,25 @@ void gemm_fp8_blockscale(Tensor& out, const Tensor& a, const Tensor& a_scale, co
   TORCH_CHECK(w.size(-1) == K && out.size(0) == M && out.size(1) == N && out.stride(1) == 1);
   TORCH_CHECK(a_scale.size(-1) == K / 128 && w_scale.size(-1) == K / 128 && w_scale.size(-2) == (N + 127) / 128);
   if (grouped) TORCH_CHECK(block_expert.has_value() && total_padded.has_value() && M % 128 == 0);
+  if (sorted_ids.has_value())
+    TORCH_CHECK(grouped && sorted_ids->scalar_type() == at::kInt && sorted_ids->is_contiguous() && sorted_ids->numel() == M);
   const c10::cuda::CUDAGuard guard(a.device());
+  static int sms_of[64] = {};
+  int& sms = sms_of[a.get_device() & 63];
+  if (sms == 0) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a.get_device());
+  int64_t floats = 0, counters = 0;
+  Tensor scratch;                                   // of this call alone: any stream, any thread
+  int* zero = nullptr;
+  if (!grouped) b200::gemm_fp8_scratch(M, N, K, sms, &floats, &counters);
+  if (floats > 0) {
+    scratch = at::empty({floats + counters}, a_scale.options());
+    zero = reinterpret_cast<int*>(scratch.data_ptr<float>() + floats);
+    C10_CUDA_CHECK(cudaMemsetAsync(zero, 0, counters * sizeof(int), cur_stream()));
+  }
   b200::gemm_fp8_blockscale(a.data_ptr(), M, a.stride(0), w.data_ptr(), E, N, K, out.data_ptr(), out.stride(0),
                             a_scale.data_ptr<float>(), w_scale.data_ptr<float>(), ptr<int>(block_expert),
-                            ptr<int>(total_padded), grouped, dtype16(out), cur_stream(), status_ptr(a));
+                            ptr<int>(total_padded), ptr<int>(sorted_ids), (int)numel,
+                            floats > 0 ? scratch.data_ptr<float>() : nullptr, zero, sms, grouped, dtype16(out), cur_stream(), status_ptr(a));
 }
 
 // kind is taken from the operand dtype: int8 -> kind::i8, anything else one byte wide -> e4m3
@@ -674,6 +730,43 @@ void gdn_run(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const
   const int rc = b200::gdn_recurrent(p, (int)q.size(2), (int)v.size(2), dtype16(q), cur_stream());
   TORCH_CHECK(rc == 0, "gdn_recurrent: head sizes must be 128 and value heads a multiple of q/k heads");
 }
+void gdn_recurrent(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g,
+                   const Tensor& beta, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
+                   const optional<Tensor>& has_initial, double scale, bool l2norm) {
+  const int64_t n = v.numel() / (v.dim() == 3 && v.size(2) > 0 ? v.size(2) : 1);
+  TORCH_CHECK(g.is_contiguous() && beta.is_contiguous() && g.scalar_type() == at::kFloat && beta.scalar_type() == at::kFloat &&
+              g.numel() == n && beta.numel() == n);
+  b200::GdnParams p{};
+  p.g = g.data_ptr<float>(); p.beta = beta.data_ptr<float>();
+  gdn_run(out, state, q, k, v, query_start_loc, state_idx, has_initial, scale, l2norm, p);
+}
+// the same with g = -exp(a_log) softplus(a + dt_bias) and beta = sigmoid(b) of ba [T, Hq, 2 Hv / Hq] = (b.., a..) per key head
+void gdn_recurrent_ba(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& ba,
+                      const Tensor& a_log, const Tensor& dt_bias, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
+                      const optional<Tensor>& has_initial, double scale, bool l2norm) {
+  TORCH_CHECK(v.dim() == 3 && ba.dim() == 2 && ba.stride(1) == 1 && ba.size(0) == v.size(0) && ba.size(1) == 2 * v.size(1) &&
+              ba.scalar_type() == v.scalar_type());
+  TORCH_CHECK(a_log.is_contiguous() && dt_bias.is_contiguous() && a_log.scalar_type() == at::kFloat &&
+              dt_bias.scalar_type() == at::kFloat && a_log.numel() == v.size(1) && dt_bias.numel() == v.size(1));
+  b200::GdnParams p{};
+  p.ba = ba.data_ptr(); p.ba_stride = ba.stride(0);
+  p.a_log = a_log.data_ptr<float>(); p.dt_bias = dt_bias.data_ptr<float>();
+  gdn_run(out, state, q, k, v, query_start_loc, state_idx, has_initial, scale, l2norm, p);
+}
+// out [T, H * D] = norm(o) * silu(z), or o * sigmoid(z) without w; z [T, groups, at least rep * D]: head h in group h / rep
+void gated_head_norm(Tensor& out, const Tensor& o, const Tensor& z, const optional<Tensor>& w, int64_t dim, double eps) {
+  TORCH_CHECK(o.dim() == 2 && out.is_contiguous() && o.is_contiguous() && out.sizes() == o.sizes() && dim > 0 &&
+              o.size(1) % dim == 0);
+  TORCH_CHECK(z.dim() == 3 && z.stride(2) == 1 && z.size(0) == o.size(0) && z.size(1) * z.size(2) == o.size(1) &&
+              z.size(2) % dim == 0);
+  TORCH_CHECK(out.scalar_type() == o.scalar_type() && z.scalar_type() == o.scalar_type());
+  if (w.has_value()) TORCH_CHECK(w->is_contiguous() && w->numel() == dim && w->scalar_type() == o.scalar_type());
+  const c10::cuda::CUDAGuard guard(o.device());
+  const int rc = b200::gated_head_norm(out.data_ptr(), o.data_ptr(), z.data_ptr(), w.has_value() ? w->data_ptr() : nullptr,
+                                       o.size(0), (int)(o.size(1) / dim), (int)dim, (int)(z.size(2) / dim), z.stride(0),
+                                       z.stride(1), (float)eps, dtype16(o), cur_stream());
+  TORCH_CHECK(rc == 0, "gated_head_norm: heads of 64, 128 or 256 entries, rows on 16 bytes");
+}
 
 
 // TurboQuant cache: uint8 [blocks, block_size, kv_heads, slot_bytes]; k, v [T, kv_heads * 128] (any row pitch)
@@ -729,43 +822,6 @@ void tq_decode(Tensor& out, const Tensor& q, const Tensor& cache, const Tensor& 
                                  seq_lens.data_ptr<int>(), (int)B, (int)hq, (int)hkv, (int)cache.size(1), cache.size(0),
                                  (int)splits, (float)scale, (int)kbits, (int)vbits, nc, dtype16(q), cur_stream());
   TORCH_CHECK(rc == 0, "tq_decode: unsupported format or GQA group (1, 2, 4, 8)");
-}
-void gdn_recurrent(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g,
-                   const Tensor& beta, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
-                   const optional<Tensor>& has_initial, double scale, bool l2norm) {
-  const int64_t n = v.numel() / (v.dim() == 3 && v.size(2) > 0 ? v.size(2) : 1);
-  TORCH_CHECK(g.is_contiguous() && beta.is_contiguous() && g.scalar_type() == at::kFloat && beta.scalar_type() == at::kFloat &&
-              g.numel() == n && beta.numel() == n);
-  b200::GdnParams p{};
-  p.g = g.data_ptr<float>(); p.beta = beta.data_ptr<float>();
-  gdn_run(out, state, q, k, v, query_start_loc, state_idx, has_initial, scale, l2norm, p);
-}
-// the same with g = -exp(a_log) softplus(a + dt_bias) and beta = sigmoid(b) of ba [T, Hq, 2 Hv / Hq] = (b.., a..) per key head
-void gdn_recurrent_ba(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& ba,
-                      const Tensor& a_log, const Tensor& dt_bias, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
-                      const optional<Tensor>& has_initial, double scale, bool l2norm) {
-  TORCH_CHECK(v.dim() == 3 && ba.dim() == 2 && ba.stride(1) == 1 && ba.size(0) == v.size(0) && ba.size(1) == 2 * v.size(1) &&
-              ba.scalar_type() == v.scalar_type());
-  TORCH_CHECK(a_log.is_contiguous() && dt_bias.is_contiguous() && a_log.scalar_type() == at::kFloat &&
-              dt_bias.scalar_type() == at::kFloat && a_log.numel() == v.size(1) && dt_bias.numel() == v.size(1));
-  b200::GdnParams p{};
-  p.ba = ba.data_ptr(); p.ba_stride = ba.stride(0);
-  p.a_log = a_log.data_ptr<float>(); p.dt_bias = dt_bias.data_ptr<float>();
-  gdn_run(out, state, q, k, v, query_start_loc, state_idx, has_initial, scale, l2norm, p);
-}
-// out [T, H * D] = norm(o) * silu(z), or o * sigmoid(z) without w; z [T, groups, at least rep * D]: head h in group h / rep
-void gated_head_norm(Tensor& out, const Tensor& o, const Tensor& z, const optional<Tensor>& w, int64_t dim, double eps) {
-  TORCH_CHECK(o.dim() == 2 && out.is_contiguous() && o.is_contiguous() && out.sizes() == o.sizes() && dim > 0 &&
-              o.size(1) % dim == 0);
-  TORCH_CHECK(z.dim() == 3 && z.stride(2) == 1 && z.size(0) == o.size(0) && z.size(1) * z.size(2) == o.size(1) &&
-              z.size(2) % dim == 0);
-  TORCH_CHECK(out.scalar_type() == o.scalar_type() && z.scalar_type() == o.scalar_type());
-  if (w.has_value()) TORCH_CHECK(w->is_contiguous() && w->numel() == dim && w->scalar_type() == o.scalar_type());
-  const c10::cuda::CUDAGuard guard(o.device());
-  const int rc = b200::gated_head_norm(out.data_ptr(), o.data_ptr(), z.data_ptr(), w.has_value() ? w->data_ptr() : nullptr,
-                                       o.size(0), (int)(o.size(1) / dim), (int)dim, (int)(z.size(2) / dim), z.stride(0),
-                                       z.stride(1), (float)eps, dtype16(o), cur_stream());
-  TORCH_CHECK(rc == 0, "gated_head_norm: heads of 64, 128 or 256 entries, rows on 16 bytes");
 }
 
 // o [T, H, 512] -> out [G, T, (H / G) * 512] with the rope dims rotated back
@@ -961,6 +1017,10 @@ TORCH_LIBRARY_FRAGMENT(b200, m) {
   m.def("moe_a2a_combine(Tensor(a!) out, Tensor y, Tensor topk_ids, Tensor? shared_out, Tensor ptrs, int ep, int rank, int experts_per_rank, int cap, Tensor(b!) local_sync, int wait_cycles) -> ()", &moe_a2a_combine);
   m.def("v4_qnorm_rope_kv_insert(Tensor(a!) q_out, Tensor(b!) cache, Tensor q, Tensor kv, Tensor slot_mapping, Tensor positions, Tensor cos_sin, float eps, int block_size) -> ()", &v4_qnorm_rope_kv_insert);
   m.def("v4_gather_dequant(Tensor(a!) dst, Tensor cache, Tensor slots, int block_size) -> ()", &v4_gather_dequant);
+  m.def("mla_rope_insert(Tensor(a!) q, Tensor(b!) qa, Tensor(c!) kv_c, Tensor(d!) k_pe, Tensor(e!) cache, Tensor kv, Tensor norm_w, Tensor positions, Tensor cos_sin, Tensor slots, float eps) -> ()", &mla_rope_insert);
+  m.def("mla_expand_keys(Tensor(a!) out, Tensor kv, Tensor k_pe, int nope) -> ()", &mla_expand_keys);
+  m.def("gdn_recurrent_ba(Tensor(a!) out, Tensor(b!) state, Tensor q, Tensor k, Tensor v, Tensor ba, Tensor a_log, Tensor dt_bias, Tensor query_start_loc, Tensor? state_idx, Tensor? has_initial, float scale, bool l2norm) -> ()", &gdn_recurrent_ba);
+  m.def("gated_head_norm(Tensor(a!) out, Tensor o, Tensor z, Tensor? w, int dim, float eps) -> ()", &gated_head_norm);
   m.def("gdn_recurrent(Tensor(a!) out, Tensor(b!) state, Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, Tensor query_start_loc, Tensor? state_idx, Tensor? has_initial, float scale, bool l2norm) -> ()", &gdn_recurrent);
   m.def("tq_slot_bytes(int kbits, int vbits) -> int", &tq_slot_bytes);
   m.def("tq_store(Tensor(a!) cache, Tensor k, Tensor v, Tensor slot_mapping, int kbits, int vbits, bool nc) -> ()", &tq_store);
@@ -987,7 +1047,7 @@ TORCH_LIBRARY_FRAGMENT(b200, m) {
   m.def("scaled_fp8_quant(Tensor(a!) q, Tensor(b!) scale, Tensor x, int mode, float scale_ub) -> ()", &scaled_fp8_quant);
   m.def("scaled_int8_quant(Tensor(a!) q, Tensor(b!) scale, Tensor(c!)? azp, Tensor x, int mode) -> ()", &scaled_int8_quant);
   m.def("merge_attn_states(Tensor(a!) out, Tensor(b!)? out_lse, Tensor p_out, Tensor p_lse, Tensor s_out, Tensor s_lse) -> ()", &merge_attn_states);
-  m.def("gemm_fp8_blockscale(Tensor(a!) out, Tensor a, Tensor a_scale, Tensor w, Tensor w_scale, Tensor? block_expert, Tensor? total_padded) -> ()", &gemm_fp8_blockscale);
+  m.def("gemm_fp8_blockscale(Tensor(a!) out, Tensor a, Tensor a_scale, Tensor w, Tensor w_scale, Tensor? block_expert, Tensor? total_padded, Tensor? sorted_ids=None, int numel=0) -> ()", &gemm_fp8_blockscale);
   m.def("scaled_mm(Tensor(a!) out, Tensor a, Tensor w, Tensor a_scale, Tensor w_scale, Tensor? azp, Tensor? azp_adj, Tensor? bias, Tensor? block_expert, Tensor? total_padded) -> ()", &scaled_mm);
   m.def("wna16_gemm(Tensor(a!) out, Tensor a, Tensor q, Tensor scales, Tensor? zeros, int bits, int group, Tensor? bias, Tensor? block_expert, Tensor? total_padded, int token_tile, int epi) -> ()", &wna16_gemm);
   m.def("indexer_logits(Tensor(a!) logits, Tensor q, Tensor w, Tensor cache, Tensor block_table, Tensor seq_lens, Tensor query_start_loc, int block_size, int max_len, bool int8, int max_query_len, int impl) -> ()", &indexer_logits);
@@ -1017,8 +1077,6 @@ TORCH_LIBRARY_FRAGMENT(b200, m) {
   m.def("rms_norm(Tensor(a!) out, Tensor x, Tensor weight, float eps, bool gemma) -> ()", &rms_norm);
   m.def("fused_add_rms_norm(Tensor(a!) x, Tensor(b!) residual, Tensor weight, float eps, bool gemma) -> ()",
         &fused_add_rms_norm);
-  m.def("gdn_recurrent_ba(Tensor(a!) out, Tensor(b!) state, Tensor q, Tensor k, Tensor v, Tensor ba, Tensor a_log, Tensor dt_bias, Tensor query_start_loc, Tensor? state_idx, Tensor? has_initial, float scale, bool l2norm) -> ()", &gdn_recurrent_ba);
-  m.def("gated_head_norm(Tensor(a!) out, Tensor o, Tensor z, Tensor? w, int dim, float eps) -> ()", &gated_head_norm);
   m.def("head_rms_norm(Tensor(a!) x, Tensor weight, float eps, int heads, int head_dim) -> ()", &head_rms_norm);
   m.def(
       "rms_norm_quant(Tensor(a!) out_q, Tensor(b!)? scale_out, Tensor? scale_in, Tensor x, Tensor(c!)? residual, "
@@ -1039,7 +1097,7 @@ TORCH_LIBRARY_FRAGMENT(b200, m) {
   m.def("activation(Tensor(a!) out, Tensor x, int act, float p0) -> ()", &activation);
   m.def(
       "act_and_mul_quant(Tensor(a!) out_q, Tensor(b!)? scale_out, Tensor? scale_in, Tensor x, int act, float p0, "
-      "float p1, int group, bool ue8m0) -> ()",
+      "float p1, int group, bool ue8m0, Tensor? sorted_ids=None, int numel=0) -> ()",
       &act_and_mul_quant);
   m.def("weak_ref_tensor(Tensor input) -> Tensor", &weak_ref_tensor);
 }

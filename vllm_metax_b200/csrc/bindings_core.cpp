@@ -173,9 +173,29 @@ void moe_align(Tensor& sorted_ids, Tensor& block_expert, Tensor& total_padded, c
   TORCH_CHECK(topk_ids.scalar_type() == at::kInt && topk_ids.is_contiguous());
   TORCH_CHECK(sorted_ids.numel() % block == 0 && block_expert.numel() >= sorted_ids.numel() / block);
   const c10::cuda::CUDAGuard guard(topk_ids.device());
+  const int64_t ints = b200::moe_align_scratch_ints((int)topk_ids.numel(), (int)experts);
+  Tensor scratch;
+  if (ints > 0) scratch = at::empty({ints}, topk_ids.options());
   b200::moe_align(sorted_ids.data_ptr<int>(), block_expert.data_ptr<int>(), total_padded.data_ptr<int>(),
-                  ptr<int>(inv_pos), topk_ids.data_ptr<int>(), ptr<int>(expert_map), topk_ids.numel(), experts, block,
-                  sorted_ids.numel(), cur_stream());
+                  ptr<int>(inv_pos), topk_ids.data_ptr<int>(), ptr<int>(expert_map), ints > 0 ? scratch.data_ptr<int>() : nullptr,
+                  topk_ids.numel(), experts, block, sorted_ids.numel(), cur_stream());
+}
+// out[inv_pos[t, k]] = x[t] (times weights[t, k]); with scales: as e4m3 with one per 128 entries.  Other rows of out stay as they are
+bool moe_scatter(Tensor& out, const optional<Tensor>& scales, const Tensor& x, const Tensor& inv_pos, int64_t topk,
+                 const optional<Tensor>& weights) {
+  TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && out.is_contiguous() && out.dim() == 2 && out.size(1) == x.size(1));
+  TORCH_CHECK(inv_pos.is_contiguous() && inv_pos.scalar_type() == at::kInt && inv_pos.numel() == x.size(0) * topk);
+  if (scales.has_value()) {
+    TORCH_CHECK(scales->is_contiguous() && scales->scalar_type() == at::kFloat && x.size(1) % 128 == 0 && out.element_size() == 1 &&
+                scales->numel() == out.size(0) * (x.size(1) / 128) && !weights.has_value());
+  } else {
+    TORCH_CHECK(out.scalar_type() == x.scalar_type());
+  }
+  if (weights.has_value())
+    TORCH_CHECK(weights->is_contiguous() && weights->scalar_type() == at::kFloat && weights->numel() == inv_pos.numel());
+  const c10::cuda::CUDAGuard guard(x.device());
+  return b200::moe_scatter(out.data_ptr(), ptr<float>(scales), x.data_ptr(), inv_pos.data_ptr<int>(), ptr<float>(weights),
+                           (int)x.size(0), (int)topk, (int)x.size(1), dtype_code(x), cur_stream()) == 0;
 }
 
 void moe_gather(Tensor& out, const Tensor& x, const Tensor& sorted_ids, const Tensor& total_padded, int64_t topk,
@@ -468,6 +488,7 @@ TORCH_LIBRARY(b200, m) {
   m.def("topk_gating(Tensor(a!) weights, Tensor(b!) ids, Tensor gating, Tensor? bias, int mode, bool renorm, float scale) -> ()", &topk_gating);
   m.def("grouped_topk(Tensor(a!) weights, Tensor(b!) ids, Tensor gating, Tensor? bias, int n_group, int topk_group, bool sigmoid, bool renorm, float scale) -> ()", &grouped_topk);
   m.def("moe_align(Tensor(a!) sorted_ids, Tensor(b!) block_expert, Tensor(c!) total_padded, Tensor(d!)? inv_pos, Tensor topk_ids, Tensor? expert_map, int experts, int block) -> ()", &moe_align);
+  m.def("moe_scatter(Tensor(a!) out, Tensor(b!)? scales, Tensor x, Tensor inv_pos, int topk, Tensor? weights=None) -> bool", &moe_scatter);
   m.def("moe_gather(Tensor(a!) out, Tensor x, Tensor sorted_ids, Tensor total_padded, int topk, Tensor? weights=None) -> ()", &moe_gather);
   m.def(
       "moe_combine(Tensor(a!) out, Tensor y, Tensor weights, Tensor inv_pos, Tensor? shared, Tensor? expert_ids=None, "

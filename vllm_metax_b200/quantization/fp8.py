@@ -78,11 +78,12 @@ class Fp8MoEMethod:
         topk = topk_ids.shape[1]
         sorted_ids, block_expert, total, inv = ops.moe_align_block_size(topk_ids, 128, layer.num_local,
                                                                         layer.expert_map, want_inverse=True)
-        a = ops.moe_gather(x, sorted_ids, total, topk)
-        aq, a_s = ops.per_token_group_quant_fp8(a, BLOCK)
-        h = ops.fp8_block_scaled_mm(aq, a_s, layer.w13_weight, layer.w13_weight_scale_inv, x.dtype, block_expert, total)
-        hq, h_s = ops.silu_and_mul_per_block_quant(h, BLOCK)
-        y = ops.fp8_block_scaled_mm(hq, h_s, layer.w2_weight, layer.w2_weight_scale_inv, x.dtype, block_expert, total)
+        aq, a_s = ops.moe_scatter_fp8(x, inv, sorted_ids, total, topk)
+        h = ops.fp8_block_scaled_mm(aq, a_s, layer.w13_weight, layer.w13_weight_scale_inv, x.dtype, block_expert, total,
+                                    sorted_ids, inv.numel())
+        hq, h_s = ops.silu_and_mul_per_block_quant(h, BLOCK, sorted_ids=sorted_ids, numel=inv.numel())
+        y = ops.fp8_block_scaled_mm(hq, h_s, layer.w2_weight, layer.w2_weight_scale_inv, x.dtype, block_expert, total,
+                                    sorted_ids, inv.numel())
         return ops.moe_combine(y, topk_weights, inv, T, shared_out)
 
 
