@@ -292,3 +292,39 @@ def test_mla_tcgen05_tiling_arithmetic_cpu():
     assert 128 * 576 * 2 + 2 * 32 * 576 * 2 + 10 * 8 + 16 + 1024 <= 232448
     # tensor memory: two score buffers of 32 fp32 columns and 256 output columns fit 512 columns
     assert 2 * 32 + 256 <= 512
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,H,absorbed,pitch", [(1, 3, 1, 576), (70, 16, 5, 2112), (600, 33, 0, 584)])
+def test_mla_rope_insert_and_keys(dtype, T, H, absorbed, pitch):
+    """The one launch between a latent layer's projections and its attention against the separate ones, bit for bit but for the
+    norm's sum (one unit of its rounding): few and many tokens, heads that do not divide, rows without a slot."""
+    from vllm_metax_b200 import _custom_ops as ops
+
+    g = torch.Generator().manual_seed(T)
+    q = torch.randn(T, H, 192, generator=g).to(dtype).cuda()
+    kv = torch.randn(T, pitch, generator=g).to(dtype).cuda()[:, pitch - 576:]
+    w = torch.randn(512, generator=g).to(dtype).cuda()
+    cs = torch.randn(900, 64, generator=g).cuda()
+    pos = torch.randint(0, 900, (T,), generator=g).cuda()
+    slots = torch.randperm(T + 9, generator=g)[:T].cuda()
+    slots[::7] = -1
+    cache = torch.zeros(-(-(T + 9) // 16), 16, 576, dtype=dtype, device="cuda")
+    want_cache = cache.clone()
+    kv_c = ops.rms_norm(kv[:, :512].contiguous(), w, 1e-6)
+    k_pe, q_pe = kv[:, 512:].contiguous(), q[..., 128:].reshape(T, -1).contiguous()
+    ops.rotary_embedding(pos, q_pe, k_pe, 64, cs, False)
+    ops.concat_and_cache_mla(kv_c, k_pe, want_cache, slots)
+    q2, qa = q.clone(), torch.zeros(absorbed, H, 576, dtype=dtype, device="cuda")
+    c2, p2 = torch.empty_like(kv_c), torch.empty_like(k_pe)
+    assert ops.mla_rope_insert(q2, qa, c2, p2, cache, kv, w, pos, cs, slots, 1e-6)
+    tol = dict(rtol=2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10, atol=1e-6)
+    assert torch.equal(q2[..., :128], q[..., :128]) and torch.equal(qa[..., 512:], q2[:absorbed, :, 128:])
+    torch.testing.assert_close(q2[..., 128:].reshape(T, -1), q_pe, **tol)
+    torch.testing.assert_close(p2, k_pe, **tol)
+    torch.testing.assert_close(c2, kv_c, **tol)
+    torch.testing.assert_close(cache, want_cache, **tol)
+    up = torch.randn(T, H, 256, generator=g).to(dtype).cuda()
+    assert torch.equal(ops.mla_expand_keys(up, p2, 128), torch.cat([up[..., :128], p2[:, None].expand(-1, H, -1)], -1))
+    ops.check_kernel_status(0)

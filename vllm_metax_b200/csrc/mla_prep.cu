@@ -6,7 +6,8 @@
 //                     place of the absorbed queries
 //   mla_expand_keys   keys of a prompt: a head's own part from the up-projection beside the shared rotated one
 //
-// Both are bound by their bytes: 16 bytes a thread and access.  The seven launches they replace took MLA_OLD, they MLA_NEW.
+// Both are bound by their bytes: 16 bytes a thread and access.  What they replace (a norm, a
+// rotation, the cache write and copies) took 54 us for 64 decode rows and 590 us for 1836 rows of prompts with 128 heads; they 4 and 55.
 #include "common.cuh"
 #include "ops.h"
 

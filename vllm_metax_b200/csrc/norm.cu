@@ -232,13 +232,16 @@ static void rms_norm_t(void* out, void* x, void* residual, const void* weight, f
                       ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(x) |
                         reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(weight)) & 15) == 0;
   const int vpt = hidden / 1024;
-  if (vec_ok && (vpt == 1 || vpt == 2 || vpt == 4 || vpt == 8)) {
+  if (vec_ok && vpt <= 8) {
 #define REG(ADD, V)                                                                                                \
   rms_norm_reg_kernel<T, ADD, V><<<tokens, 128, 0, stream>>>((T*)out, (T*)x, (T*)residual, (const T*)weight, eps,  \
                                                              hidden, x_stride, out_stride, mode)
 #define REGV(ADD)                                                                                                  \
   do {                                                                                                             \
-    if (vpt == 1) REG(ADD, 1); else if (vpt == 2) REG(ADD, 2); else if (vpt == 4) REG(ADD, 4); else REG(ADD, 8);   \
+    switch (vpt) {                                                                                                 \
+      case 1: REG(ADD, 1); break; case 2: REG(ADD, 2); break; case 3: REG(ADD, 3); break; case 4: REG(ADD, 4); break; \
+      case 5: REG(ADD, 5); break; case 6: REG(ADD, 6); break; case 7: REG(ADD, 7); break; default: REG(ADD, 8);    \
+    }                                                                                                              \
   } while (0)
     if (residual) REGV(true); else REGV(false);
 #undef REGV

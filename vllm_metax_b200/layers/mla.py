@@ -70,16 +70,36 @@ class MLAAttention(nn.Module):
         self.W_UK.copy_(w[:, : self.qk_nope])
         self.W_UV.copy_(w[:, self.qk_nope:].transpose(1, 2))
 
+    def rope_insert(self, positions, q, kv, norm, rope, sparse: bool):
+        """Everything between the projections and the attention in one launch: ``q [T, H, nope+rope]`` rotated in place,
+        ``kv [T, 576]`` (latent, shared key part) normed, rotated and written to the cache.  Returns ``(kv_c, k_pe, qa)`` for
+        ``forward``, or None where another path applies (other caches, context parallel steps, CPU)."""
+        ctx = get_forward_context()
+        md, cache = ctx.attn_metadata, ctx.kv_caches[self.layer_idx]["mla"]
+        if not q.is_cuda or cache.dtype != q.dtype or q.dtype == torch.float32 or rope.is_neox \
+                or "pcp_slots_all" in md.extra or "dcp_ctx_lens" in md.extra or kv.stride(0) % 8 or kv.data_ptr() % 16:
+            return None
+        T, H = q.shape[0], self.num_heads
+        pure = md.extra.get("prefill_no_context", False) and not sparse
+        qa = torch.empty(md.num_decode_tokens if pure else T, H, self.kv_lora + self.qk_rope, dtype=q.dtype, device=q.device)
+        kv_c = torch.empty(T, self.kv_lora, dtype=q.dtype, device=q.device)
+        k_pe = torch.empty(T, self.qk_rope, dtype=q.dtype, device=q.device)
+        done = ops.mla_rope_insert(q, qa, kv_c, k_pe, cache, kv, norm.weight, positions, rope.cos_sin_cache, md.slot_mapping,
+                                   norm.eps)
+        return (kv_c, k_pe, qa) if done else None
+
     def forward(self, q: torch.Tensor, kv_c: torch.Tensor, k_pe: torch.Tensor, kv_b_proj=None,
-                topk_indices: Optional[torch.Tensor] = None) -> torch.Tensor:
+                topk_indices: Optional[torch.Tensor] = None, qa: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``q [T, H, nope+rope]`` (rope already applied), ``kv_c [T, 512]`` normed, ``k_pe [T, 64]`` roped.
-        Returns ``[T, H * v_head]``."""
+        Returns ``[T, H * v_head]``.  ``qa``: of :meth:`rope_insert`, which has filled the cache."""
         ctx = get_forward_context()
         md = ctx.attn_metadata
         cache = ctx.kv_caches[self.layer_idx]["mla"]
         T, H = q.shape[0], self.num_heads
         pcp_slots = md.extra.get("pcp_slots_all")
-        if pcp_slots is not None:
+        if qa is not None:
+            pass
+        elif pcp_slots is not None:
             # prefill context parallel: this copy computed a slice of every chunk; the copies exchange their latent
             # rows and each writes all of them into its own (replicated) cache, after which the slice is an ordinary
             # request of length "end of the slice" for the kernels below - parallel/pcp.py
@@ -98,18 +118,21 @@ class MLAAttention(nn.Module):
         mqa_end = ndt if pure_prefill else T
         if mqa_end > 0:
             n_req = nd if pure_prefill else md.num_reqs
-            qa = self._absorb_q(q[:mqa_end])
+            if qa is None:
+                qa = self._absorb_q(q[:mqa_end])
+            else:                                       # beside the rotated part, which is there
+                torch.bmm(q[:mqa_end, :, : self.qk_nope].transpose(0, 1), self.W_UK,
+                          out=qa[..., : self.kv_lora].transpose(0, 1))
             lat = ops.mla_decode(qa, cache, md.block_table[:n_req], md.seq_lens[:n_req], self.scale,
                                  query_start_loc=md.query_start_loc[:n_req + 1],
                                  topk_indices=None if topk_indices is None else topk_indices[:mqa_end],
                                  max_seq_len=md.max_seq_len)
-            out[:mqa_end] = torch.bmm(lat.transpose(0, 1), self.W_UV).transpose(0, 1)
+            torch.bmm(lat.transpose(0, 1), self.W_UV, out=out[:mqa_end].transpose(0, 1))
         if pure_prefill and T > ndt:
             kv = kv_b_proj(kv_c[ndt:]).view(T - ndt, H, self.qk_nope + self.v_head)
-            k = torch.cat([kv[..., : self.qk_nope], k_pe[ndt:, None, :].expand(-1, H, -1)], dim=-1).contiguous()
-            v = kv[..., self.qk_nope:].contiguous()
+            k = ops.mla_expand_keys(kv, k_pe[ndt:], self.qk_nope)
             qsl = md.prefill_query_start_loc
-            ops.varlen_attention(q[ndt:].contiguous(), k, v, qsl, qsl, self.scale, out=out[ndt:],
+            ops.varlen_attention(q[ndt:].contiguous(), k, kv[..., self.qk_nope:], qsl, qsl, self.scale, out=out[ndt:],
                                  max_q_len=md.max_prefill_query_len, causal=True)
         return out.reshape(T, H * self.v_head)
 

@@ -142,18 +142,22 @@ class DeepseekV2MLAAttention(nn.Module):
         q_lora = None
         if self.q_lora:
             qkv = self.fused_qkv_a_proj(h)
-            q_lora = self.q_a_layernorm(qkv[:, : self.q_lora].contiguous())
+            q_lora = qkv[:, : self.q_lora]                # (the norm reads wider rows where they start on 16 bytes)
+            q_lora = self.q_a_layernorm(q_lora if qkv.stride(0) % 8 == 0 else q_lora.contiguous())
             kv_a = qkv[:, self.q_lora:]
             q = self.q_b_proj(q_lora)
         else:
             q = self.q_proj(h)
             kv_a = self.kv_a_proj_with_mqa(h)
-        kv_c = self.kv_a_layernorm(kv_a[:, : self.kv_lora].contiguous())
-        k_pe = kv_a[:, self.kv_lora:].contiguous()
         q = q.view(T, self.num_heads, self.qk_dim)
-        q_pe = q[..., self.nope:].reshape(T, -1).contiguous()
-        ops.rotary_embedding(positions, q_pe, k_pe, self.rope_dim, self.rope.cos_sin_cache, False)
-        q = torch.cat([q[..., : self.nope], q_pe.view(T, self.num_heads, self.rope_dim)], dim=-1)
+        kv_c, k_pe, qa = self.attn.rope_insert(positions, q, kv_a, self.kv_a_layernorm, self.rope, self.indexer is not None) \
+            or (None, None, None)
+        if qa is None:
+            kv_c = self.kv_a_layernorm(kv_a[:, : self.kv_lora].contiguous())
+            k_pe = kv_a[:, self.kv_lora:].contiguous()
+            q_pe = q[..., self.nope:].reshape(T, -1).contiguous()
+            ops.rotary_embedding(positions, q_pe, k_pe, self.rope_dim, self.rope.cos_sin_cache, False)
+            q = torch.cat([q[..., : self.nope], q_pe.view(T, self.num_heads, self.rope_dim)], dim=-1)
         topk_idx = None
         if self.indexer is not None:
             from ..attention.metadata import get_forward_context
@@ -161,7 +165,7 @@ class DeepseekV2MLAAttention(nn.Module):
             ctx = get_forward_context()
             caches = ctx.kv_caches[self.layer_idx]
             topk_idx = self.indexer(h, q_lora, positions, self.rope, caches["idx"], ctx.attn_metadata.block_size)
-        a = self.attn(q, kv_c, k_pe, self.kv_b_proj, topk_idx)
+        a = self.attn(q, kv_c, k_pe, self.kv_b_proj, topk_idx, qa)
         return self.o_proj(a)
 
 
