@@ -503,3 +503,58 @@ def test_alibi_bias_in_prefill_and_decode(D):
     got_d = ops.paged_attention_decode(q.cuda(), cache.cuda(), bt.cuda(), sl.cuda(), D ** -0.5, query_start_loc=qsl.cuda(),
                                        max_q_len=max(qlens), max_seq_len=max(lens), alibi_slopes=slopes.cuda())
     torch.testing.assert_close(got_d.float().cpu(), want, rtol=3e-2, atol=3e-2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens", [[1], [900], [0, 1, 64, 65, 0, 3], [17] * 300, [5000, 3, 129, 1, 700, 64], [2048 - 13 * i for i in range(48)]])
+@pytest.mark.parametrize("Hq,Hkv,D,kind", [(32, 8, 128, 0), (64, 8, 128, 1), (16, 2, 256, 0), (24, 2, 128, 0), (32, 2, 128, 1), (6, 6, 64, 0),
+                                           (5, 1, 80, 0)])
+def test_decode_shared_out_evenly(lens, Hq, Hkv, D, kind, kernel_status_ok):
+    """One token per sequence: ranges that end inside sequences and hold many, sequences cut into many parts, empty ones, fewer
+    units than CTAs, windows, sinks, capped scores; 16-bit and int8 caches, 8 and 16 rows of heads, padded head sizes; a scratch
+    that is kept, whose counters are zero again after each call."""
+    g = torch.Generator().manual_seed(len(lens) + D)
+    bs, B = 64, len(lens)
+    nb = [-(-n // bs) for n in lens]
+    table = torch.zeros(B, max(nb) + 1, dtype=torch.int32)
+    perm, at = torch.randperm(sum(nb) + 1, generator=g), 0
+    for i, n in enumerate(nb):
+        table[i, :n] = perm[at: at + n]
+        at += n
+    q = torch.randn(B, Hq, D, generator=g).bfloat16()
+    sl = torch.tensor(lens, dtype=torch.int32)
+    scales = None
+    if kind:
+        cache = torch.randint(-127, 128, (sum(nb) + 1, 2, bs, Hkv, D), generator=g, dtype=torch.int8)
+        scales = torch.rand(sum(nb) + 1, 2, bs, Hkv, generator=g) * 0.012 + 0.004
+        deq = cache.float() * scales[..., None]
+    else:
+        cache = torch.randn(sum(nb) + 1, 2, bs, Hkv, D, generator=g).bfloat16()
+        deq = cache.float()
+    sinks = torch.randn(Hq, generator=g)
+    scratch = ops.decode_scratch(Hq, Hkv, D, "cuda")
+    for kw in (dict(), dict(window=100, softcap=20.0), dict(sinks=sinks), dict(scratch=scratch), dict(scratch=scratch, window=70)):
+        lse = None if kw.get("sinks") is not None else torch.empty(Hq, B, device="cuda")
+        kc = {k: v.cuda() if torch.is_tensor(v) else v for k, v in kw.items()}
+        got = ops.paged_attention_decode(q.cuda(), cache.cuda(), table.cuda(), sl.cuda(), D ** -0.5, kv_scales=None if scales is None else scales.cuda(),
+                                         lse_out=lse, max_seq_len=max(lens), **kc).float().cpu()
+        assert not bool(scratch[:16384].any())
+        for i, n in enumerate(lens):
+            if n == 0:
+                assert float(got[i].abs().max()) == 0.0
+                continue
+            rows = deq[table[i, : nb[i]].long()]
+            k, v = (rows[:, j].reshape(-1, Hkv, D)[:n].repeat_interleave(Hq // Hkv, 1) for j in (0, 1))
+            s = torch.einsum("hd,nhd->hn", q[i].float(), k) * D ** -0.5
+            if kw.get("softcap"):
+                s = kw["softcap"] * torch.tanh(s / kw["softcap"])
+            if kw.get("window"):
+                s[:, : max(0, n - kw["window"])] = float("-inf")
+            full = torch.cat([s, sinks[:, None]], 1) if kw.get("sinks") is not None else s
+            p = full.softmax(-1)[:, :n]
+            want = torch.einsum("hn,nhd->hd", p, v)
+            # weights are rounded to bf16 (2^-9 each, at random signs), the result once more
+            bound = 2.0 ** -8 * want.abs() + 2.0 ** -8 * torch.einsum("hn,nhd->hd", p, v.abs())
+            assert bool(((got[i] - want).abs() <= bound + 1e-5).all()), (i, n, float((got[i] - want).abs().max()))
+            if lse is not None:
+                torch.testing.assert_close(lse[:, i].cpu(), full.logsumexp(-1), rtol=1e-4, atol=2e-3)

@@ -35,7 +35,7 @@ CUMEM_LIB = ROOT / "cumem_allocator.so"
 CORE_UNITS = ("attn_prefill_pingpong", "attn_prefill_tcgen05", "gemm_grouped_tcgen05", "gemm_pair_tcgen05", "gemm_simt",
               "gemm_splitk_tcgen05", "gemm_streamk_tcgen05", "gemm_tcgen05", "moe", "residual_norm", "rope_angles", "sampling")
 UNIT_SETS = {
-    "gqa": ("attn_decode", "head_norm_rope", "paged_attn_simt"),
+    "gqa": ("attn_decode", "attn_decode_stream", "head_norm_rope", "paged_attn_simt"),
     "hybrid": ("residual_conv", "rglru"),
     "latent": ("fused_misc", "latent_attn", "mla_decode", "mla_decode_tcgen05"),
     "recurrent": ("causal_conv1d", "channel_delta", "gla", "prenorm"),

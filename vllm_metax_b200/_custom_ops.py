@@ -454,17 +454,26 @@ def decode_num_splits(batch: int, num_kv_heads: int, max_seq_len: int, row_tiles
     return max(1, min(want, max(1, max_seq_len // 256), 32))
 
 
+def decode_scratch(q_heads: int, kv_heads: int, head_size: int, device, sms: int = 148) -> torch.Tensor:
+    """Zeroed scratch for ``paged_attention_decode``, which leaves its counters zero: one for the steps that follow one another in a
+    stream (captured graphs).  Too small a one is not used."""
+    rows = 8 if q_heads <= 8 * kv_heads else 16
+    head = 64 if head_size <= 64 else 128 if head_size <= 128 else 256
+    return torch.zeros(16384 + 3 * sms * 2 * (rows * head + 2 * rows), dtype=torch.float32, device=device)
+
+
 def paged_attention_decode(q, kv_cache, block_table, seq_lens, scale, *, out=None, kv_scales=None,
                            query_start_loc=None, max_q_len: int = 1, window: int = -1, softcap: float = 0.0,
                            sinks=None, lse_out=None, num_splits: int = 0, max_seq_len: int = 0, k_scale=1.0,
                            v_scale=1.0, causal=True, workspace=None, alibi_slopes=None, distance_bias=None, gate=None,
-                           out_scale: float = 1.0, chunk: int = 0, sigmoid_shift=None):
+                           out_scale: float = 1.0, chunk: int = 0, sigmoid_shift=None, scratch=None):
     """Decode attention over the paged cache; ``q [T, Hq, D]``.  ``alibi_slopes [Hq]`` (f32) adds
     ``slope * (kv position - query position)`` to the scores, ``distance_bias [Hq, L]`` (f32) the entry of the distance (the
     last one from L - 1 on).  ``chunk`` > 0: a position sees its own chunk of that many, counted from 0.  ``sigmoid_shift [Hq]``
     (f32): no softmax, a key's weight is ``sigmoid(score + shift)``.  The result is multiplied by ``out_scale`` and, with ``gate
     [T, Hq * Dv]`` or ``[T, Hq]`` (rows may be part of wider ones), by its sigmoid; ``out``'s token rows may be part of wider
-    ones too.  ``kv_cache``: the 5-D cache or a pair of ``kv_views``.  fp32 caches and 16-bit heads wider than 256 run on the
+    ones too.  ``scratch``: of ``decode_scratch``, for callers that keep one across steps of one stream.  ``kv_cache``: the 5-D
+    cache or a pair of ``kv_views``.  fp32 caches and 16-bit heads wider than 256 run on the
     CUDA cores."""
     if _use_cuda(q):
         k, v = kv_views(kv_cache)
@@ -483,7 +492,7 @@ def paged_attention_decode(q, kv_cache, block_table, seq_lens, scale, *, out=Non
         torch.ops.b200.paged_attention_decode(out, q, k, v, kv_scales, block_table, seq_lens, query_start_loc,
                                               scale, window, softcap, sinks, lse_out, ws, num_splits, B, max_q_len,
                                               k_scale, v_scale, causal, alibi_slopes, distance_bias, gate, out_scale,
-                                              chunk, sigmoid_shift)
+                                              chunk, sigmoid_shift, not batch_invariant(), scratch)
         return out
     B = seq_lens.shape[0]
     qsl = query_start_loc if query_start_loc is not None else torch.arange(B + 1, dtype=torch.int32, device=q.device)

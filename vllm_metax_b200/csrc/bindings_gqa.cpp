@@ -20,7 +20,7 @@ void paged_attention_decode(Tensor& out, const Tensor& q, const Tensor& k_cache,
                             const optional<Tensor>& workspace, int64_t num_splits, int64_t batch, int64_t max_q_len,
                             double k_scale, double v_scale, bool causal, const optional<Tensor>& alibi_slopes,
                             const optional<Tensor>& distance_bias, const optional<Tensor>& gate, double out_scale, int64_t chunk,
-                            const optional<Tensor>& sigmoid_shift) {
+                            const optional<Tensor>& sigmoid_shift, bool stream, const optional<Tensor>& scratch) {
   TORCH_CHECK(q.dim() == 3 && q.stride(2) == 1 && q.stride(1) == q.size(2), "q must be [T, Hq, D] with packed heads");
   on_device_of(q, {&out, &k_cache, &v_cache, &block_table, &seq_lens},
                {&kv_scales, &query_start_loc, &sinks, &lse_out, &workspace, &alibi_slopes, &distance_bias, &gate, &sigmoid_shift});
@@ -74,6 +74,22 @@ void paged_attention_decode(Tensor& out, const Tensor& q, const Tensor& k_cache,
   if (kind == 0)
     TORCH_CHECK(k_cache.scalar_type() == q.scalar_type() && pv.page_stride % 8 == 0 && q.stride(0) % 8 == 0 && aligned(q) &&
                 aligned(k_cache) && aligned(v_cache), "paged attention: rows must start on 16 bytes");
+  if (stream && !query_start_loc.has_value() && max_q_len == 1 && batch == T && b200::decode_stream_serves(p, kind, (int)batch)) {
+    static int sms_of[64] = {};
+    int& sms = sms_of[q.get_device() & 63];
+    if (sms == 0) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, q.get_device());
+    int64_t floats = 0;
+    b200::decode_stream_scratch(p, kind, dtype16(q), (int)batch, sms, &floats);
+    // the caller's, zero in front, or one of this call alone
+    const bool given = scratch.has_value() && scratch->scalar_type() == at::kFloat && scratch->is_contiguous() &&
+                       scratch->get_device() == q.get_device() && scratch->numel() >= floats + b200::kDecodeCounters;
+    const Tensor own = given ? *scratch : at::empty({floats + b200::kDecodeCounters}, q.options().dtype(at::kFloat));
+    int* counters = reinterpret_cast<int*>(own.data_ptr<float>());
+    if (!given) C10_CUDA_CHECK(cudaMemsetAsync(counters, 0, batch * p.num_kv_heads * sizeof(int), cur_stream()));
+    b200::decode_stream(p, kind, dtype16(q), (int)batch, sms, own.data_ptr<float>() + b200::kDecodeCounters, counters, given,
+                        cur_stream());
+    return;
+  }
   if (p.num_splits > 1) {
     TORCH_CHECK(workspace.has_value(), "split-KV decode needs a workspace");
     const int64_t need = p.num_splits * (int64_t)T * Hq * (D + 1);
@@ -151,7 +167,7 @@ TORCH_LIBRARY_FRAGMENT(b200, m) {
       "Tensor seq_lens, Tensor? query_start_loc, float scale, int window, float softcap, Tensor? sinks, "
       "Tensor(b!)? lse_out, Tensor(c!)? workspace, int num_splits, int batch, int max_q_len, float k_scale, "
       "float v_scale, bool causal, Tensor? alibi_slopes=None, Tensor? distance_bias=None, Tensor? gate=None, "
-      "float out_scale=1.0, int chunk=0, Tensor? sigmoid_shift=None) -> ()",
+      "float out_scale=1.0, int chunk=0, Tensor? sigmoid_shift=None, bool stream=False, Tensor(d!)? scratch=None) -> ()",
       &paged_attention_decode);
   m.def(
       "head_norm_rope(Tensor(a!)? q_out, Tensor qkv, int q_off, int k_off, int v_off, Tensor(b!)? k_cache, Tensor(c!)? v_cache, "

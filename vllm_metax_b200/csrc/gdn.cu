@@ -5,7 +5,8 @@
 //   S  <- S + k_t u^T
 //   o_t = S^T (scale * q_t)
 //
-// G = 4 tokens are taken at a time, one for decode steps (gdn_step_kernel).  With S as it is before the group, G_t the sum of g over the group's
+// bf16 prompts go by chunks of 16 tokens on the tensor cores (further down); decode steps a token at a time (gdn_step_kernel);
+// fp16 prompts by groups of G = 4 on the fp32 units, as follows.  With S as it is before the group, G_t the sum of g over the group's
 // tokens up to t and D_tj = exp(G_t - G_j) (never above 1):
 //
 //   u_t = beta_t (v_t - exp(G_t) k_t . S - sum_{j<t} D_tj (k_t . k_j) u_j)
@@ -22,7 +23,7 @@
 // way in registers meanwhile.  What bounds it: for prompts the fp32 units (13 multiply-adds per state element and 4 tokens); for
 // decode steps the state's read and write.
 // 4 prompts of 3949 tokens in all (the longest 2048), 32 heads: 3382 us with a token at a time and a thread per column,
-// 705 us now.  64 decode rows: 58.6 us, now 49.5 us.
+// 705 us by groups, 313 us by chunks.  64 decode rows: 58.6 us, now 49.5 us.
 // The state is read from / written to a slot pool, so that decode steps and chunked prefill continue where the last call stopped.
 // Covers ChunkGatedDeltaRule.forward (vllm_metax/registry/custom_ops/layers/mamba/qwen_gdn_linear_attn.py:16-88)
 // and the fused recurrent decode step of the same block.

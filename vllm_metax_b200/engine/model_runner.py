@@ -115,6 +115,7 @@ class ModelRunner:
         self._alloc_state_slots()
         self._enable_fused_tp()
         self.graphs: dict[int, tuple] = {}
+        self._decode_scratch: Optional[torch.Tensor] = None
         self.use_graphs = self.is_cuda and not cfg.enforce_eager and envs.B200_CUDA_GRAPHS
         # replicas that share their experts exchange tokens in every MoE layer with sizes agreed on the host, and
         # their steps differ in shape (one decodes while another prefills): a replayed graph would skip the host
@@ -716,6 +717,11 @@ class ModelRunner:
             md.extra["state_indices"] = self.state_dev[:bucket]
             md.extra["state_has_init"] = self.state_dev[B: B + bucket]
         spec = self.model.kv_cache_spec()
+        if spec["kind"] == "gqa":                 # one for all captured steps: they follow one another in a stream
+            if self._decode_scratch is None:
+                hq = spec["num_kv_heads"] * (self.cfg.model.num_attention_heads // self.cfg.model.num_key_value_heads)
+                self._decode_scratch = ops.decode_scratch(hq, spec["num_kv_heads"], spec["head_size"], self.device, self.sms)
+            md.extra["decode_scratch"] = self._decode_scratch
         if md.decode_num_splits > 1 and spec["kind"] == "gqa":
             hq = spec["num_kv_heads"] * (self.cfg.model.num_attention_heads // self.cfg.model.num_key_value_heads)
             md.decode_workspace = torch.empty(md.decode_num_splits * bucket * hq * (spec["head_size"] + 1),

@@ -75,6 +75,10 @@ class StaticWorkload:
             prefill_query_start_loc=r.prefill_qsl[:1], max_prefill_query_len=0)
         if r.model.kv_cache_spec()["kind"] == "gqa":          # other caches choose in their own attention op
             md.decode_num_splits = ops.decode_num_splits(N, r.model.kv_cache_spec()["num_kv_heads"], self.P + self.O, 1, r.sms)
+        if r.model.kv_cache_spec()["kind"] == "gqa":
+            spec = r.model.kv_cache_spec()
+            hq = r.cfg.model.num_attention_heads // max(1, r.cfg.parallel.tensor_parallel_size)
+            md.extra["decode_scratch"] = ops.decode_scratch(hq, spec["num_kv_heads"], spec["head_size"], dev, r.sms)
         if md.decode_num_splits > 1:
             spec = r.model.kv_cache_spec()
             hq = r.cfg.model.num_attention_heads // max(1, r.cfg.parallel.tensor_parallel_size)

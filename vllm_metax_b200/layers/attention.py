@@ -149,7 +149,8 @@ class Attention(nn.Module):
                                        sinks=self.sinks, num_splits=md.decode_num_splits, max_seq_len=md.max_seq_len,
                                        k_scale=self.k_scale, v_scale=self.v_scale, workspace=md.decode_workspace,
                                        alibi_slopes=self.alibi_slopes, distance_bias=self.distance_bias, gate=gates[0],
-                                       out_scale=self.out_scale, chunk=self.chunk, sigmoid_shift=self.sigmoid_shift)
+                                       out_scale=self.out_scale, chunk=self.chunk, sigmoid_shift=self.sigmoid_shift,
+                                       scratch=md.extra.get("decode_scratch"))
         if md.num_prefills > 0:
             ops.paged_attention_prefill(q3[ndt:], kv_cache, md.block_table[nd:], md.seq_lens[nd:],
                                         md.prefill_query_start_loc, self.scale, out=out[ndt:], kv_scales=kv_scales,
