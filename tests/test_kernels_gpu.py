@@ -558,3 +558,32 @@ def test_decode_shared_out_evenly(lens, Hq, Hkv, D, kind, kernel_status_ok):
             assert bool(((got[i] - want).abs() <= bound + 1e-5).all()), (i, n, float((got[i] - want).abs().max()))
             if lse is not None:
                 torch.testing.assert_close(lse[:, i].cpu(), full.logsumexp(-1), rtol=1e-4, atol=2e-3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bs", [16, 64, 128])
+@pytest.mark.parametrize("Hq,Hkv", [(16, 2), (6, 2)])
+@pytest.mark.parametrize("kw", [dict(), dict(window=70), dict(softcap=15.0), dict(causal=False)])
+def test_prefill_of_256_wide_heads(bs, Hq, Hkv, kw, kernel_status_ok):
+    """The one-tile tcgen05 kernel on paged 256-wide heads, portions behind context and without, lengths around its tiles (16
+    tokens of 8 heads or 128 of one, 64 keys), against the decode kernel's 16-row tiles on the same cache."""
+    g = torch.Generator().manual_seed(bs + Hq)
+    qlens, past = [1, 15, 16, 129, 63, 200], [0, 64, 3, 0, 129, 1]
+    lens = [a + b for a, b in zip(qlens, past)]
+    nb = [-(-n // bs) for n in lens]
+    table, perm, at = torch.zeros(len(lens), max(nb), dtype=torch.int32), torch.randperm(sum(nb), generator=g), 0
+    for i, n in enumerate(nb):
+        table[i, :n] = perm[at: at + n]
+        at += n
+    q = torch.randn(sum(qlens), Hq, 256, generator=g).bfloat16().cuda()
+    cache = torch.randn(sum(nb), 2, bs, Hkv, 256, generator=g).bfloat16().cuda()
+    qsl = torch.tensor([0] + list(torch.tensor(qlens).cumsum(0)), dtype=torch.int32).cuda()
+    sl = torch.tensor(lens, dtype=torch.int32).cuda()
+    l1, l2 = (torch.empty(Hq, q.shape[0], device="cuda") for _ in range(2))
+    args, sizes = (q, cache, table.cuda(), sl), dict(max_q_len=max(qlens), max_seq_len=max(lens))
+    got = ops.paged_attention_prefill(*args, qsl, 256 ** -0.5, **sizes, **kw)
+    want = ops.paged_attention_decode(*args, 256 ** -0.5, query_start_loc=qsl, lse_out=l2, **sizes, **kw)
+    # both round weights to bf16 (2^-9 of each, weights of 1 / n random values of size 1) and the result (2^-9)
+    torch.testing.assert_close(got.float(), want.float(), rtol=2.0 ** -6, atol=2.0 ** -6)
+    # with the log-sum-exp: the decode kernel itself
+    assert torch.equal(ops.paged_attention_prefill(*args, qsl, 256 ** -0.5, lse_out=l1, **sizes, **kw), want) and torch.equal(l1, l2)

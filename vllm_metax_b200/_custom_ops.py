@@ -529,7 +529,13 @@ def paged_attention_prefill(q, kv_cache, block_table, seq_lens, query_start_loc,
         k, v = kv_views(kv_cache)
         out = torch.empty(q.shape[0], q.shape[1], v.shape[-1], dtype=q.dtype, device=q.device) if out is None else out
         B = seq_lens.shape[0]
-        if k.dtype == q.dtype and q.dtype != torch.float32 and k.shape[-1] <= 192 and v.shape[-1] <= 128 and kv_scales is None:
+        # 256-wide heads: the one-tile tcgen05 kernel, for plain softmax attention into packed rows (its log-sum-exp is that of
+        # weights rounded to 16 bits: callers that ask for it keep the other)
+        plain256 = lse_out is None and k.shape[-1] == v.shape[-1] == 256 and distance_bias is None and gate is None and out_scale == 1.0 \
+            and chunk == 0 and sigmoid_shift is None and out.is_contiguous() and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 \
+            and (128 % k.shape[1] == 0 or k.shape[1] % 128 == 0) and k.shape[1] % 16 == 0
+        if k.dtype == q.dtype and q.dtype != torch.float32 and kv_scales is None \
+                and (k.shape[-1] <= 192 and v.shape[-1] <= 128 or plain256):
             if distance_bias is not None and bias_tiles is None:
                 bias_tiles = distance_bias_tiles(distance_bias, q.shape[1] // k.shape[2])
             torch.ops.b200.attention_prefill(out, q, k, v, block_table, seq_lens, query_start_loc, None,

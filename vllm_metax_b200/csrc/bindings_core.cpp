@@ -327,9 +327,10 @@ void attention_prefill(Tensor& out, const Tensor& q, const Tensor& k_src, const 
     return e != nullptr && std::atoi(e) != 0;
   }();
   const bool extras = distance_bias.has_value() || gate.has_value() || p.chunk > 0 || sigmoid_shift.has_value() || out_scale != 1.0 || !out.is_contiguous();
-  const bool packed = extras ? false : paged ? DQK == DV && (DQK == 64 || DQK == 128)                // the one-tile kernel wants that
+  const bool packed = extras ? false : paged ? DQK == DV && (DQK == 64 || DQK == 128 || DQK == 256)               // the one-tile kernel wants that
                             : p.k_head_stride == DQK && p.v_head_stride == DV;
-  const int rc = single_tile && packed
+  // (256-wide heads: only the one-tile kernel has them)
+  const int rc = (single_tile || DQK == 256) && packed
                      ? b200::attention_prefill(p, q.data_ptr(), q.stride(0), kptr, vptr, ks, vs, total_kv, DQK, DV,
                                                dtype16(q), batch, max_q_len, cur_stream())
                      : b200::attention_prefill_pp(p, q.data_ptr(), q.stride(0), kptr, vptr, ks, vs, total_kv, DQK, DV,
