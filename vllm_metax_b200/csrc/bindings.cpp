@@ -721,11 +721,12 @@ void gdn_run(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const
   p.has_initial = has_initial.has_value() ? has_initial->data_ptr<int>() : nullptr;
   p.tokens = T; p.q_stride = q.stride(0); p.k_stride = k.stride(0); p.v_stride = v.stride(0);
   p.batch = (int)B; p.hq = (int)hq; p.hv = (int)hv; p.l2norm = l2norm; p.scale = (float)scale;
-  Tensor lengths;                                     // (a step of decode rows only has no groups of tokens)
-  p.lengths = nullptr;
-  if (T > B) {
-    lengths = at::empty({b200::gdn_lengths_bytes(T, (int)hq)}, q.options().dtype(at::kByte));
-    p.lengths = reinterpret_cast<const b200::GdnLengths*>(lengths.data_ptr());
+  Tensor scratch;
+  p.step = T <= B;                                    // (a step of decode rows only)
+  if (!p.step) {
+    scratch = at::empty({b200::gdn_scratch_bytes(T, (int)B, (int)hq, (int)hv, dtype16(q))}, q.options().dtype(at::kByte));
+    p.lengths = reinterpret_cast<const b200::GdnLengths*>(scratch.data_ptr());
+    p.chunks = reinterpret_cast<const float*>(scratch.data_ptr());
   }
   const int rc = b200::gdn_recurrent(p, (int)q.size(2), (int)v.size(2), dtype16(q), cur_stream());
   TORCH_CHECK(rc == 0, "gdn_recurrent: head sizes must be 128 and value heads a multiple of q/k heads");

@@ -27,9 +27,13 @@
 // The state is read from / written to a slot pool, so that decode steps and chunked prefill continue where the last call stopped.
 // Covers ChunkGatedDeltaRule.forward (vllm_metax/registry/custom_ops/layers/mamba/qwen_gdn_linear_attn.py:16-88)
 // and the fused recurrent decode step of the same block.
+#include <type_traits>
+
 #include "common.cuh"
+#include "attn_decode.cuh"
 #include "f32x2.cuh"
 #include "ops.h"
+#include "pdl.cuh"
 
 namespace b200 {
 
@@ -47,8 +51,10 @@ constexpr int kThreads = kCols / 4 * kLanes;
 // 8 lanes per (token, key head).
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
-gdn_lengths_kernel(GdnLengths* __restrict__ out, const T* __restrict__ q, const T* __restrict__ k, int tokens, int hq,
+gdn_lengths_kernel(GdnLengths* out, const T* q, const T* k, int tokens, int hq,
                    int64_t q_stride, int64_t k_stride, float scale, int l2norm) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t w = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3);
   const int lane = threadIdx.x & 7;
   const bool live = w < (int64_t)tokens * hq;
@@ -131,6 +137,8 @@ __device__ __forceinline__ void gdn_gates(const GdnParams& p, int64_t t, int h, 
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(kThreads, 3)
 gdn_kernel(const GdnParams p) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int G = 4, NS = 16, NB = 2;                        // tokens of a group, of a stage; stages
   constexpr int KQ = NS * (kD / 8) / kThreads;
   const int b = blockIdx.z, h = blockIdx.y, hk = h / (p.hv / p.hq), col0 = blockIdx.x * kCols;
@@ -379,11 +387,356 @@ gdn_kernel(const GdnParams p) {
   }
 }
 
+// ------------------------------------------------------------------------------------------ chunks of 16 tokens (bf16)
+// The recurrence over a chunk as products of 16 x 16 and 16 x 128 matrices on the tensor cores: with L_tj = beta_t D_tj k_t . k_j
+// (j < t), U = (I + L)^-1 (beta V - A K S), O = C Q S + M U, S <- e^G S + K^T (W U), where A, C and W are factors per token.  What
+// depends on q, k and the gates alone comes from a kernel in front, for all chunks at once.  q and k are the 16-bit rows
+// themselves; everything of 32 bits (the state, U) goes in as three bf16 terms, which hold its 24 bits, so the products are as
+// exact as fp32 ones.  Bound by the mma.sync rate along the longest sequence: 144 products a chunk and warp.
+constexpr int kC = 16;                     // tokens of a chunk
+constexpr int kChunkFloats = 2 * kC * kC + 5 * kC;   // T, M; factors a, beta, c, w; e^G of the last token
+
+// The chunk of index `at` in the order of the sequences: its sequence and first token, or false behind the last.  A whole warp.
+__device__ __forceinline__ bool gdn_locate(const int* __restrict__ qsl, int batch, int at, int lane, int& seq, int& first, int& end) {
+  int before = 0;
+  for (int b0 = 0; b0 < batch; b0 += 32) {
+    const int b = b0 + lane;
+    const int n = b < batch ? (qsl[b + 1] - qsl[b] + kC - 1) / kC : 0;
+    int inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, at < before + inc);
+    if (hit) {
+      const int src = __ffs(hit) - 1;
+      const int start = before + __shfl_sync(0xffffffffu, inc - n, src);
+      seq = b0 + src;
+      first = qsl[seq] + (at - start) * kC;
+      end = qsl[seq + 1];
+      return true;
+    }
+    before += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  return false;
+}
+
+// Rows t0 .. of n tokens, kD entries each, as bf16 with swizzled 16-byte chunks; rows from n on are zero.
+template <bool VEC>
+__device__ __forceinline__ void gdn_copy_rows(__nv_bfloat16* dst, const __nv_bfloat16* __restrict__ src, int64_t stride, int n, int tid,
+                                              int threads) {
+  for (int i = tid; i < kC * (kD / 8); i += threads) {
+    const int r = i / (kD / 8), c = i % (kD / 8);
+    void* d = dst + r * kD + ((c ^ (r & 7)) * 8);
+    const __nv_bfloat16* at = src + r * stride + c * 8;
+    if constexpr (VEC) {
+      cp_async16(d, r < n ? at : src, r < n);
+    } else {
+      __nv_bfloat16 x[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = r < n ? at[e] : __float2bfloat16_rn(0.f);
+      *reinterpret_cast<uint4*>(d) = *reinterpret_cast<const uint4*>(x);
+    }
+  }
+}
+
+// One CTA per (chunk, key head), a warp per value head of it in turn: (I + L)^-1 with L_tj = beta_t D_tj k_t . k_j (j < t), M_tj =
+// D_tj q_t . k_j (j <= t), both of unit vectors, and the factors of the sums with the state.
+template <bool VEC>
+__global__ void __launch_bounds__(128)
+gdn_chunk_prepare_kernel(const GdnParams p) {
+  using T = __nv_bfloat16;
+  pdl_trigger();
+  pdl_wait();
+  __shared__ __align__(128) T s_k[kC * kD], s_q[kC * kD];
+  __shared__ float s_kk[kC][kC], s_qk[kC][kC], s_ik[kC], s_iq[kC], s_l[4][kC][kC + 1];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, hk = blockIdx.y;
+  int seq, first, end;
+  if (!gdn_locate(p.query_start_loc, p.batch, blockIdx.x, lane, seq, first, end)) return;
+  const int n = min(kC, end - first);
+  gdn_copy_rows<VEC>(s_k, reinterpret_cast<const T*>(p.k) + first * p.k_stride + hk * kD, p.k_stride, n, tid, 128);
+  gdn_copy_rows<VEC>(s_q, reinterpret_cast<const T*>(p.q) + first * p.q_stride + hk * kD, p.q_stride, n, tid, 128);
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  if (warp < 2) {                                   // k k^T, q k^T: the products of bf16 are exact, their sums in fp32
+    float d[2][4] = {};
+    const T* a = warp == 0 ? s_k : s_q;
+#pragma unroll
+    for (int ks = 0; ks < kD / 16; ++ks) {
+      uint32_t af[4], bf[4];
+      const int mat = lane >> 3;
+      const int ra = (mat & 1) * 8 + (lane & 7), rb = (mat >> 1) * 8 + (lane & 7);
+      ldmatrix_x4(af, a + ra * kD + (((2 * ks + (mat >> 1)) ^ (ra & 7)) * 8));
+      ldmatrix_x4(bf, s_k + rb * kD + (((2 * ks + (mat & 1)) ^ (rb & 7)) * 8));
+      mma16816<T>(d[0], af, bf[0], bf[1]);
+      mma16816<T>(d[1], af, bf[2], bf[3]);
+    }
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        (warp == 0 ? s_kk : s_qk)[(lane >> 2) + (e >> 1) * 8][nt * 8 + 2 * (lane & 3) + (e & 1)] = d[nt][e];
+  } else if (warp == 2) {                           // |q|^2, two lanes a token
+    const int r = lane >> 1;
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float f[8];
+      unpack8<T>(*reinterpret_cast<const uint4*>(s_q + r * kD + ((((lane & 1) * 8 + i) ^ (r & 7)) * 8)), f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss = fmaf(f[e], f[e], ss);
+    }
+    ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+    if (!(lane & 1)) s_iq[r] = (p.l2norm ? rsqrtf(ss + 1e-6f) : 1.f) * p.scale;
+  }
+  __syncthreads();
+  if (tid < kC) s_ik[tid] = p.l2norm ? rsqrtf(s_kk[tid][tid] + 1e-6f) : 1.f;
+  __syncthreads();
+  const int rep = p.hv / p.hq;
+  for (int hr = warp; hr < rep; hr += 4) {
+    const int h = hk * rep + hr, t = lane & (kC - 1);
+    float g = 0.f, beta = 0.f;
+    if (t < n) gdn_gates<T>(p, first + t, h, g, beta);
+    float upto = g;                                 // sums over the chunk's tokens up to this one
+#pragma unroll
+    for (int o = 1; o < kC; o <<= 1) {
+      const float v = __shfl_up_sync(0xffffffffu, upto, o, kC);
+      if (t >= o) upto += v;
+    }
+    const float all = __shfl_sync(0xffffffffu, upto, kC - 1, kC);
+    float* out = const_cast<float*>(p.chunks) + ((int64_t)blockIdx.x * p.hv + h) * kChunkFloats;
+    float after = 0.f;                              // those behind this token, summed by themselves
+    {
+      float v = __shfl_down_sync(0xffffffffu, g, 1, kC);
+      after = t + 1 < kC ? v : 0.f;
+#pragma unroll
+      for (int o = 1; o < kC; o <<= 1) {
+        v = __shfl_down_sync(0xffffffffu, after, o, kC);
+        if (t + o < kC) after += v;
+      }
+    }
+    if (lane < kC) {
+      const float e = expf(upto), ik = s_ik[t];
+      float* f = out + 2 * kC * kC;
+      f[t] = beta * e * ik;
+      f[kC + t] = beta;
+      f[2 * kC + t] = s_iq[t] * e;
+      f[3 * kC + t] = expf(after) * ik;
+      if (t == 0) f[4 * kC] = expf(all);
+    }
+    // lanes t and t + 16: every other column j.  D_tj = exp(g_{j+1} + .. + g_t), each sum by itself
+    float between = 0.f;
+#pragma unroll
+    for (int j = kC - 1; j >= 0; --j) {
+      const float gj = __shfl_sync(0xffffffffu, g, (j + 1) & (kC - 1), kC);
+      if (j < t) between += gj;
+      if ((j & 1) != (lane >> 4)) continue;
+      const float d = expf(between);
+      s_l[warp][t][j] = j < t ? beta * d * s_kk[t][j] * s_ik[t] * s_ik[j] : 0.f;
+      out[kC * kC + t * kC + j] = j <= t ? d * s_qk[t][j] * s_iq[t] * s_ik[j] : 0.f;
+    }
+    __syncwarp();
+    if (lane < kC) {                                // column `lane` of the inverse by forward substitution
+      float x[kC];
+#pragma unroll
+      for (int r = 0; r < kC; ++r) {
+        float v = r == lane ? 1.f : 0.f;
+#pragma unroll
+        for (int j = 0; j < r; ++j) v = fmaf(-s_l[warp][r][j], x[j], v);
+        x[r] = v;
+        out[r * kC + lane] = v;
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// fp32 pairs as three bf16 terms each, which hold all 24 bits.
+__device__ __forceinline__ void split3(float a, float b, uint32_t (&t)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    t[i] = *reinterpret_cast<const uint32_t*>(&v);
+    a -= __uint_as_float(t[i] << 16);
+    b -= __uint_as_float(t[i] & 0xffff0000u);
+  }
+}
+
+constexpr int kWarpCols = 16, kChunkWarps = 4, kPadR = kC + 2;
+
+// One CTA = one (sequence, value head, 64 value columns), a warp 16 columns of the state, transposed, as accumulators of
+// m16n8k16: they are the second operand of the products with k and q as they stand, and take the update as products with k.
+template <bool VEC>
+__global__ void __launch_bounds__(kChunkWarps * 32, 2)
+gdn_chunk_kernel(const GdnParams p) {
+  using T = __nv_bfloat16;
+  constexpr int CV = kWarpCols * kChunkWarps, TH = kChunkWarps * 32;
+  pdl_trigger();
+  pdl_wait();
+  __shared__ __align__(128) T s_k[2][kC * kD], s_q[2][kC * kD];
+  __shared__ __align__(16) T s_v[2][kC][CV];
+  __shared__ __align__(16) float s_f[2][kChunkFloats];
+  __shared__ __align__(16) float s_r[kChunkWarps][kC][kPadR], s_d[kChunkWarps][kC][kPadR];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tl = lane & 3;
+  const int b = blockIdx.z, h = blockIdx.y, hk = h / (p.hv / p.hq), col0 = blockIdx.x * CV + warp * kWarpCols;
+  const int t0 = p.query_start_loc[b], t1 = p.query_start_loc[b + 1];
+  if (t1 <= t0) return;
+  int chunk = 0;                                    // index of the sequence's first chunk
+  for (int i = lane; i < b; i += 32) chunk += (p.query_start_loc[i + 1] - p.query_start_loc[i] + kC - 1) / kC;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) chunk += __shfl_xor_sync(0xffffffffu, chunk, o);
+  const int slot = p.state_idx ? p.state_idx[b] : -1;
+  float* st = slot >= 0 ? p.state + (((int64_t)slot * p.hv + h) * kD) * kD + col0 : nullptr;
+  const T *gk = reinterpret_cast<const T*>(p.k) + hk * kD, *gqr = reinterpret_cast<const T*>(p.q) + hk * kD,
+          *gv = reinterpret_cast<const T*>(p.v) + h * kD + blockIdx.x * CV;
+  auto fetch = [&](int tc, int at, int buf) {
+    const int n = min(kC, t1 - tc);
+    gdn_copy_rows<VEC>(s_k[buf], gk + tc * p.k_stride, p.k_stride, n, tid, TH);
+    gdn_copy_rows<VEC>(s_q[buf], gqr + tc * p.q_stride, p.q_stride, n, tid, TH);
+    {
+      const int r = tid / (CV / 8), c = tid % (CV / 8) * 8;            // (128 threads: 16 rows of 8 pieces)
+      const T* at8 = gv + (int64_t)(tc + r) * p.v_stride + c;
+      if constexpr (VEC) {
+        cp_async16(&s_v[buf][r][c], r < n ? at8 : gv, r < n);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s_v[buf][r][c + e] = r < n ? at8[e] : __float2bfloat16_rn(0.f);
+      }
+    }
+    const float* f = p.chunks + ((int64_t)at * p.hv + h) * kChunkFloats;
+    for (int i = tid; i < kChunkFloats / 4; i += TH) cp_async16(&s_f[buf][i * 4], f + i * 4, true);
+    cp_async_commit();
+  };
+  static_assert(TH == kC * (CV / 8) && kChunkFloats % 4 == 0, "one piece of v a thread");
+  fetch(t0, chunk, 0);
+  float S[kD / 8][4];                               // keys 8 i + 2 tl, + 1 of columns gq and gq + 8
+  {
+    const bool init = st != nullptr && (p.has_initial == nullptr || p.has_initial[b] != 0);
+#pragma unroll
+    for (int i = 0; i < kD / 8; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) S[i][e] = init ? st[(int64_t)(8 * i + 2 * tl + (e & 1)) * kD + gq + (e >> 1) * 8] : 0.f;
+  }
+  int buf = 0;
+  for (int tc = t0; tc < t1; tc += kC, ++chunk, buf ^= 1) {
+    cp_async_wait<0>();
+    __syncthreads();                                // this chunk is here; the other buffer has been used up
+    if (tc + kC < t1) fetch(tc + kC, chunk + 1, buf ^ 1);
+    const float *fT = s_f[buf], *fM = fT + kC * kC, *fa = fM + kC * kC, *fb = fa + kC, *fc = fb + kC, *fw = fc + kC;
+    // ---- k . S and q . S: [16 tokens] x [columns 0..7, 8..15 of the warp]
+    float dk[2][4] = {}, dq[2][4] = {};
+#pragma unroll
+    for (int ks = 0; ks < kD / 16; ++ks) {
+      uint32_t ka[4], qa[4];
+      const int mat = lane >> 3, r = (mat & 1) * 8 + (lane & 7), o = r * kD + (((2 * ks + (mat >> 1)) ^ (r & 7)) * 8);
+      ldmatrix_x4(ka, s_k[buf] + o);
+      ldmatrix_x4(qa, s_q[buf] + o);
+#pragma unroll
+      for (int cg = 0; cg < 2; ++cg) {
+        uint32_t lo[3], hi[3];
+        split3(S[2 * ks][2 * cg], S[2 * ks][2 * cg + 1], lo);
+        split3(S[2 * ks + 1][2 * cg], S[2 * ks + 1][2 * cg + 1], hi);
+#pragma unroll
+        for (int i = 2; i >= 0; --i) {
+          mma16816<T>(dk[cg], ka, lo[i], hi[i]);
+          mma16816<T>(dq[cg], qa, lo[i], hi[i]);
+        }
+      }
+    }
+    // ---- right-hand sides, then a column per pair of lanes
+#pragma unroll
+    for (int cg = 0; cg < 2; ++cg)
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        const int t = gq + hf * 8, c = cg * 8 + 2 * tl;
+        const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&s_v[buf][t][warp * kWarpCols + c]);
+        *reinterpret_cast<float2*>(&s_r[warp][t][c]) = make_float2(fb[t] * __low2float(v) - fa[t] * dk[cg][2 * hf],
+                                                                   fb[t] * __high2float(v) - fa[t] * dk[cg][2 * hf + 1]);
+        *reinterpret_cast<float2*>(&s_d[warp][t][c]) = make_float2(dq[cg][2 * hf], dq[cg][2 * hf + 1]);
+      }
+    __syncwarp();
+    const int col = lane & 15, half = lane >> 4;    // this lane: rows 2 i + half
+    float R[kC], u[8], U[kC];
+#pragma unroll
+    for (int t = 0; t < kC; ++t) R[t] = s_r[warp][t][col];
+    auto rows = [&](const float* m, const float (&x)[kC], int i) {     // row 2 i + half of a lower triangle times x
+      float acc = 0.f;
+#pragma unroll
+      for (int j = 0; j < 2 * i + 2; j += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(m + (2 * i + half) * kC + j);
+        acc = fmaf(a.x, x[j], acc);
+        acc = fmaf(a.y, x[j + 1], acc);
+        acc = fmaf(a.z, x[j + 2], acc);
+        acc = fmaf(a.w, x[j + 3], acc);
+      }
+      return acc;
+    };
+#pragma unroll
+    for (int i = 0; i < 8; ++i) u[i] = rows(fT, R, i);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float other = __shfl_xor_sync(0xffffffffu, u[i], 16);
+      U[2 * i] = half ? other : u[i];
+      U[2 * i + 1] = half ? u[i] : other;
+    }
+    __syncwarp();                                   // (s_r has been read: it takes the update, columns first)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int t = 2 * i + half;
+      const float o = fmaf(fc[t], s_d[warp][t][col], rows(fM, U, i));
+      if (tc + t < t1) reinterpret_cast<T*>(p.out)[((int64_t)(tc + t) * p.hv + h) * kD + col0 + col] = __float2bfloat16_rn(o);
+      s_r[warp][col][t] = fw[t] * u[i];
+    }
+    __syncwarp();
+    // ---- S <- e^G S + W^T k
+    uint32_t w[4][3];
+    {
+      float2 x = *reinterpret_cast<const float2*>(&s_r[warp][gq][2 * tl]);
+      split3(x.x, x.y, w[0]);
+      x = *reinterpret_cast<const float2*>(&s_r[warp][gq + 8][2 * tl]);
+      split3(x.x, x.y, w[1]);
+      x = *reinterpret_cast<const float2*>(&s_r[warp][gq][2 * tl + 8]);
+      split3(x.x, x.y, w[2]);
+      x = *reinterpret_cast<const float2*>(&s_r[warp][gq + 8][2 * tl + 8]);
+      split3(x.x, x.y, w[3]);
+    }
+    const float last = fw[kC];
+#pragma unroll
+    for (int i = 0; i < kD / 8; i += 2) {
+      uint32_t kt[4];
+      const int mat = lane >> 3, r = (mat & 1) * 8 + (lane & 7);
+      ldmatrix_x4_trans(kt, s_k[buf] + r * kD + (((i + (mat >> 1)) ^ (r & 7)) * 8));
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        S[i][e] *= last;
+        S[i + 1][e] *= last;
+      }
+#pragma unroll
+      for (int j = 2; j >= 0; --j) {
+        const uint32_t a[4] = {w[0][j], w[1][j], w[2][j], w[3][j]};
+        mma16816<T>(S[i], a, kt[0], kt[1]);
+        mma16816<T>(S[i + 1], a, kt[2], kt[3]);
+      }
+    }
+    __syncwarp();                                   // s_r, s_d are rewritten by the next chunk
+  }
+  if (st != nullptr) {
+#pragma unroll
+    for (int i = 0; i < kD / 8; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) st[(int64_t)(8 * i + 2 * tl + (e & 1)) * kD + gq + (e >> 1) * 8] = S[i][e];
+  }
+}
+
 // Decode rows: one CTA = one (sequence, value head), tokens one at a time.  A warp holds 16 rows of S, a lane 4 columns of them, so
 // that a warp reads and writes whole rows of 512 bytes, all before the first product; the warps' sums meet in shared memory.
 template <typename T>
 __global__ void __launch_bounds__(256, 2)
 gdn_step_kernel(const GdnParams p) {
+  pdl_trigger();
+  pdl_wait();
   const int b = blockIdx.x, h = blockIdx.y, hk = h / (p.hv / p.hq), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t t0 = p.query_start_loc[b], t1 = p.query_start_loc[b + 1];
   if (t1 <= t0) return;
@@ -454,31 +807,45 @@ gdn_step_kernel(const GdnParams p) {
   }
 }
 
+int64_t gdn_max_chunks(int64_t tokens, int batch) { return tokens / kC + batch; }
+
 template <typename T>
 void launch(const GdnParams& p, cudaStream_t stream) {
   auto wide = [](const void* at, int64_t stride) { return (reinterpret_cast<uintptr_t>(at) & 15) == 0 && stride % 8 == 0; };
   const bool vec = wide(p.q, p.q_stride) && wide(p.k, p.k_stride) && wide(p.v, p.v_stride);
   const dim3 grid(kD / kCols, p.hv, p.batch);
-  if (p.lengths == nullptr) {
-    gdn_step_kernel<T><<<dim3(p.batch, p.hv), 256, 0, stream>>>(p);
+  if (p.step) {
+    pdl_run(gdn_step_kernel<T>, dim3(p.batch, p.hv), 256, 0, stream, p);
     return;
   }
-  const int64_t rows = p.tokens * p.hq;
-  const unsigned blocks = (unsigned)((rows + 31) / 32);
-  GdnLengths* len = const_cast<GdnLengths*>(p.lengths);
-#define GDN_RUN(V)                                                                                                        \
-  gdn_lengths_kernel<T, V><<<blocks, 256, 0, stream>>>(len, (const T*)p.q, (const T*)p.k, (int)p.tokens, p.hq, p.q_stride,      \
-                                                       p.k_stride, p.scale, p.l2norm);                                    \
-  gdn_kernel<T, V><<<grid, kThreads, 0, stream>>>(p)
-  if (vec) { GDN_RUN(true); } else { GDN_RUN(false); }
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+    const dim3 chunks((unsigned)gdn_max_chunks(p.tokens, p.batch), p.hq), parts(kD / (kWarpCols * kChunkWarps), p.hv, p.batch);
+    if (vec) {
+      pdl_run(gdn_chunk_prepare_kernel<true>, chunks, 128, 0, stream, p);
+      pdl_run(gdn_chunk_kernel<true>, parts, kChunkWarps * 32, 0, stream, p);
+    } else {
+      pdl_run(gdn_chunk_prepare_kernel<false>, chunks, 128, 0, stream, p);
+      pdl_run(gdn_chunk_kernel<false>, parts, kChunkWarps * 32, 0, stream, p);
+    }
+  } else {
+    const unsigned blocks = (unsigned)((p.tokens * p.hq + 31) / 32);
+    GdnLengths* len = const_cast<GdnLengths*>(p.lengths);
+#define GDN_RUN(V)                                                                                                            \
+  pdl_run(gdn_lengths_kernel<T, V>, blocks, 256, 0, stream, len, (const T*)p.q, (const T*)p.k, (int)p.tokens, p.hq, p.q_stride, \
+          p.k_stride, p.scale, p.l2norm);                                                                                     \
+  pdl_run(gdn_kernel<T, V>, grid, kThreads, 0, stream, p)
+    if (vec) { GDN_RUN(true); } else { GDN_RUN(false); }
 #undef GDN_RUN
+  }
 }
 
 // DIM / 8 lanes per (token, head).
 template <typename T, int DIM>
 __global__ void __launch_bounds__(256)
-gated_head_norm_kernel(T* __restrict__ out, const T* __restrict__ o, const T* __restrict__ z, const T* __restrict__ w,
+gated_head_norm_kernel(T* out, const T* o, const T* z, const T* w,
                        int64_t rows, int heads, int rep, int64_t z_stride, int64_t z_group, float eps) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int L = DIM / 8;
   const int64_t r = (int64_t)blockIdx.x * (256 / L) + threadIdx.x / L;
   const int c = threadIdx.x % L * 8;
@@ -519,7 +886,7 @@ int gated_head_norm(void* out, const void* o, const void* z, const void* w, int6
   if (rows <= 0) return 0;
   const unsigned blocks = (unsigned)((rows + 256 / (dim / 8) - 1) / (256 / (dim / 8)));
 #define GHN(T, D)                                                                                                            \
-  gated_head_norm_kernel<T, D><<<blocks, 256, 0, stream>>>((T*)out, (const T*)o, (const T*)z, (const T*)w, rows, heads, rep, \
+  pdl_run(gated_head_norm_kernel<T, D>, blocks, 256, 0, stream, (T*)out, (const T*)o, (const T*)z, (const T*)w, rows, heads, rep, \
                                                            z_stride, z_group, eps)
   if (dtype == 0) {
     if (dim == 64) GHN(__nv_bfloat16, 64); else if (dim == 128) GHN(__nv_bfloat16, 128); else GHN(__nv_bfloat16, 256);
@@ -530,7 +897,9 @@ int gated_head_norm(void* out, const void* o, const void* z, const void* w, int6
   return 0;
 }
 
-int64_t gdn_lengths_bytes(int64_t tokens, int hq) { return tokens * hq * (int64_t)sizeof(GdnLengths); }
+int64_t gdn_scratch_bytes(int64_t tokens, int batch, int hq, int hv, int dtype) {
+  return dtype == 0 ? gdn_max_chunks(tokens, batch) * hv * kChunkFloats * (int64_t)sizeof(float) : tokens * hq * (int64_t)sizeof(GdnLengths);
+}
 
 // Returns 0, or 1 when the head sizes are not 128 / the head counts do not divide.
 int gdn_recurrent(const GdnParams& p, int dk, int dv, int dtype, cudaStream_t stream) {
