@@ -487,7 +487,7 @@ void small_gemm(Tensor& out, const Tensor& a, const Tensor& w, const optional<Te
   const int rc = b200::small_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), bias.has_value() ? bias->data_ptr() : nullptr,
                                   a.size(0), w.size(0), a.size(1), a.stride(0), w.stride(0), out.stride(0), dtype16(a),
                                   f32 ? 1 : 0, cur_stream());
-  TORCH_CHECK(rc == 0, "small_gemm: needs M <= 32, K % 32 == 0 and 16-byte aligned rows (rc=", rc, ")");
+  TORCH_CHECK(rc == 0, "small_gemm: needs M <= 64, K % 32 == 0 and 16-byte aligned rows (rc=", rc, ")");
 }
 
 void fused_qk_norm_rope(Tensor& qkv, const Tensor& q_weight, const Tensor& k_weight, const Tensor& cos_sin,

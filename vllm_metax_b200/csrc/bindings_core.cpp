@@ -64,6 +64,16 @@ void gemm(Tensor& out, const Tensor& a, const Tensor& w, const optional<Tensor>&
                        w.stride(0), out.stride(0), ldr, dtype16(a), cur_stream(), status_ptr(a), epi_arg);
     return;
   }
+  // A router, or another narrow product of a decode batch: the stream-K kernel's fixed costs are most of its 13 us there
+  // (64 x 128 x 2048: 8.9 us here).  From a few MB of weights on it streams them faster, and re-reading the tokens for every 8
+  // columns, as this kernel does, begins to count.
+  if (force_bn == 0 && M <= 64 && N <= 512 && (int64_t)N * K <= (1 << 21) && epi == 0 && !residual.has_value() && K % 32 == 0) {
+    const auto wide = [](const void* at) { return (reinterpret_cast<uintptr_t>(at) & 15) == 0; };
+    if (wide(a.data_ptr()) && wide(w.data_ptr()) &&
+        b200::small_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), ptr(bias), M, N, K, a.stride(0), w.stride(0), out.stride(0),
+                         dtype16(a), 0, cur_stream()) == 0)
+      return;
+  }
   // stream-K over CTA pairs for skinny problems: decode batches and narrow tensor-parallel shards (force_bn 2000
   // pins it).  Its scratch (partial tiles + arrival counters) is allocated once per device and stream-ordered
   // use is assumed, like every other op of this library.
