@@ -205,3 +205,22 @@ def test_moe_rows_from_the_pairs(dtype, tokens, topk, hidden, experts):
     for k in range(topk):
         acc = torch.where((iv[:, k] >= 0)[:, None], acc + w[:, k: k + 1] * y[iv[:, k].clamp_min(0)].float(), acc)
     torch.testing.assert_close(out.float(), acc, rtol=2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10, atol=1e-5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,topk,E,N,K,epi", [(3, 2, 4, 256, 128, 0), (64, 8, 128, 1536, 256, 1), (500, 3, 5, 300, 72, 0)])
+def test_grouped_products_without_padding(T, topk, E, N, K, epi):
+    """One, a few and all rows of a block, both tile widths, a ragged contraction: padding rows hold NaN, are not read, and the
+    others equal those of the call that takes every row."""
+    g = torch.Generator().manual_seed(T)
+    ids = torch.stack([torch.randperm(E, generator=g)[:topk] for _ in range(T)]).to(torch.int32).cuda()
+    sorted_ids, be, total, inv = ops.moe_align_block_size(ids, 128, E, want_inverse=True)
+    real = sorted_ids < ids.numel()
+    x = torch.randn(T, K, generator=g).bfloat16().cuda()
+    a = ops.moe_scatter(x, inv, sorted_ids, total, topk)
+    a[~real] = float("nan")
+    w = torch.randn(E, N, K, generator=g).bfloat16().cuda()
+    got = ops.gemm_grouped(a, w, be, total, epi, None, sorted_ids, ids.numel())
+    want = ops.gemm_grouped(torch.where(real[:, None], a, torch.zeros_like(a)), w, be, total, epi)
+    assert torch.equal(got[real], want[real]) and bool(torch.isfinite(got[real]).all())
+    ops.check_kernel_status(0)

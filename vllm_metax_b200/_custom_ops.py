@@ -794,9 +794,10 @@ def moe_gather(x, sorted_ids, total_padded, topk: int, weights=None):
     return out
 
 
-def gemm_grouped(a, w, block_expert, total_padded, epi: int = 0, act_params=None):
+def gemm_grouped(a, w, block_expert, total_padded, epi: int = 0, act_params=None, sorted_ids=None, numel: int = 0):
     """Per-row-block expert GEMM: ``a [R, K]`` (R multiple of 128), ``w [E, N, K]`` -> ``[R, N]`` (``N/2`` with a gated
-    epilogue over row-interleaved gate/up weights).  ``epi``: a code of ``EPI_CODES``, ``act_params`` its numbers."""
+    epilogue over row-interleaved gate/up weights).  ``epi``: a code of ``EPI_CODES``, ``act_params`` its numbers.
+    ``sorted_ids``: rows with ids from ``numel`` on are padding at the end of an expert's rows; what they become nobody reads."""
     gated = epi in EPI_GATES
     if _use_cuda(a):
         n_out = w.shape[1] // 2 if gated else w.shape[1]
@@ -804,7 +805,7 @@ def gemm_grouped(a, w, block_expert, total_padded, epi: int = 0, act_params=None
         if a.dtype == torch.float32 or a.shape[1] % 8 != 0 or not _tma_ok(a, w, out) or (gated and w.shape[1] % 16 != 0):
             torch.ops.b200.gemm_simt(out, a, w, None, epi, act_params, block_expert, total_padded)
         else:
-            torch.ops.b200.gemm_grouped(out, a, w, block_expert, total_padded, epi, act_params)
+            torch.ops.b200.gemm_grouped(out, a, w, block_expert, total_padded, epi, act_params, sorted_ids, numel)
         return out
     R = a.shape[0]
     nblk = R // 128

@@ -239,8 +239,12 @@ void moe_sum(Tensor& out, const Tensor& in) {
 }
 
 void gemm_grouped(Tensor& out, const Tensor& a, const Tensor& w, const Tensor& block_expert,
-                  const Tensor& total_padded, int64_t act, const optional<Tensor>& act_params) {
-  on_device_of(a, {&out, &w, &block_expert, &total_padded}, {&act_params});
+                  const Tensor& total_padded, int64_t act, const optional<Tensor>& act_params, const optional<Tensor>& sorted_ids,
+                  int64_t numel) {
+  on_device_of(a, {&out, &w, &block_expert, &total_padded}, {&act_params, &sorted_ids});
+  if (sorted_ids.has_value()) {
+    TORCH_CHECK(sorted_ids->scalar_type() == at::kInt && sorted_ids->is_contiguous() && sorted_ids->numel() == a.size(0));
+  }
   const b200::Epi epi = make_epi(out, a, act, act_params);
   const bool gate = b200::epi_is_gate((int)act);
   TORCH_CHECK(!gate || w.size(1) % 16 == 0, "gated epilogue: N % 16 == 0");
@@ -249,8 +253,8 @@ void gemm_grouped(Tensor& out, const Tensor& a, const Tensor& w, const Tensor& b
   TORCH_CHECK(out.size(0) == a.size(0) && out.size(1) == (gate ? w.size(1) / 2 : w.size(1)));
   const c10::cuda::CUDAGuard guard(a.device());
   b200::gemm_grouped(a.data_ptr(), a.size(0), a.stride(0), w.data_ptr(), w.size(0), w.size(1), w.size(2),
-                     out.data_ptr(), out.stride(0), block_expert.data_ptr<int>(), total_padded.data_ptr<int>(), epi,
-                     dtype16(a), cur_stream(), status_ptr(a));
+                     out.data_ptr(), out.stride(0), block_expert.data_ptr<int>(), total_padded.data_ptr<int>(),
+                     ptr<int>(sorted_ids), (int)numel, epi, dtype16(a), cur_stream(), status_ptr(a));
 }
 
 void attention_prefill(Tensor& out, const Tensor& q, const Tensor& k_src, const optional<Tensor>& v_src,
@@ -506,7 +510,7 @@ TORCH_LIBRARY(b200, m) {
       "Tensor? through=None, int identity_from=0) -> ()",
       &moe_combine);
   m.def("moe_sum(Tensor(a!) out, Tensor inp) -> ()", &moe_sum);
-  m.def("gemm_grouped(Tensor(a!) out, Tensor a, Tensor w, Tensor block_expert, Tensor total_padded, int epi, Tensor? act_params=None) -> ()", &gemm_grouped);
+  m.def("gemm_grouped(Tensor(a!) out, Tensor a, Tensor w, Tensor block_expert, Tensor total_padded, int epi, Tensor? act_params=None, Tensor? sorted_ids=None, int numel=0) -> ()", &gemm_grouped);
   m.def(
       "attention_prefill(Tensor(a!) out, Tensor q, Tensor k_src, Tensor? v_src, Tensor? block_table, "
       "Tensor? seq_lens, Tensor query_start_loc, Tensor? kv_start_loc, float scale, int window, float softcap, "

@@ -226,8 +226,8 @@ void moe_combine(void* out, const void* y, const float* weights, const int* inv_
                  cudaStream_t stream);
 void moe_sum(void* out, const void* in, int tokens, int topk, int hidden, int dtype, cudaStream_t stream);
 void gemm_grouped(const void* A, int max_rows, int lda, const void* W, int E, int N, int K, void* C, int ldc,
-                  const int* block_expert, const int* total_padded, Epi epi, int dtype, cudaStream_t stream,
-                  void* status);
+                  const int* block_expert, const int* total_padded, const int* sorted_ids, int numel, Epi epi, int dtype,
+                  cudaStream_t stream, void* status);
 // ---- quant.cu / gemm_fp8_blockscale.cu
 void per_token_group_quant(void* q, float* scales, const void* x, int64_t rows, int K, int group, int int8, int ue8m0,
                            int col_major, float eps, int dtype, cudaStream_t stream);

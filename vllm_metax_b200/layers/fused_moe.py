@@ -76,8 +76,8 @@ def expert_rows(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_weigh
                                                                     expert_map, want_inverse=True)
     topk_weights = topk_weights.contiguous()
     a = ops.moe_scatter(x, inv, sorted_ids, total, topk, topk_weights if weight_input else None)
-    h = ops.gemm_grouped(a, w13, block_expert, total, epi=epi, act_params=epi_params)
-    y = ops.gemm_grouped(h, w2, block_expert, total, epi=0)
+    h = ops.gemm_grouped(a, w13, block_expert, total, epi, epi_params, sorted_ids, inv.numel())
+    y = ops.gemm_grouped(h, w2, block_expert, total, 0, None, sorted_ids, inv.numel())
     ident = identity_from is not None
     return ExpertRows(y, None if weight_input else topk_weights, inv, topk_ids if ident else None, x if ident else None,
                       identity_from or 0, shared_out, topk)
