@@ -587,3 +587,28 @@ def test_prefill_of_256_wide_heads(bs, Hq, Hkv, kw, kernel_status_ok):
     torch.testing.assert_close(got.float(), want.float(), rtol=2.0 ** -6, atol=2.0 ** -6)
     # with the log-sum-exp: the decode kernel itself
     assert torch.equal(ops.paged_attention_prefill(*args, qsl, 256 ** -0.5, lse_out=l1, **sizes, **kw), want) and torch.equal(l1, l2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,K", [(640, 2048), (6144, 4096), (1001, 1000), (28672, 512), (576, 14336)])
+def test_few_tokens_against_a_weight(dtype, M, N, K, kernel_status_ok):
+    """Rows that do not fill a CTA's eight, a contraction that ends inside a warp's piece, bias, residual and gated rows: sums of
+    products exact in fp32, rounded once (gated: the two factors first)."""
+    g = torch.Generator().manual_seed(N + M)
+    a = torch.randn(M, K, generator=g).to(dtype).cuda()
+    w = (torch.randn(N, K, generator=g) / K ** 0.5).to(dtype).cuda()
+    b = torch.randn(N, generator=g).to(dtype).cuda()
+    r = torch.randn(M, N, generator=g).to(dtype).cuda()
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    want = a.double() @ w.double().T
+    if N % 8 == 0:
+        torch.testing.assert_close(ops.gemm(a, w).double(), want, rtol=eps, atol=1e-5)
+        torch.testing.assert_close(ops.gemm(a, w, bias=b, residual=r).double(), want + b.double() + r.double(), rtol=eps, atol=1e-5)
+    if N % 16 == 0:
+        f = lambda x: x.to(dtype).double()
+        gate, up = f(want[:, 0::2]), f(want[:, 1::2])
+        got = ops.gemm_silu_mul(a, w).double()
+        # either factor may be the neighbouring number of its type, then one rounding
+        torch.testing.assert_close(got, torch.nn.functional.silu(gate) * up, rtol=5 * eps, atol=1e-4)

@@ -33,7 +33,7 @@ CUMEM_LIB = ROOT / "cumem_allocator.so"
 
 # the units behind bindings_core.cpp, what each set adds behind bindings_<set>.cpp, and the sets of each group
 CORE_UNITS = ("attn_prefill_pingpong", "attn_prefill_tcgen05", "gemm_grouped_tcgen05", "gemm_pair_tcgen05", "gemm_simt",
-              "gemm_splitk_tcgen05", "gemm_streamk_tcgen05", "gemm_tcgen05", "moe", "residual_norm", "rope_angles", "sampling", "small_gemm")
+              "gemm_splitk_tcgen05", "gemm_streamk_tcgen05", "gemm_tcgen05", "gemv", "moe", "residual_norm", "rope_angles", "sampling", "small_gemm")
 UNIT_SETS = {
     "gqa": ("attn_decode", "attn_decode_stream", "head_norm_rope", "paged_attn_simt"),
     "hybrid": ("residual_conv", "rglru"),

@@ -74,6 +74,16 @@ void gemm(Tensor& out, const Tensor& a, const Tensor& w, const optional<Tensor>&
                          dtype16(a), 0, cur_stream()) == 0)
       return;
   }
+  // up to four tokens: the weight as a stream over its rows.  The head of a model (whole tiles for every SM many times over)
+  // streams as fast on the tensor-core kernel.
+  if (force_bn == 0 && M <= 4 && epi <= 1) {
+    static int sms_of[64] = {};
+    int& sms = sms_of[a.get_device() & 63];
+    if (sms == 0) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a.get_device());
+    if (b200::gemv(out.data_ptr(), a.data_ptr(), w.data_ptr(), ptr(bias), ptr(residual), M, N, K, a.stride(0), w.stride(0),
+                   out.stride(0), ldr, epi == 1, dtype16(a), sms, cur_stream()) == 0)
+      return;
+  }
   // stream-K over CTA pairs for skinny problems: decode batches and narrow tensor-parallel shards (force_bn 2000
   // pins it).  Its scratch (partial tiles + arrival counters) is allocated once per device and stream-ordered
   // use is assumed, like every other op of this library.

@@ -255,6 +255,8 @@ void gemm_wna16(const void* A, int M, int lda, const void* Q, const void* scales
                 const int* block_expert, const int* total_padded, int grouped, int token_tile, int epi, int dtype,
                 cudaStream_t stream, void* status);
 // ---- small_gemm.cu
+int gemv(void* C, const void* A, const void* W, const void* bias, const void* residual, int M, int N, int K, int lda, int ldw,
+         int ldc, int ldr, int gate, int dtype, int sms, cudaStream_t stream);   // gemv.cu
 int small_gemm(void* C, const void* A, const void* W, const void* bias, int M, int N, int K, int lda, int ldw, int ldc,
                int dtype, int out_kind, cudaStream_t stream);
 // ---- fused_misc.cu
