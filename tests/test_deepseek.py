@@ -313,7 +313,7 @@ def test_mla_rope_insert_and_keys(dtype, T, H, absorbed, pitch):
     cache = torch.zeros(-(-(T + 9) // 16), 16, 576, dtype=dtype, device="cuda")
     want_cache = cache.clone()
     kv_c = ops.rms_norm(kv[:, :512].contiguous(), w, 1e-6)
-    k_pe, q_pe = kv[:, 512:].contiguous(), q[..., 128:].reshape(T, -1).contiguous()
+    k_pe, q_pe = kv[:, 512:].clone(memory_format=torch.contiguous_format), q[..., 128:].reshape(T, -1).clone()
     ops.rotary_embedding(pos, q_pe, k_pe, 64, cs, False)
     ops.concat_and_cache_mla(kv_c, k_pe, want_cache, slots)
     q2, qa = q.clone(), torch.zeros(absorbed, H, 576, dtype=dtype, device="cuda")

@@ -224,3 +224,19 @@ def test_grouped_products_without_padding(T, topk, E, N, K, epi):
     want = ops.gemm_grouped(torch.where(real[:, None], a, torch.zeros_like(a)), w, be, total, epi)
     assert torch.equal(got[real], want[real]) and bool(torch.isfinite(got[real]).all())
     ops.check_kernel_status(0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,K,N", [(1, 8, 8), (64, 2048, 2048), (5, 3000, 4104)])
+def test_gate_of_a_shared_expert(dtype, T, K, N):
+    """Rows shorter than a CTA and longer than one pass of it, strided tokens: an exact product up to fp32 sums, one rounding."""
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, 2 * K, generator=g).to(dtype).cuda()[:, :K]
+    w = (torch.randn(1, K, generator=g) / K ** 0.5).to(dtype).cuda()
+    y = torch.randn(T, N, generator=g).to(dtype).cuda()
+    with torch.no_grad():
+        got = ops.sigmoid_dot_scale(x, w, y)
+    want = torch.sigmoid(x.double() @ w.double().T) * y.double()
+    # one rounding to the type, of 8 or 11 significant bits; the sigmoid's exponential and the sum to 2^-18
+    torch.testing.assert_close(got.double(), want, rtol=(2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * 1.05, atol=1e-6)

@@ -454,6 +454,18 @@ def decode_num_splits(batch: int, num_kv_heads: int, max_seq_len: int, row_tiles
     return max(1, min(want, max(1, max_seq_len // 256), 32))
 
 
+def sigmoid_dot_scale(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
+    """``sigmoid(x . w)`` of each row times the row of ``y`` (the gate of a shared expert); ``w [1, K]``."""
+    ok = lambda a: a.dim() == 2 and a.dtype == x.dtype and a.stride(1) == 1 and a.stride(0) % 8 == 0 and a.shape[1] % 8 == 0 \
+        and a.data_ptr() % 16 == 0
+    if _use_cuda(x) and x.dtype in (torch.bfloat16, torch.float16) and ok(x) and ok(y) and ok(w) and w.shape == (1, x.shape[1]) \
+            and y.shape[0] == x.shape[0] and not torch.is_grad_enabled():
+        out = torch.empty(y.shape, dtype=y.dtype, device=y.device)
+        torch.ops.b200.sigmoid_dot_scale(out, x, w.view(-1), y)
+        return out
+    return (torch.sigmoid(torch.nn.functional.linear(x, w).float()) * y.float()).to(y.dtype)
+
+
 def decode_scratch(q_heads: int, kv_heads: int, head_size: int, device, sms: int = 148) -> torch.Tensor:
     """Zeroed scratch for ``paged_attention_decode``, which leaves its counters zero: one for the steps that follow one another in a
     stream (captured graphs).  Too small a one is not used."""

@@ -731,6 +731,16 @@ void gdn_run(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const
   const int rc = b200::gdn_recurrent(p, (int)q.size(2), (int)v.size(2), dtype16(q), cur_stream());
   TORCH_CHECK(rc == 0, "gdn_recurrent: head sizes must be 128 and value heads a multiple of q/k heads");
 }
+void sigmoid_dot_scale(Tensor& out, const Tensor& x, const Tensor& w, const Tensor& y) {
+  on_device_of(x, {&out, &w, &y}, {});
+  TORCH_CHECK(x.dim() == 2 && y.dim() == 2 && out.sizes() == y.sizes() && out.is_contiguous() && x.size(0) == y.size(0) &&
+                  w.is_contiguous() && w.numel() == x.size(1) && x.stride(1) == 1 && y.stride(1) == 1 &&
+                  x.scalar_type() == y.scalar_type() && w.scalar_type() == x.scalar_type() && out.scalar_type() == x.scalar_type(),
+              "sigmoid_dot_scale: out and y [T, N], x [T, K], w [K] of one 16-bit type");
+  const int rc = b200::sigmoid_dot_scale(out.data_ptr(), x.data_ptr(), w.data_ptr(), y.data_ptr(), x.size(0), (int)x.size(1),
+                                         (int)y.size(1), x.stride(0), y.stride(0), dtype16(x), cur_stream());
+  TORCH_CHECK(rc == 0, "sigmoid_dot_scale: rows must be 16-byte aligned");
+}
 void gdn_recurrent(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g,
                    const Tensor& beta, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
                    const optional<Tensor>& has_initial, double scale, bool l2norm) {
@@ -1022,6 +1032,7 @@ TORCH_LIBRARY_FRAGMENT(b200, m) {
   m.def("mla_expand_keys(Tensor(a!) out, Tensor kv, Tensor k_pe, int nope) -> ()", &mla_expand_keys);
   m.def("gdn_recurrent_ba(Tensor(a!) out, Tensor(b!) state, Tensor q, Tensor k, Tensor v, Tensor ba, Tensor a_log, Tensor dt_bias, Tensor query_start_loc, Tensor? state_idx, Tensor? has_initial, float scale, bool l2norm) -> ()", &gdn_recurrent_ba);
   m.def("gated_head_norm(Tensor(a!) out, Tensor o, Tensor z, Tensor? w, int dim, float eps) -> ()", &gated_head_norm);
+  m.def("sigmoid_dot_scale(Tensor(a!) out, Tensor x, Tensor w, Tensor y) -> ()", &sigmoid_dot_scale);
   m.def("gdn_recurrent(Tensor(a!) out, Tensor(b!) state, Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, Tensor query_start_loc, Tensor? state_idx, Tensor? has_initial, float scale, bool l2norm) -> ()", &gdn_recurrent);
   m.def("tq_slot_bytes(int kbits, int vbits) -> int", &tq_slot_bytes);
   m.def("tq_store(Tensor(a!) cache, Tensor k, Tensor v, Tensor slot_mapping, int kbits, int vbits, bool nc) -> ()", &tq_store);

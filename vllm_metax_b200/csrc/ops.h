@@ -356,6 +356,10 @@ struct MlaRopeInsertParams {
 void mla_rope_insert(const MlaRopeInsertParams& p, int dtype, cudaStream_t stream);
 void mla_expand_keys(void* out, const void* kv, const void* k_pe, int64_t tokens, int heads, int nope, int kv_dim,
                      cudaStream_t stream);
+// ---- activation.cu
+int sigmoid_dot_scale(void* out, const void* x, const void* w, const void* y, int64_t rows, int K, int N, int64_t x_stride,
+                      int64_t y_stride, int dtype, cudaStream_t stream);
+
 // ---- gdn.cu
 struct GdnLengths;
 struct GdnParams {

@@ -14,6 +14,7 @@ from typing import Iterable, Optional
 import torch
 import torch.nn as nn
 
+from .. import _custom_ops as ops
 from ..config import ModelConfig
 from ..layers.basic import RMSNorm
 from ..layers.fused_moe import FusedMoE
@@ -43,7 +44,7 @@ class SparseMoeBlock(nn.Module):
             return None
         y = self.shared_expert(x)
         if self.shared_expert_gate is not None:
-            y = (torch.sigmoid(torch.nn.functional.linear(x, self.shared_expert_gate.weight).float()) * y.float()).to(y.dtype)
+            y = ops.sigmoid_dot_scale(x, self.shared_expert_gate.weight, y)
         return y
 
     def forward(self, x):
