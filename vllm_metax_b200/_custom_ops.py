@@ -1034,12 +1034,10 @@ def wna16_gemm(x, qweight, scales, zeros, bits: int, group: int, *, bias=None, b
 
 
 # --------------------------------------------------------------------------- MLA
-def mla_decode_num_splits(tokens: int, heads: int, kv: int, window: int = 0, fp8: bool = False, tcgen05: bool = False) -> int:
+def mla_decode_num_splits(tokens: int, heads: int, kv: int, window: int = 0, fp8: bool = False) -> int:
     # heads per CTA as chosen by the kernel launcher (csrc/mla_decode.cu:mla_decode_heads_per_cta)
     hpc = 16 if heads <= 16 else (32 if (heads <= 32 or fp8) else 64)
     ctas = tokens * ((heads + hpc - 1) // hpc)
-    if tcgen05:
-        ctas = 2 * tokens * ((heads + 127) // 128)           # 128 heads x half the latent per CTA
     if window > 0:
         kv = min(kv, window)
     return 1 if ctas >= 148 else max(1, min((296 + ctas - 1) // ctas, kv // 256, 16))
@@ -1050,23 +1048,25 @@ def mla_decode(q, mla_cache, block_table, seq_lens, scale, *, query_start_loc=No
                kv_rank: int = 512, workspace=None):
     """Absorbed MLA over the latent cache (dense, or sparse with ``topk_indices [T, topk]``).
     ``q [T, H, 576]`` -> ``[T, H, 512]``.  ``impl``: 0 = choose, 1 = mma.sync kernel, 2 = tcgen05 kernel (dense 16-bit
-    caches; csrc/mla_decode_tcgen05.cu) or fail.  "Choose" takes the tcgen05 kernel for 64 heads per rank or more only
-    with ``B200_MLA_TCGEN05=1``.  Other sizes: cache rows ``[kv_rank latent | rotated part | padding]``, queries of the same
+    caches; csrc/mla_decode_tcgen05.cu, which divides the work itself whatever ``num_splits``) or fail.  "Choose" takes the tcgen05
+    kernel for 64 heads per rank or more, unless results must not depend on the batch or ``B200_MLA_TCGEN05=0``.  Other sizes: cache rows ``[kv_rank latent | rotated part | padding]``, queries of the same
     row length, output ``[T, H, kv_rank]``.  ``window`` > 0: only the last ``window`` visible positions.  ``workspace``: for
     the partial results of splits, where the caller owns it (fp32)."""
     if _use_cuda(q):
         T, H, _ = q.shape
         if q.dtype == torch.float32 or kv_rank > 512:      # CUDA-core kernel: one pass
             num_splits = 1
-        if impl == 0 and not envs.B200_MLA_TCGEN05:
+        if impl == 0 and (not envs.B200_MLA_TCGEN05 or batch_invariant()):
             impl = 1
         out = torch.empty(T, H, kv_rank, dtype=q.dtype, device=q.device) if out is None else out
         if num_splits <= 0 and batch_invariant():
             num_splits = 1
         if num_splits <= 0:
             kv = topk_indices.shape[1] if topk_indices is not None else (max_seq_len or 4096)
-            tcgen05 = impl != 1 and topk_indices is None and mla_cache.dtype != torch.uint8 and (impl == 2 or H >= 64)
-            num_splits = mla_decode_num_splits(T, H, kv, window, mla_cache.dtype == torch.uint8, tcgen05)
+            num_splits = mla_decode_num_splits(T, H, kv, window, mla_cache.dtype == torch.uint8)
+            if impl != 1 and (impl == 2 or H >= 64) and topk_indices is None and window <= 0 and T <= 1024 and kv_rank == 512 \
+                    and mla_cache.dtype == q.dtype and q.shape[2] == mla_cache.shape[2] == 576 and mla_cache.shape[1] % 32 == 0:
+                num_splits = 1                                   # (that kernel divides the work itself)
         ws = workspace
         if num_splits > 1 and (ws is None or ws.numel() < num_splits * T * H * (kv_rank + 1)):
             ws = _decode_workspace(q.device, num_splits * T * H * (kv_rank + 1))

@@ -40,6 +40,21 @@ void mla_decode(Tensor& out, const Tensor& q, const Tensor& cache, const Tensor&
   p.total_tokens = q.size(0);
   p.batch = seq_lens.size(0);
   p.scale = (float)scale;
+  if (impl != 1 && !rec && q.scalar_type() != at::kFloat && (impl == 2 || p.num_heads >= 64) && b200::mla_decode_tc_serves(p)) {
+    if (p.total_tokens <= 0) return;
+    const c10::cuda::CUDAGuard guard(q.device());
+    static int sms_of[64] = {};
+    int& sms = sms_of[q.get_device() & 63];
+    if (sms == 0) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, q.get_device());
+    int64_t floats = 0, ints = 0;
+    b200::mla_decode_tc_scratch(p, sms, &floats, &ints);
+    const Tensor own = at::empty({floats + ints}, q.options().dtype(at::kFloat));
+    int* counters = reinterpret_cast<int*>(own.data_ptr<float>() + floats);
+    C10_CUDA_CHECK(cudaMemsetAsync(counters, 0, ints * sizeof(int), cur_stream()));
+    p.status = reinterpret_cast<b200::StatusWord*>(status_ptr(q));
+    b200::mla_decode_tc(p, dtype16(q), sms, own.data_ptr<float>(), counters, cur_stream());
+    return;
+  }
   if (p.num_splits > 1) {
     const int64_t need = p.num_splits * (int64_t)p.total_tokens * p.num_heads * (p.kv_rank + 1);
     TORCH_CHECK(workspace.has_value() && workspace->numel() >= need, "mla_decode workspace too small");
@@ -50,7 +65,9 @@ void mla_decode(Tensor& out, const Tensor& q, const Tensor& cache, const Tensor&
   const c10::cuda::CUDAGuard guard(q.device());
   // fp32 caches, and 16-bit sizes outside the tensor-core kernel's range, run on the CUDA cores
   const bool f32 = q.scalar_type() == at::kFloat;
-  int rc = f32 ? -1 : b200::mla_decode(p, rec, dtype16(q), cur_stream(), (int)impl);
+  // asked for, the tcgen05 kernel stands for itself; windows, other latent sizes and more tokens than it lists go on
+  const bool alone = impl == 2 && p.window <= 0 && p.kv_rank == 512 && p.q_dim == 576 && p.row_elems == 576 && p.total_tokens <= 1024;
+  int rc = f32 || alone ? -1 : b200::mla_decode(p, rec, dtype16(q), cur_stream());
   if (rc != 0 && impl != 2 && !rec && !topk_indices.has_value() && !lse_out.has_value() && p.num_splits == 1)
     rc = b200::latent_attn_simt(p, dtype_code(q), cur_stream());
   TORCH_CHECK(rc == 0, "mla_decode: no kernel serves this call (impl ", impl, ", latent ", p.kv_rank, ", row ", p.row_elems, ")");

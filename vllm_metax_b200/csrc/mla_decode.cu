@@ -13,6 +13,7 @@
 // `window` of them.
 // Sparse (DeepSeek sparse attention): only the positions listed in topk_indices[t, :] (-1 = none).
 //
+// Dense 16-bit caches of these sizes with 64 heads or more take mla_decode_tcgen05.cu instead.
 // One CTA = one query token x 16 / 32 / 64 heads x one KV split; 8 warps walk 64-token latent tiles through a
 // two-slot cp.async ring (see the kernel's comment for the division of work).  The latent rows of a token are
 // read once per CTA, so the more heads a CTA covers the less cache traffic; with 16 heads per rank (TP 8 of 128
@@ -507,7 +508,7 @@ static void launch_mla_reduce(const MlaDecodeParams& p, cudaStream_t stream) {
       (T*)p.out, p.lse_out, p.part_out, p.part_lse, p.num_splits, p.total_tokens, p.num_heads, p.kv_rank);
 }
 
-int mla_decode(const MlaDecodeParams& p, int fp8_records, int dtype, cudaStream_t stream, int impl) {
+int mla_decode(const MlaDecodeParams& p, int fp8_records, int dtype, cudaStream_t stream) {
   if (p.total_tokens <= 0) return 0;
   bool done = false;
   if (p.kv_rank != kMlaDV || p.q_dim != kMlaD || (!fp8_records && p.row_elems != kMlaD)) {
@@ -515,11 +516,7 @@ int mla_decode(const MlaDecodeParams& p, int fp8_records, int dtype, cudaStream_
     const int rc = dtype == 0 ? launch_mla_sizes<__nv_bfloat16>(p, stream) : launch_mla_sizes<__half>(p, stream);
     if (rc != 0) return rc;
     done = true;
-  } else if (p.window > 0) {
-    impl = 1;                                   // the tcgen05 kernel has no window
   }
-  if (!done && impl != 1 && !fp8_records && (impl == 2 || p.num_heads >= 64)) done = mla_decode_tc(p, dtype, stream) == 0;
-  if (!done && impl == 2) return -1;
   if (!done) {
     if (dtype == 0) {
       if (fp8_records) launch_mla<__nv_bfloat16, true>(p, stream); else launch_mla<__nv_bfloat16, false>(p, stream);

@@ -576,9 +576,11 @@ int reduce_rms(const ReduceRmsParams& p, int dtype, cudaStream_t stream);
 // ---- mla_decode.cu
 // impl: 0 = choose (tcgen05 kernel for dense 16-bit caches from 64 heads per rank up), 1 = mma.sync kernel,
 // 2 = tcgen05 kernel or fail.  Returns 0, or -1 when impl 2 was asked for and that kernel does not serve the call.
-int mla_decode(const MlaDecodeParams& p, int fp8_records, int dtype, cudaStream_t stream, int impl = 1);
-// ---- mla_decode_tcgen05.cu: 0 = launched, -1 = not served
-int mla_decode_tc(const MlaDecodeParams& p, int dtype, cudaStream_t stream);
+int mla_decode(const MlaDecodeParams& p, int fp8_records, int dtype, cudaStream_t stream);
+// ---- mla_decode_tcgen05.cu
+bool mla_decode_tc_serves(const MlaDecodeParams& p);
+void mla_decode_tc_scratch(const MlaDecodeParams& p, int sms, int64_t* floats, int64_t* ints);
+void mla_decode_tc(const MlaDecodeParams& p, int dtype, int sms, float* parts, int* counters, cudaStream_t stream);
 // ---- indexer.cu
 void indexer_logits(float* logits, int64_t logits_stride, const void* q, const float* w, const void* cache,
                     const int* block_table, int max_blocks, const int* seq_lens, const int* query_start_loc,

@@ -65,7 +65,7 @@ environment_variables: dict[str, Callable[[], Any]] = {
     "B200_GDN_CHUNKED_MIN_TOKENS": _int("B200_GDN_CHUNKED_MIN_TOKENS", 256),
     # Absorbed-MLA decode on tcgen05 (csrc/mla_decode_tcgen05.cu) for dense 16-bit caches from 64 heads per rank up;
     # 0 = the mma.sync kernel unless a call asks for the tcgen05 one.
-    "B200_MLA_TCGEN05": _flag("B200_MLA_TCGEN05", "0"),
+    "B200_MLA_TCGEN05": _flag("B200_MLA_TCGEN05", "1"),
     # Prepare step k + 1 on the host (schedule, staging buffers) while the device runs step k; 0 = strictly in turn.
     "B200_OVERLAP_SCHEDULING": _flag("B200_OVERLAP_SCHEDULING", "1"),
     # Pipeline parallel: keep one step per stage in flight (disjoint request sets) instead of running lock-step.
