@@ -612,3 +612,66 @@ def test_few_tokens_against_a_weight(dtype, M, N, K, kernel_status_ok):
         got = ops.gemm_silu_mul(a, w).double()
         # either factor may be the neighbouring number of its type, then one rounding
         torch.testing.assert_close(got, torch.nn.functional.silu(gate) * up, rtol=5 * eps, atol=1e-4)
+
+
+def _decode_case(Hq, Hkv, dqk, dv, lens, dtype, int8=False, bs=64, seed=0):
+    """Queries of one token per sequence, a shuffled cache (16 bits: pages for ``_decode_views``), and the result in fp32 from the
+    cache's numbers with a bound."""
+    g = torch.Generator().manual_seed(seed + Hq * dqk)
+    nb = [-(-n // bs) for n in lens]
+    table, perm, at = torch.zeros(len(lens), max(nb) + 1, dtype=torch.int32), torch.randperm(sum(nb) + 1, generator=g), 0
+    for i, n in enumerate(nb):
+        table[i, :n] = perm[at: at + n]
+        at += n
+    q = torch.randn(len(lens), Hq, dqk, generator=g).to(dtype)
+    scales = None
+    if int8:
+        kv = torch.randint(-127, 128, (sum(nb) + 1, 2, bs, Hkv, dqk), generator=g, dtype=torch.int8)
+        scales = torch.rand(sum(nb) + 1, 2, bs, Hkv, generator=g) * 0.012 + 0.004
+        k, v = (kv[:, j].float() * scales[:, j, ..., None] for j in (0, 1))
+        cache = kv
+    else:
+        cache = torch.randn(sum(nb) + 1, bs * Hkv * (dqk + dv), generator=g).to(dtype)       # a page: keys, then values
+        k, v = (t.float() for t in _decode_views(cache, bs, Hkv, dqk, dv))
+    want, mass = torch.zeros(len(lens), Hq, dv), torch.zeros(len(lens), Hq, dv)
+    for i, n in enumerate(lens):
+        if n:
+            kk, vv = (t[table[i, : nb[i]].long()].reshape(-1, Hkv, t.shape[-1])[:n].repeat_interleave(Hq // Hkv, 1) for t in (k, v))
+            p = (torch.einsum("hd,nhd->hn", q[i].float(), kk) * dqk ** -0.5).softmax(-1)
+            want[i], mass[i] = torch.einsum("hn,nhd->hd", p, vv), torch.einsum("hn,nhd->hd", p, vv.abs())
+    # a weight is rounded to 16 bits, and once more the result
+    u = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12
+    return q, cache, scales, table, torch.tensor(lens, dtype=torch.int32), want, 2 * u * want.abs() + 2 * u * mass + 1e-5
+
+
+def _decode_views(pages, bs, Hkv, dqk, dv):
+    n = bs * Hkv * dqk
+    return pages[:, :n].unflatten(1, (bs, Hkv, dqk)), pages[:, n:].unflatten(1, (bs, Hkv, dv))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("Hq,Hkv,dqk,dv", [(8, 1, 256, 256), (10, 1, 256, 256), (16, 1, 256, 256), (24, 2, 192, 192), (18, 2, 160, 160),
+                                           (12, 1, 256, 128), (9, 1, 128, 136), (17, 1, 256, 256)])
+def test_decode_of_wide_heads_in_large_groups(dtype, Hq, Hkv, dqk, dv):
+    """Heads wider than 128 in groups around 8 and 16 query heads per key head, where the kernels for one token per sequence part:
+    a call of its own, one with a kept scratch, and a replayed graph."""
+    lens = [1, 900, 0, 65, 64, 2100, 17]
+    q, cache, _, table, sl, want, bound = _decode_case(Hq, Hkv, dqk, dv, lens, dtype)
+    qd, td, ld, cd = q.cuda(), table.cuda(), sl.cuda(), _decode_views(cache.cuda(), 64, Hkv, dqk, dv)
+    out = torch.full((len(lens), Hq, dv), float("nan"), dtype=dtype, device="cuda")
+    ws = torch.empty(32 * len(lens) * Hq * (dv + 1), device="cuda")
+    run = lambda **kw: ops.paged_attention_decode(qd, cd, td, ld, dqk ** -0.5, out=out, max_seq_len=max(lens), workspace=ws, **kw)
+    check = lambda: bool(((out.float().cpu() - want).abs() <= bound).all())
+    for kw in ({}, dict(scratch=ops.decode_scratch(Hq, Hkv, max(dqk, dv), "cuda"))):
+        out.fill_(float("nan"))
+        run(**kw)
+        assert check()
+        stream = torch.cuda.Stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            run(**kw)
+        for _ in range(2):
+            out.fill_(float("nan"))
+            graph.replay()
+            assert check()

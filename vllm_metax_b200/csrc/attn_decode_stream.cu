@@ -33,7 +33,7 @@
 namespace b200 {
 namespace {
 
-constexpr int kWarps = 4, kThreads = 128, kTile = 16, kStages = 3, kMaxBatch = 1024;
+constexpr int kWarps = 4, kThreads = 128, kTile = 16, kStages = 3, kMaxBatch = 1024, kMaxSmem = 227 * 1024;
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 
 template <int D, int KIND, int ROWS>
@@ -526,25 +526,34 @@ paged_decode_stream_kernel(const DecodeParams p, int batch, float* parts, int* c
 }
 
 template <typename T, int D, int KIND, int ROWS>
-int run(const DecodeParams& p, int batch, int sms, float* parts, int* counters, bool early, int64_t* floats, cudaStream_t stream) {
+cudaError_t run(const DecodeParams& p, int batch, int sms, float* parts, int* counters, bool early, int64_t* floats, cudaStream_t stream) {
   using S = StreamSmem<D, KIND, ROWS>;
   const int bytes = S::total(batch);
   const int fit = D > 128 ? 1 : KIND == 1 ? 3 : 2, room = 228 * 1024 / (bytes + 1024);
   const int slots = sms * (fit < room ? fit : room), groups = slots / p.num_kv_heads > 1 ? slots / p.num_kv_heads : 1;
   if (floats != nullptr) {
     *floats = (int64_t)groups * p.num_kv_heads * 2 * (S::kState / 4);
-    return 0;
+    return cudaSuccess;
   }
   auto kern = paged_decode_stream_kernel<T, D, KIND, ROWS>;
   // a per-device attribute of the kernel: set on every launch (cheap) rather than once per process
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (early) pdl_run(kern, groups * p.num_kv_heads, kThreads, bytes, stream, p, batch, parts, counters);
-  else kern<<<groups * p.num_kv_heads, kThreads, bytes, stream>>>(p, batch, parts, counters);
-  return 0;
+  const cudaError_t set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (set != cudaSuccess) return set;
+  if (early) return pdl_run(kern, groups * p.num_kv_heads, kThreads, bytes, stream, p, batch, parts, counters);
+  kern<<<groups * p.num_kv_heads, kThreads, bytes, stream>>>(p, batch, parts, counters);
+  return cudaPeekAtLastError();
+}
+
+// Shared memory of the instantiation that `dispatch` takes.
+int smem_of(int group, int head, int kind, int batch) {
+#define TOTAL(D, K) (group <= 8 ? StreamSmem<D, K, 8>::total(batch) : StreamSmem<D, K, 16>::total(batch))
+  if (kind == 1) return TOTAL(128, 1);
+  return head <= 64 ? TOTAL(64, 0) : head <= 128 ? TOTAL(128, 0) : TOTAL(256, 0);
+#undef TOTAL
 }
 
 template <typename T>
-int dispatch(const DecodeParams& p, int kind, int batch, int sms, float* parts, int* counters, bool early, int64_t* floats,
+cudaError_t dispatch(const DecodeParams& p, int kind, int batch, int sms, float* parts, int* counters, bool early, int64_t* floats,
              cudaStream_t stream) {
   const int g = p.num_q_heads / p.num_kv_heads, head = p.dqk > p.dv ? p.dqk : p.dv;
 #define RUN(D, K) (g <= 8 ? run<T, D, K, 8>(p, batch, sms, parts, counters, early, floats, stream) \
@@ -558,11 +567,12 @@ int dispatch(const DecodeParams& p, int kind, int batch, int sms, float* parts, 
 
 }  // namespace
 
-// Whether the kernel serves a step of `batch` sequences of one token each.
+// Whether the kernel serves a step of `batch` sequences of one token each.  16 rows of heads wider than 128 would take 240 KB of
+// shared memory, of which a CTA may have 227: these stay in attn_decode.cu.
 bool decode_stream_serves(const DecodeParams& p, int kv_kind, int batch) {
   const int head = p.dqk > p.dv ? p.dqk : p.dv;
   if (batch <= 0 || batch > kMaxBatch || p.num_q_heads > 16 * p.num_kv_heads || batch * p.num_kv_heads > kDecodeCounters ||
-      p.block_size % kTile != 0)
+      p.block_size % kTile != 0 || smem_of(p.num_q_heads / p.num_kv_heads, head, kv_kind, batch) > kMaxSmem)
     return false;
   return kv_kind == 0 ? p.dqk % 8 == 0 && p.dv % 8 == 0 && head <= 256 : kv_kind == 1 && p.dqk == 128 && p.dv == 128;
 }
@@ -574,10 +584,10 @@ void decode_stream_scratch(const DecodeParams& p, int kv_kind, int dtype, int ba
   else dispatch<__half>(p, kv_kind, batch, sms, nullptr, nullptr, false, floats, nullptr);
 }
 
-void decode_stream(const DecodeParams& p, int kv_kind, int dtype, int batch, int sms, float* parts, int* counters, bool early,
-                   cudaStream_t stream) {
-  if (dtype == 0) dispatch<__nv_bfloat16>(p, kv_kind, batch, sms, parts, counters, early, nullptr, stream);
-  else dispatch<__half>(p, kv_kind, batch, sms, parts, counters, early, nullptr, stream);
+cudaError_t decode_stream(const DecodeParams& p, int kv_kind, int dtype, int batch, int sms, float* parts, int* counters, bool early,
+                          cudaStream_t stream) {
+  return dtype == 0 ? dispatch<__nv_bfloat16>(p, kv_kind, batch, sms, parts, counters, early, nullptr, stream)
+                    : dispatch<__half>(p, kv_kind, batch, sms, parts, counters, early, nullptr, stream);
 }
 
 }  // namespace b200

@@ -86,8 +86,8 @@ void paged_attention_decode(Tensor& out, const Tensor& q, const Tensor& k_cache,
     const Tensor own = given ? *scratch : at::empty({floats + b200::kDecodeCounters}, q.options().dtype(at::kFloat));
     int* counters = reinterpret_cast<int*>(own.data_ptr<float>());
     if (!given) C10_CUDA_CHECK(cudaMemsetAsync(counters, 0, batch * p.num_kv_heads * sizeof(int), cur_stream()));
-    b200::decode_stream(p, kind, dtype16(q), (int)batch, sms, own.data_ptr<float>() + b200::kDecodeCounters, counters, given,
-                        cur_stream());
+    C10_CUDA_CHECK(b200::decode_stream(p, kind, dtype16(q), (int)batch, sms, own.data_ptr<float>() + b200::kDecodeCounters, counters,
+                                       given, cur_stream()));
     return;
   }
   if (p.num_splits > 1) {

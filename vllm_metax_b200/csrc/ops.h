@@ -179,8 +179,8 @@ void act_and_mul_quant(void* out_q, float* scale_out, const float* scale_in, con
 // ---- attention
 bool decode_stream_serves(const DecodeParams& p, int kv_kind, int batch);
 void decode_stream_scratch(const DecodeParams& p, int kv_kind, int dtype, int batch, int sms, int64_t* floats);
-void decode_stream(const DecodeParams& p, int kv_kind, int dtype, int batch, int sms, float* parts, int* counters, bool early,
-                   cudaStream_t stream);
+cudaError_t decode_stream(const DecodeParams& p, int kv_kind, int dtype, int batch, int sms, float* parts, int* counters, bool early,
+                          cudaStream_t stream);
 constexpr int kDecodeCounters = 16384;   // ints in front of a decode step's scratch
 int paged_attention_decode(const DecodeParams& p, int kv_kind, int dtype, int batch, int max_q_len, cudaStream_t stream);
 // paged_attn_simt.cu: the same on the CUDA cores for fp32 caches and head sizes beyond the tensor-core kernels
