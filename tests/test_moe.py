@@ -240,3 +240,52 @@ def test_gate_of_a_shared_expert(dtype, T, K, N):
     want = torch.sigmoid(x.double() @ w.double().T) * y.double()
     # one rounding to the type, of 8 or 11 significant bits; the sigmoid's exponential and the sum to 2^-18
     torch.testing.assert_close(got.double(), want, rtol=(2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * 1.05, atol=1e-6)
+
+
+def test_kernels_that_start_early_wait_before_their_loads():
+    """A kernel that may run beside the one in front of it waits first, and its loads are none that a compiler may move in front
+    of the wait: those through const pointers with ``__restrict__``."""
+    import pathlib
+    import re
+
+    found = 0
+    for src in sorted((pathlib.Path(ops.__file__).parent / "csrc").glob("*.cu")):
+        text = re.sub(r"//[^\n]*", "", src.read_text())
+        early = set(re.findall(r"pdl_run\((\w+)", text)) - {"kern"} | set(re.findall(r"auto kern = (\w+)", text) if "pdl_" in text else [])
+        for head, body in re.findall(r"__global__([^{;]*)\{(.*?)\n\}", text, re.S):
+            name = re.findall(r"(\w+)\s*\(", re.sub(r"__launch_bounds__\s*\((?:[^()]|\([^()]*\))*\)", "", head))[0]
+            if name not in early and "pdl_wait" not in body and "pdl_trigger" not in body:
+                continue
+            found += 1
+            assert "pdl_wait();" in body, (src.name, name)
+            assert "__restrict__" not in head, (src.name, name)
+    assert found >= 9
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,N,K", [(1, 2048, 512), (2, 2048, 4096), (3, 7168, 2048), (4, 512, 2048), (33, 512, 2048), (64, 256, 512)])
+def test_gate_behind_a_product_in_a_graph(dtype, T, N, K, kernel_status_ok):
+    """The gate starts while the product in front of it, which makes its rows, still runs: replays over changing inputs give what
+    the two calls give one after the other."""
+    g = torch.Generator().manual_seed(T)
+    h = torch.empty(T, K, dtype=dtype, device="cuda")
+    x = torch.empty(T, 2048, dtype=dtype, device="cuda")
+    w = (torch.randn(N, K, generator=g) / K ** 0.5).to(dtype).cuda()
+    gate = (torch.randn(1, 2048, generator=g) / 50).to(dtype).cuda()
+    first = lambda a: torch.mul(a, 2.0)                     # (a kernel in front of the product, so that this starts early too)
+    step = lambda: ops.sigmoid_dot_scale(x, gate, ops.gemm(first(h), w))
+    with torch.no_grad():
+        h.zero_(), x.zero_()
+        step()
+        torch.cuda.synchronize()
+        graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=stream):
+            for _ in range(4):                              # (several in a row: the one in front of a product is a gate)
+                out = step()
+        for _ in range(20):
+            h.copy_(torch.randn(T, K, generator=g))
+            x.copy_(torch.randn(T, 2048, generator=g))
+            want = step().clone()
+            graph.replay()
+            assert torch.equal(out, want)

@@ -58,8 +58,7 @@ __device__ __forceinline__ float gated(int act, float g, float u, float p0, floa
 // 57 us for 3949 rows; 2.3 and 15 us here, bound by its launch and by the rows' bytes.
 template <typename T>
 __global__ void __launch_bounds__(256)
-sigmoid_dot_scale_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ y, int K, int N,
-                         int64_t x_stride, int64_t y_stride) {
+sigmoid_dot_scale_kernel(T* out, const T* x, const T* w, const T* y, int K, int N, int64_t x_stride, int64_t y_stride) {
   pdl_trigger();
   pdl_wait();
   __shared__ float red[32];

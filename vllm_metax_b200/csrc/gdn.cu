@@ -397,7 +397,7 @@ constexpr int kC = 16;                     // tokens of a chunk
 constexpr int kChunkFloats = 2 * kC * kC + 5 * kC;   // T, M; factors a, beta, c, w; e^G of the last token
 
 // The chunk of index `at` in the order of the sequences: its sequence and first token, or false behind the last.  A whole warp.
-__device__ __forceinline__ bool gdn_locate(const int* __restrict__ qsl, int batch, int at, int lane, int& seq, int& first, int& end) {
+__device__ __forceinline__ bool gdn_locate(const int* qsl, int batch, int at, int lane, int& seq, int& first, int& end) {
   int before = 0;
   for (int b0 = 0; b0 < batch; b0 += 32) {
     const int b = b0 + lane;
@@ -424,7 +424,7 @@ __device__ __forceinline__ bool gdn_locate(const int* __restrict__ qsl, int batc
 
 // Rows t0 .. of n tokens, kD entries each, as bf16 with swizzled 16-byte chunks; rows from n on are zero.
 template <bool VEC>
-__device__ __forceinline__ void gdn_copy_rows(__nv_bfloat16* dst, const __nv_bfloat16* __restrict__ src, int64_t stride, int n, int tid,
+__device__ __forceinline__ void gdn_copy_rows(__nv_bfloat16* dst, const __nv_bfloat16* src, int64_t stride, int n, int tid,
                                               int threads) {
   for (int i = tid; i < kC * (kD / 8); i += threads) {
     const int r = i / (kD / 8), c = i % (kD / 8);

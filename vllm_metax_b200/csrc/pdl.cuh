@@ -3,8 +3,8 @@
 //
 // A kernel launched by pdl_run calls pdl_wait() in every thread before it touches anything that an earlier kernel may write or
 // read - weights too, which a copy just before may have filled; a prefetch into L2, the point where all accesses meet, is the one
-// thing that may come earlier.  Its pointer parameters carry no __restrict__: a load through a const one counts as a read of
-// unchanging memory, which the compiler is free to move in front of the wait.  Only a launch that is captured into a graph right
+// thing that may come earlier.  Pointers in a file of such kernels carry no __restrict__: a load through a const one counts as a
+// read of unchanging memory, which the compiler is free to move in front of the wait.  Only a launch that is captured into a graph right
 // behind another kernel may start early: the wait covers kernels, and what else stands in front - small host-to-device copies, a
 // memset, several nodes - has its ordinary order.
 // pdl_trigger() lets the next kernel start as soon as every CTA of this one has got that far; it says nothing about results, for
