@@ -251,3 +251,18 @@ def test_fp8_grouped_mm_without_padding(T, topk, E, N, K):
         want = ad[e == i] @ wd.T
         torch.testing.assert_close(out[rows[e == i]].double(), want, rtol=2.0 ** -8 * 1.01, atol=1e-5 * float(want.abs().max()))
     ops.check_kernel_status(0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,K", [(2112, 7168), (576, 2048), (7168, 2304)])
+def test_fp8_block_scaled_rows_alone_and_in_company(N, K, monkeypatch, kernel_status_ok):
+    """With results that must not depend on the batch, a row's product has the same bits alone and among any number of others."""
+    monkeypatch.setattr(ops, "_batch_invariant", True)
+    g = torch.Generator().manual_seed(N)
+    a = torch.randn(2100, K, generator=g).to(torch.float8_e4m3fn).cuda()
+    w = torch.randn(N, K, generator=g).to(torch.float8_e4m3fn).cuda()
+    a_s = (torch.rand(2100, K // 128, generator=g) + 0.5).cuda()
+    w_s = (torch.rand(-(-N // 128), K // 128, generator=g) + 0.5).cuda()
+    want = ops.fp8_block_scaled_mm(a, a_s, w, w_s)
+    for M in (1, 64, 130, 700):
+        assert torch.equal(ops.fp8_block_scaled_mm(a[:M], a_s[:M], w, w_s), want[:M])

@@ -951,7 +951,7 @@ def fp8_block_scaled_mm(aq, a_scale, wq, w_scale, out_dtype=torch.bfloat16, bloc
         n = wq.shape[-2]
         out = torch.empty(aq.shape[0], n, dtype=out_dtype, device=aq.device)
         torch.ops.b200.gemm_fp8_blockscale(out, aq, a_scale.contiguous(), wq, w_scale.contiguous(), block_expert,
-                                           total_padded, sorted_ids, numel)
+                                           total_padded, sorted_ids, numel, not batch_invariant())
         return out
     if wq.dim() == 2:
         return ref.fp8_block_scaled_mm(aq, a_scale, wq, w_scale, out_dtype)

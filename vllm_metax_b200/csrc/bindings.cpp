@@ -199,7 +199,7 @@ void merge_attn_states(Tensor& out, const optional<Tensor>& out_lse, const Tenso
 }
 void gemm_fp8_blockscale(Tensor& out, const Tensor& a, const Tensor& a_scale, const Tensor& w, const Tensor& w_scale,
                          const optional<Tensor>& block_expert, const optional<Tensor>& total_padded,
-                         const optional<Tensor>& sorted_ids, int64_t numel) {
+                         const optional<Tensor>& sorted_ids, int64_t numel, bool cut) {
   const bool grouped = w.dim() == 3;
   TORCH_CHECK(a.dim() == 2 && a.stride(1) == 1 && w.is_contiguous() && a_scale.is_contiguous() && w_scale.is_contiguous());
   TORCH_CHECK(a.element_size() == 1 && w.element_size() == 1 && a.size(1) % 128 == 0 && a.stride(0) % 16 == 0);
@@ -217,7 +217,7 @@ void gemm_fp8_blockscale(Tensor& out, const Tensor& a, const Tensor& a_scale, co
   int64_t floats = 0, counters = 0;
   Tensor scratch;                                   // of this call alone: any stream, any thread
   int* zero = nullptr;
-  if (!grouped) b200::gemm_fp8_scratch(M, N, K, sms, &floats, &counters);
+  if (!grouped && cut) b200::gemm_fp8_scratch(M, N, K, sms, &floats, &counters);
   if (floats > 0) {
     scratch = at::empty({floats + counters}, a_scale.options());
     zero = reinterpret_cast<int*>(scratch.data_ptr<float>() + floats);
@@ -1059,7 +1059,7 @@ TORCH_LIBRARY_FRAGMENT(b200, m) {
   m.def("scaled_fp8_quant(Tensor(a!) q, Tensor(b!) scale, Tensor x, int mode, float scale_ub) -> ()", &scaled_fp8_quant);
   m.def("scaled_int8_quant(Tensor(a!) q, Tensor(b!) scale, Tensor(c!)? azp, Tensor x, int mode) -> ()", &scaled_int8_quant);
   m.def("merge_attn_states(Tensor(a!) out, Tensor(b!)? out_lse, Tensor p_out, Tensor p_lse, Tensor s_out, Tensor s_lse) -> ()", &merge_attn_states);
-  m.def("gemm_fp8_blockscale(Tensor(a!) out, Tensor a, Tensor a_scale, Tensor w, Tensor w_scale, Tensor? block_expert, Tensor? total_padded, Tensor? sorted_ids=None, int numel=0) -> ()", &gemm_fp8_blockscale);
+  m.def("gemm_fp8_blockscale(Tensor(a!) out, Tensor a, Tensor a_scale, Tensor w, Tensor w_scale, Tensor? block_expert, Tensor? total_padded, Tensor? sorted_ids=None, int numel=0, bool cut=True) -> ()", &gemm_fp8_blockscale);
   m.def("scaled_mm(Tensor(a!) out, Tensor a, Tensor w, Tensor a_scale, Tensor w_scale, Tensor? azp, Tensor? azp_adj, Tensor? bias, Tensor? block_expert, Tensor? total_padded) -> ()", &scaled_mm);
   m.def("wna16_gemm(Tensor(a!) out, Tensor a, Tensor q, Tensor scales, Tensor? zeros, int bits, int group, Tensor? bias, Tensor? block_expert, Tensor? total_padded, int token_tile, int epi) -> ()", &wna16_gemm);
   m.def("indexer_logits(Tensor(a!) logits, Tensor q, Tensor w, Tensor cache, Tensor block_table, Tensor seq_lens, Tensor query_start_loc, int block_size, int max_len, bool int8, int max_query_len, int impl) -> ()", &indexer_logits);

@@ -14,7 +14,8 @@
 // Dense tiles go down M first within groups of kGroupM row blocks, so that the CTAs of a wave share weights and A stays in L2.
 // With few tiles (decode rows, narrow products) the (tile, k block) space is cut into one contiguous range per CTA (stream-K):
 // a CTA whose range covers part of a tile leaves an fp32 partial in a slot of its own, and the one that arrives last at the tile
-// adds them in CTA order.  Nobody waits.
+// adds them in CTA order.  Nobody waits.  Where K is cut follows the number of rows: results that must not depend on the batch take
+// whole tiles, whose sums run through K in one order whatever the tile.
 // Grouped mode: A is the expert-sorted padded activation matrix, W [E, N, K], w_scale
 // [E, N/128, K/128]; block_expert / total_padded as in gemm_grouped_tcgen05.cu.  With `sorted_ids`, rows of padding (at a block's
 // end) are neither read, folded nor written: with a handful of rows per expert they are most of a block.
