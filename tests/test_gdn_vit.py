@@ -310,3 +310,29 @@ def test_gdn_gates_and_norm_in_the_kernels():
         y = gdn.gated_head_norm(o1.reshape(T, -1), z, None, d)
         want = o1.float() * torch.sigmoid(z.reshape(T, -1, d).float())
         torch.testing.assert_close(y.view(T, -1, d).float(), want, rtol=2.0 ** -7, atol=1e-6)
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gdn_rows_alone_and_in_company(dtype, monkeypatch):
+    """With results that must not depend on the batch, a decode row and a prompt have the same outputs and states, bit for bit,
+    alone, beside one another, and with the prompt cut in two."""
+    from vllm_metax_b200 import _custom_ops as ops
+    from vllm_metax_b200.ops.gdn import gated_delta_rule, gated_delta_rule_ba
+
+    monkeypatch.setattr(ops, "_batch_invariant", True)
+    q, k, v, g, beta, _, state, _, _ = _gdn_case(dtype, seed=11, lens=(1, 50))
+    ba = torch.randn(51, 8, generator=torch.Generator().manual_seed(12)).to(dtype)
+    a_log, dt = torch.zeros(4), torch.ones(4)
+    cuda = lambda *ts: [t.cuda() for t in ts]
+    ints = lambda *x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    q, k, v, g, beta, ba, a_log, dt = cuda(q, k, v, g, beta, ba, a_log, dt)
+    for gates in (lambda r: (gated_delta_rule, (g[r], beta[r])), lambda r: (gated_delta_rule_ba, (ba[r], a_log, dt))):
+        def run(lo, hi, qsl, slots, s):
+            fn, more = gates(slice(lo, hi))
+            return fn(q[lo:hi], k[lo:hi], v[lo:hi], *more, qsl, s, slots, torch.ones_like(slots))
+
+        s_all, s_cut = state.cuda(), state.cuda()
+        want = run(0, 51, ints(0, 1, 51), ints(2, 0), s_all)
+        parts = [run(0, 1, ints(0, 1), ints(2), s_cut), run(1, 20, ints(0, 19), ints(0), s_cut), run(20, 51, ints(0, 31), ints(0), s_cut)]
+        assert torch.equal(torch.cat(parts), want) and torch.equal(s_cut, s_all)

@@ -57,8 +57,8 @@ environment_variables: dict[str, Callable[[], Any]] = {
     # Batch-invariant execution (the reference's VLLM_BATCH_INVARIANT, vllm_metax/v1/attention/backends/flash_attn.py:1063,
     # 1145): a request's tokens must not depend on what else is in its step.  Every reduction whose order follows the
     # batch is pinned: decode attention and MLA decode run unsplit, GEMMs take one fixed tile shape without split-K /
-    # stream-K / CTA pairs / operand swap, block-scaled fp8 products whole tiles, cascade attention and the fused
-    # tensor-parallel collectives are off.
+    # stream-K / CTA pairs / operand swap, block-scaled fp8 products whole tiles, the gated delta rule goes a token at a
+    # time, cascade attention and the fused tensor-parallel collectives are off.
     "B200_BATCH_INVARIANT": _flag("B200_BATCH_INVARIANT", "0"),
     # Gated delta rule (Qwen3-Next): prompt chunks of at least MIN_TOKENS tokens take the chunked matrix form
     # (ops/gdn.py:gated_delta_rule_chunked, PyTorch products) instead of the recurrent kernel.  0 = always recurrent.

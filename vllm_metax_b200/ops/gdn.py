@@ -142,12 +142,12 @@ def gated_delta_rule(q, k, v, g, beta, query_start_loc, state=None, state_indice
         state = torch.zeros(1, Hv, 128, 128, dtype=torch.float32, device=q.device)
         state_indices = None
     out = torch.empty_like(v)
-    ops._launches += 2 if q.shape[0] > query_start_loc.numel() - 1 else 1
+    ops._launches += 2 if q.shape[0] > query_start_loc.numel() - 1 and not ops.batch_invariant() else 1
     torch.ops.b200.gdn_recurrent(
         out, state, q, k, v, g.float().contiguous(), beta.float().contiguous(), query_start_loc.int().contiguous(),
         None if state_indices is None else state_indices.int().contiguous(),
         None if has_initial_state is None else has_initial_state.int().contiguous(),
-        q.shape[-1] ** -0.5 if scale is None else scale, l2norm)
+        q.shape[-1] ** -0.5 if scale is None else scale, l2norm, ops.batch_invariant())
     return out
 
 
@@ -167,12 +167,12 @@ def gated_delta_rule_ba(q, k, v, ba, a_log, dt_bias, query_start_loc, state=None
 
     ops.load_native()
     out = torch.empty(v.shape, dtype=v.dtype, device=v.device)
-    ops._launches += 2 if T > query_start_loc.numel() - 1 else 1
+    ops._launches += 2 if T > query_start_loc.numel() - 1 and not ops.batch_invariant() else 1
     torch.ops.b200.gdn_recurrent_ba(
         out, state, q, k, v, ba, a_log, dt_bias, query_start_loc.int().contiguous(),
         None if state_indices is None else state_indices.int().contiguous(),
         None if has_initial_state is None else has_initial_state.int().contiguous(),
-        q.shape[-1] ** -0.5 if scale is None else scale, l2norm)
+        q.shape[-1] ** -0.5 if scale is None else scale, l2norm, ops.batch_invariant())
     return out
 
 
