@@ -336,3 +336,28 @@ def test_gdn_rows_alone_and_in_company(dtype, monkeypatch):
         want = run(0, 51, ints(0, 1, 51), ints(2, 0), s_all)
         parts = [run(0, 1, ints(0, 1), ints(2), s_cut), run(1, 20, ints(0, 19), ints(0), s_cut), run(20, 51, ints(0, 31), ints(0), s_cut)]
         assert torch.equal(torch.cat(parts), want) and torch.equal(s_cut, s_all)
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("at", [0, 1, 6, 15, 16, 30])
+def test_gdn_tokens_in_front_of_a_bad_one(dtype, bad, at):
+    """An infinity or NaN in a token changes no bit of the outputs of those before it, of other columns (a bad value), of other
+    heads or of other sequences (a bad key or decay)."""
+    from vllm_metax_b200.ops.gdn import gated_delta_rule
+
+    q, k, v, g, beta, qsl, state, idx, has = (t.cuda() for t in _gdn_case(dtype, seed=5, lens=(31, 3, 17)))
+    run = lambda k_, v_, g_: gated_delta_rule(q, k_, v_, g_, beta, qsl, state.clone(), idx, has)
+    want = run(k, v, g)
+    assert bool(torch.isfinite(want).all())
+    v2, k2, g2 = v.clone(), k.clone(), g.clone()
+    v2[at, 1, 40] = bad
+    got = run(k, v2, g)
+    assert torch.equal(got[:at], want[:at]) and torch.equal(got[31:], want[31:]) and not bool(torch.isfinite(got[at, 1, 40]))
+    others = torch.arange(128, device="cuda") != 40
+    assert torch.equal(got[..., others], want[..., others]) and torch.equal(got[:, [0, 2, 3]], want[:, [0, 2, 3]])
+    k2[at, 1, 7] = bad
+    g2[at, 2] = bad
+    for got, same in ((run(k2, v, g), [0, 1]), (run(k, v, g2), [0, 1, 3])):
+        assert torch.equal(got[:at], want[:at]) and torch.equal(got[31:], want[31:]) and torch.equal(got[:, same], want[:, same])

@@ -662,15 +662,17 @@ gdn_chunk_kernel(const GdnParams p) {
     float R[kC], u[8], U[kC];
 #pragma unroll
     for (int t = 0; t < kC; ++t) R[t] = s_r[warp][t][col];
-    auto rows = [&](const float* m, const float (&x)[kC], int i) {     // row 2 i + half of a lower triangle times x
+    // Row 2 i + half of a lower triangle times x.  Entries behind the row's own token are left out: the triangle's zeros would make
+    // a NaN of an infinity or NaN there.
+    auto rows = [&](const float* m, const float (&x)[kC], int i) {
       float acc = 0.f;
 #pragma unroll
-      for (int j = 0; j < 2 * i + 2; j += 4) {
+      for (int j = 0; j <= 2 * i; j += 4) {
         const float4 a = *reinterpret_cast<const float4*>(m + (2 * i + half) * kC + j);
-        acc = fmaf(a.x, x[j], acc);
-        acc = fmaf(a.y, x[j + 1], acc);
-        acc = fmaf(a.z, x[j + 2], acc);
-        acc = fmaf(a.w, x[j + 3], acc);
+        const float f[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (j + e <= 2 * i + 1) acc = fmaf(f[e], j + e <= 2 * i || half ? x[j + e] : 0.f, acc);
       }
       return acc;
     };
