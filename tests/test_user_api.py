@@ -171,3 +171,32 @@ print("RESULT", json.dumps(alone == together))
     from vllm_metax_b200 import _custom_ops as ops
 
     assert not ops.batch_invariant() and ops.decode_num_splits(1, 1, 100000) > 1       # off by default
+
+
+@pytest.mark.gpu
+def test_norms_of_rows_alone_and_in_company():
+    """B200_BATCH_INVARIANT=1 (in a fresh interpreter): a row's norm has the same bits alone and among any number of others, at
+    widths of all the kernels."""
+    import subprocess
+    import sys
+
+    code = """
+import torch
+from vllm_metax_b200 import _custom_ops as ops
+g = torch.Generator().manual_seed(0)
+for hidden in (576, 1024, 1536, 2048, 3072, 4096, 5120, 7168, 8192):
+    x = torch.randn(300, hidden, generator=g).bfloat16().cuda()
+    r = torch.randn(300, hidden, generator=g).bfloat16().cuda()
+    w = torch.randn(hidden, generator=g).bfloat16().cuda()
+    want, a, b = ops.rms_norm(x, w, 1e-6), x.clone(), r.clone()
+    ops.fused_add_rms_norm(a, b, w, 1e-6)
+    for n in (1, 7, 31, 32, 64, 200, 256):
+        c, d = x[:n].clone(), r[:n].clone()
+        ops.fused_add_rms_norm(c, d, w, 1e-6)
+        assert torch.equal(ops.rms_norm(x[:n].clone(), w, 1e-6), want[:n]), (hidden, n)
+        assert torch.equal(c, a[:n]) and torch.equal(d, b[:n]), (hidden, n)
+print("RESULT true")
+"""
+    env = dict(os.environ, B200_BATCH_INVARIANT="1", PYTHONPATH=ROOT)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=ROOT, env=env, timeout=300)
+    assert r.returncode == 0 and "RESULT true" in r.stdout, (r.stdout[-500:], r.stderr[-1500:])

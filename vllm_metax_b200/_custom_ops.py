@@ -431,7 +431,7 @@ def batch_invariant() -> bool:
         _batch_invariant = bool(envs.B200_BATCH_INVARIANT)
         if _batch_invariant:
             for name in ("B200_GEMM_STREAMK", "B200_GEMM_SPLITK", "B200_GEMM_PAIR", "B200_FUSED_TP_COLLECTIVES",
-                         "B200_CASCADE_ATTENTION", "B200_CUSTOM_ALLREDUCE"):
+                         "B200_CASCADE_ATTENTION", "B200_CUSTOM_ALLREDUCE", "B200_NORM_BY_ROWS"):
                 os.environ[name] = "0"
     return _batch_invariant
 

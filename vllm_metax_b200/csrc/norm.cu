@@ -4,6 +4,8 @@
 // staged once in shared memory so global memory is read exactly once.
 // Parity: csrc/layernorm_kernels.cu:15,100,172 and layernorm_quant_kernels.cu:23-161,
 // quantization/fused_kernels/fused_layernorm_dynamic_per_token_quant.cu:49-95 of the reference.
+#include <cstdlib>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -217,9 +219,18 @@ __global__ void rms_norm_quant_kernel(uint8_t* __restrict__ out_q, float* __rest
   }
 }
 
+// B200_NORM_BY_ROWS=0: a row's sum runs in one order whatever the number of rows, in one kernel with one number of threads
+static bool one_order() {
+  static const bool on = [] {
+    const char* e = std::getenv("B200_NORM_BY_ROWS");
+    return e != nullptr && std::atoi(e) == 0;
+  }();
+  return on;
+}
+
 static int norm_threads(int hidden, int tokens) {
   int th = hidden / 8;
-  const int cap = tokens < 256 ? 1024 : 256;
+  const int cap = tokens < 256 || one_order() ? 1024 : 256;
   th = th < 32 ? 32 : th;
   th = th > cap ? cap : th;
   return (th + 31) / 32 * 32;
@@ -228,7 +239,7 @@ static int norm_threads(int hidden, int tokens) {
 template <typename T>
 static void rms_norm_t(void* out, void* x, void* residual, const void* weight, float eps, int tokens, int hidden,
                        int64_t x_stride, int64_t out_stride, int mode, cudaStream_t stream) {
-  const bool vec_ok = hidden % 1024 == 0 && x_stride % 8 == 0 && out_stride % 8 == 0 && tokens >= 32 &&
+  const bool vec_ok = hidden % 1024 == 0 && x_stride % 8 == 0 && out_stride % 8 == 0 && tokens >= 32 && !one_order() &&
                       ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(x) |
                         reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(weight)) & 15) == 0;
   const int vpt = hidden / 1024;

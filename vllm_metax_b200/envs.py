@@ -58,7 +58,7 @@ environment_variables: dict[str, Callable[[], Any]] = {
     # 1145): a request's tokens must not depend on what else is in its step.  Every reduction whose order follows the
     # batch is pinned: decode attention and MLA decode run unsplit, GEMMs take one fixed tile shape without split-K /
     # stream-K / CTA pairs / operand swap, block-scaled fp8 products whole tiles, the gated delta rule goes a token at a
-    # time, cascade attention and the fused tensor-parallel collectives are off.
+    # time, RMS norms take one kernel, cascade attention and the fused tensor-parallel collectives are off.
     "B200_BATCH_INVARIANT": _flag("B200_BATCH_INVARIANT", "0"),
     # Gated delta rule (Qwen3-Next): prompt chunks of at least MIN_TOKENS tokens take the chunked matrix form
     # (ops/gdn.py:gated_delta_rule_chunked, PyTorch products) instead of the recurrent kernel.  0 = always recurrent.
@@ -73,6 +73,8 @@ environment_variables: dict[str, Callable[[], Any]] = {
     "B200_PP_OVERLAP": _flag("B200_PP_OVERLAP", "1"),
     # Stream-K CTA-pair GEMM for skinny problems (read by the native GEMM dispatcher; 0 = tile / split-K kernels).
     "B200_GEMM_STREAMK": _flag("B200_GEMM_STREAMK", "1"),
+    # RMS norms choose their kernel by the number of rows (read by native code; 0 = one kernel, one order of sums).
+    "B200_NORM_BY_ROWS": _flag("B200_NORM_BY_ROWS", "1"),
     # One query tile per CTA in the prefill attention kernel (read by the native dispatcher; debug only).
     "B200_ATTN_PREFILL_SINGLE": _flag("B200_ATTN_PREFILL_SINGLE", "0"),
     # Sequence-parallel MoE through the NVLink dispatch / combine kernels instead of experts-on-all-tokens + all-reduce.
