@@ -328,3 +328,36 @@ def test_mla_rope_insert_and_keys(dtype, T, H, absorbed, pitch):
     up = torch.randn(T, H, 256, generator=g).to(dtype).cuda()
     assert torch.equal(ops.mla_expand_keys(up, p2, 128), torch.cat([up[..., :128], p2[:, None].expand(-1, H, -1)], -1))
     ops.check_kernel_status(0)
+
+
+def test_mla_layer_with_gradients_cpu():
+    """The layer in grad mode: outputs as without, and the gradient of the queries (a finite difference along one direction)."""
+    from vllm_metax_b200.attention.metadata import AttentionMetadata, ForwardContext, set_forward_context
+    from vllm_metax_b200.layers.mla import MLAAttention
+
+    g = torch.Generator().manual_seed(3)
+    at = MLAAttention(2, 0.1, 32, 64, 32, 512, 0, torch.float32)
+    at.set_kv_b(torch.randn(2 * 64, 512, generator=g) * 0.05)
+    q, kv_c, k_pe = (torch.randn(*s, generator=g) for s in ((3, 2, 96), (3, 512), (3, 64)))
+    cache = torch.randn(4, 16, 576, generator=g)
+    ints = lambda *x: torch.tensor(x, dtype=torch.int32)
+    md = AttentionMetadata(num_tokens=3, num_reqs=3, num_decodes=3, num_decode_tokens=3, query_start_loc=ints(0, 1, 2, 3),
+                           seq_lens=ints(5, 6, 7), block_table=ints(0, 1, 2)[:, None].contiguous(),
+                           slot_mapping=torch.tensor([4, 21, 38]), max_query_len=1, max_seq_len=16, block_size=16,
+                           prefill_query_start_loc=ints(0), max_prefill_query_len=0)
+
+    def run(x):
+        with set_forward_context(ForwardContext(md, [{"mla": cache.clone()}], torch.tensor([4, 5, 6]))):
+            return at(x, kv_c, k_pe)
+
+    with torch.no_grad():
+        want = run(q)
+    q.requires_grad_()
+    got = run(q)
+    assert got.requires_grad and torch.equal(got.detach(), want)
+    got.square().sum().backward()
+    d = torch.randn(q.shape, generator=g)
+    with torch.no_grad():
+        f = lambda e: float(run(q + e * d).double().square().sum())
+        # (central differences of steps h: relative errors of h^2 and of 2^-24 / h)
+        assert abs((f(1e-2) - f(-1e-2)) / 2e-2 - float((q.grad * d).sum())) < 1e-2 * float((q.grad.norm() * d.norm()))

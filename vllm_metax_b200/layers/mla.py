@@ -121,13 +121,12 @@ class MLAAttention(nn.Module):
             if qa is None:
                 qa = self._absorb_q(q[:mqa_end])
             else:                                       # beside the rotated part, which is there
-                torch.bmm(q[:mqa_end, :, : self.qk_nope].transpose(0, 1), self.W_UK,
-                          out=qa[..., : self.kv_lora].transpose(0, 1))
+                _bmm_into(qa[..., : self.kv_lora].transpose(0, 1), q[:mqa_end, :, : self.qk_nope].transpose(0, 1), self.W_UK)
             lat = ops.mla_decode(qa, cache, md.block_table[:n_req], md.seq_lens[:n_req], self.scale,
                                  query_start_loc=md.query_start_loc[:n_req + 1],
                                  topk_indices=None if topk_indices is None else topk_indices[:mqa_end],
                                  max_seq_len=md.max_seq_len)
-            torch.bmm(lat.transpose(0, 1), self.W_UV, out=out[:mqa_end].transpose(0, 1))
+            _bmm_into(out[:mqa_end].transpose(0, 1), lat.transpose(0, 1), self.W_UV)
         if pure_prefill and T > ndt:
             kv = kv_b_proj(kv_c[ndt:]).view(T - ndt, H, self.qk_nope + self.v_head)
             k = ops.mla_expand_keys(kv, k_pe[ndt:], self.qk_nope)
@@ -191,6 +190,14 @@ class MLAAttention(nn.Module):
         q_nope, q_pe = q[..., : self.qk_nope], q[..., self.qk_nope:]
         ql = torch.bmm(q_nope.transpose(0, 1), self.W_UK).transpose(0, 1)      # [T, H, 512]
         return torch.cat([ql, q_pe], dim=-1).contiguous()
+
+
+def _bmm_into(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor) -> None:
+    """``out = a @ w`` per head, written in place unless a gradient is asked for (which ``out=`` does not take)."""
+    if torch.is_grad_enabled() and (a.requires_grad or w.requires_grad or out.requires_grad):
+        out.copy_(torch.bmm(a, w))
+    else:
+        torch.bmm(a, w, out=out)
 
 
 def sparse_attn_indexer(q_fp8: torch.Tensor, weights: torch.Tensor, k: torch.Tensor, idx_cache: torch.Tensor,
