@@ -240,3 +240,48 @@ def test_qkv_norm_rope_insert_gpu(fp8_idx, kernel_status_ok):
                                       hq, hk, ws[0].cuda(), ws[1].cuda())
     assert none is None
     torch.testing.assert_close(q2.float().cpu(), q_ref, **tol)
+
+
+@pytest.mark.gpu
+def test_tensors_of_another_device_are_refused():
+    """Each tensor of a call in turn on the host, where a kernel must not follow its pointer: refused before any launch."""
+    from vllm_metax_b200 import _custom_ops as ops
+
+    ops.load_native()
+    dev = dict(device="cuda")
+    b16 = lambda *s: torch.zeros(*s, dtype=torch.bfloat16, **dev)
+    f32 = lambda *s: torch.zeros(*s, **dev)
+    i32 = lambda *x: torch.tensor(x, dtype=torch.int32, **dev)
+    i64 = lambda *x: torch.tensor(x, dtype=torch.int64, **dev)
+    e4m3 = lambda *s: torch.zeros(*s, **dev).to(torch.float8_e4m3fn)
+    n = torch.ops.b200
+    calls = [
+        (n.mla_rope_insert, [b16(2, 3, 192), b16(2, 3, 576), b16(2, 512), b16(2, 64), b16(1, 16, 576), b16(2, 576), b16(512), i64(0, 1),
+                             f32(4, 64), i64(0, 1), 1e-6]),
+        (n.mla_expand_keys, [b16(2, 3, 192), b16(2, 3, 256), b16(2, 64), 128]),
+        (n.gdn_recurrent, [b16(2, 2, 128), f32(2, 2, 128, 128), b16(2, 1, 128), b16(2, 1, 128), b16(2, 2, 128), f32(2, 2), f32(2, 2),
+                           i32(0, 1, 2), i32(0, 1), i32(1, 1), 1.0, True]),
+        (n.gdn_recurrent_ba, [b16(2, 2, 128), f32(2, 2, 128, 128), b16(2, 1, 128), b16(2, 1, 128), b16(2, 2, 128), b16(2, 4), f32(2), f32(2),
+                              i32(0, 1, 2), i32(0, 1), i32(1, 1), 1.0, True]),
+        (n.gated_head_norm, [b16(2, 256), b16(2, 256), b16(2, 2, 128), b16(128), 128, 1e-6]),
+        (n.sigmoid_dot_scale, [b16(2, 64), b16(2, 64), b16(64), b16(2, 64)]),
+        (n.moe_align, [i32(*[0] * 256), i32(0, 0), i32(0), i32(0, 0), i32(0, 1), i32(0, 1), 2, 128]),
+        (n.moe_scatter, [b16(128, 256), None, b16(2, 256), i32(0, 1), 1, f32(2, 1)]),
+        (n.moe_scatter, [e4m3(128, 256), f32(128, 2), b16(2, 256), i32(0, 1), 1, None]),
+        (n.moe_combine, [b16(2, 256), b16(128, 256), f32(2, 1), i32(0, 1), b16(2, 256), None, None, 0]),
+        (n.act_and_mul_quant, [e4m3(128, 256), f32(128, 2), None, b16(128, 512), 0, 0.0, 7.0, 128, False, i32(*[0] * 128), 128]),
+        (n.gemm_fp8_blockscale, [b16(128, 128), e4m3(128, 128), f32(128, 1), e4m3(1, 128, 128), f32(1, 1, 1), i32(0), i32(128),
+                                 i32(*[0] * 128), 128]),
+        (n.gemm_grouped, [b16(128, 128), b16(128, 128), b16(1, 128, 128), i32(0), i32(128), 0, None, i32(*[0] * 128), 128]),
+        (n.paged_attention_decode, [b16(1, 2, 128), b16(1, 2, 128), b16(1, 16, 2, 128), b16(1, 16, 2, 128), None, i32(0)[None], i32(1), None,
+                                    1.0, -1, 0.0, None, None, None, 1, 1, 1, 1.0, 1.0, True, None, None, None, 1.0, 0, None, True,
+                                    ops.decode_scratch(2, 2, 128, "cuda")]),
+    ]
+    for op, args in calls:
+        op(*args)                                           # (served as it is)
+        for i, a in enumerate(args):
+            if torch.is_tensor(a):
+                with pytest.raises(RuntimeError):
+                    op(*args[:i], a.cpu(), *args[i + 1:])
+    torch.cuda.synchronize()
+    ops.check_kernel_status(0)

@@ -94,6 +94,7 @@ void concat_and_cache_mla(const Tensor& kv_c, const Tensor& k_pe, Tensor& cache,
 // q [T, H, D] in place (its last 64 entries), kv [T, 576] with a row pitch; kv_c, k_pe, the cache rows and qa [n, H, 576] are written
 void mla_rope_insert(Tensor& q, Tensor& qa, Tensor& kv_c, Tensor& k_pe, Tensor& cache, const Tensor& kv, const Tensor& norm_w,
                      const Tensor& positions, const Tensor& cos_sin, const Tensor& slots, double eps) {
+  on_device_of(q, {&qa, &kv_c, &k_pe, &cache, &kv, &norm_w, &positions, &cos_sin, &slots});
   const int64_t T = q.size(0);
   TORCH_CHECK(q.dim() == 3 && q.is_contiguous() && q.size(2) % 8 == 0 && q.size(2) >= 64 && kv.dim() == 2 && kv.size(0) == T &&
               kv.size(1) == 576 && kv.stride(1) == 1 && kv.stride(0) % 8 == 0);
@@ -117,6 +118,7 @@ void mla_rope_insert(Tensor& q, Tensor& qa, Tensor& kv_c, Tensor& k_pe, Tensor& 
 }
 // out [T, H, nope + 64] = (kv [T, H, D][..., :nope] | k_pe [T, 64])
 void mla_expand_keys(Tensor& out, const Tensor& kv, const Tensor& k_pe, int64_t nope) {
+  on_device_of(kv, {&out, &k_pe});
   TORCH_CHECK(kv.dim() == 3 && kv.is_contiguous() && out.is_contiguous() && k_pe.is_contiguous() && out.dim() == 3);
   TORCH_CHECK(nope % 8 == 0 && kv.size(2) % 8 == 0 && nope <= kv.size(2) && out.size(0) == kv.size(0) && out.size(1) == kv.size(1) &&
               out.size(2) == nope + 64 && k_pe.numel() == kv.size(0) * 64);
@@ -152,6 +154,7 @@ void activation(Tensor& out, const Tensor& x, int64_t act, double p0) {
 void act_and_mul_quant(Tensor& out_q, const optional<Tensor>& scale_out, const optional<Tensor>& scale_in,
                        const Tensor& x, int64_t act, double p0, double p1, int64_t group, bool ue8m0,
                        const optional<Tensor>& sorted_ids, int64_t numel) {
+  on_device_of(x, {&out_q}, {&scale_out, &scale_in, &sorted_ids});
   TORCH_CHECK(x.is_contiguous() && out_q.is_contiguous());
   if (sorted_ids.has_value())
     TORCH_CHECK(sorted_ids->is_contiguous() && sorted_ids->scalar_type() == at::kInt &&
@@ -200,6 +203,7 @@ void merge_attn_states(Tensor& out, const optional<Tensor>& out_lse, const Tenso
 void gemm_fp8_blockscale(Tensor& out, const Tensor& a, const Tensor& a_scale, const Tensor& w, const Tensor& w_scale,
                          const optional<Tensor>& block_expert, const optional<Tensor>& total_padded,
                          const optional<Tensor>& sorted_ids, int64_t numel, bool cut) {
+  on_device_of(a, {&out, &a_scale, &w, &w_scale}, {&block_expert, &total_padded, &sorted_ids});
   const bool grouped = w.dim() == 3;
   TORCH_CHECK(a.dim() == 2 && a.stride(1) == 1 && w.is_contiguous() && a_scale.is_contiguous() && w_scale.is_contiguous());
   TORCH_CHECK(a.element_size() == 1 && w.element_size() == 1 && a.size(1) % 128 == 0 && a.stride(0) % 16 == 0);
@@ -703,6 +707,7 @@ void v4_gather_dequant(Tensor& dst, const Tensor& cache, const Tensor& slots, in
 void gdn_run(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& query_start_loc,
              const optional<Tensor>& state_idx, const optional<Tensor>& has_initial, double scale, bool l2norm, bool by_token,
              b200::GdnParams& p) {
+  on_device_of(q, {&out, &state, &k, &v, &query_start_loc}, {&state_idx, &has_initial});
   TORCH_CHECK(q.dim() == 3 && k.dim() == 3 && v.dim() == 3 && q.stride(2) == 1 && k.stride(2) == 1 && v.stride(2) == 1);
   TORCH_CHECK(q.stride(1) == q.size(2) && k.stride(1) == k.size(2) && v.stride(1) == v.size(2) && k.sizes() == q.sizes());
   const int64_t T = q.size(0), hq = q.size(1), hv = v.size(1);
@@ -744,6 +749,7 @@ void sigmoid_dot_scale(Tensor& out, const Tensor& x, const Tensor& w, const Tens
 void gdn_recurrent(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g,
                    const Tensor& beta, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
                    const optional<Tensor>& has_initial, double scale, bool l2norm, bool by_token) {
+  on_device_of(q, {&g, &beta});
   const int64_t n = v.numel() / (v.dim() == 3 && v.size(2) > 0 ? v.size(2) : 1);
   TORCH_CHECK(g.is_contiguous() && beta.is_contiguous() && g.scalar_type() == at::kFloat && beta.scalar_type() == at::kFloat &&
               g.numel() == n && beta.numel() == n);
@@ -755,6 +761,7 @@ void gdn_recurrent(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k,
 void gdn_recurrent_ba(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& ba,
                       const Tensor& a_log, const Tensor& dt_bias, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
                       const optional<Tensor>& has_initial, double scale, bool l2norm, bool by_token) {
+  on_device_of(q, {&ba, &a_log, &dt_bias});
   TORCH_CHECK(v.dim() == 3 && ba.dim() == 2 && ba.stride(1) == 1 && ba.size(0) == v.size(0) && ba.size(1) == 2 * v.size(1) &&
               ba.scalar_type() == v.scalar_type());
   TORCH_CHECK(a_log.is_contiguous() && dt_bias.is_contiguous() && a_log.scalar_type() == at::kFloat &&
@@ -766,6 +773,7 @@ void gdn_recurrent_ba(Tensor& out, Tensor& state, const Tensor& q, const Tensor&
 }
 // out [T, H * D] = norm(o) * silu(z), or o * sigmoid(z) without w; z [T, groups, at least rep * D]: head h in group h / rep
 void gated_head_norm(Tensor& out, const Tensor& o, const Tensor& z, const optional<Tensor>& w, int64_t dim, double eps) {
+  on_device_of(o, {&out, &z}, {&w});
   TORCH_CHECK(o.dim() == 2 && out.is_contiguous() && o.is_contiguous() && out.sizes() == o.sizes() && dim > 0 &&
               o.size(1) % dim == 0);
   TORCH_CHECK(z.dim() == 3 && z.stride(2) == 1 && z.size(0) == o.size(0) && z.size(1) * z.size(2) == o.size(1) &&

@@ -190,6 +190,7 @@ void grouped_topk(Tensor& weights, Tensor& ids, const Tensor& gating, const opti
 
 void moe_align(Tensor& sorted_ids, Tensor& block_expert, Tensor& total_padded, const optional<Tensor>& inv_pos,
                const Tensor& topk_ids, const optional<Tensor>& expert_map, int64_t experts, int64_t block) {
+  on_device_of(topk_ids, {&sorted_ids, &block_expert, &total_padded}, {&inv_pos, &expert_map});
   TORCH_CHECK(topk_ids.scalar_type() == at::kInt && topk_ids.is_contiguous());
   TORCH_CHECK(sorted_ids.numel() % block == 0 && block_expert.numel() >= sorted_ids.numel() / block);
   const c10::cuda::CUDAGuard guard(topk_ids.device());
@@ -203,6 +204,7 @@ void moe_align(Tensor& sorted_ids, Tensor& block_expert, Tensor& total_padded, c
 // out[inv_pos[t, k]] = x[t] (times weights[t, k]); with scales: as e4m3 with one per 128 entries.  Other rows of out stay as they are
 bool moe_scatter(Tensor& out, const optional<Tensor>& scales, const Tensor& x, const Tensor& inv_pos, int64_t topk,
                  const optional<Tensor>& weights) {
+  on_device_of(x, {&out, &inv_pos}, {&scales, &weights});
   TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && out.is_contiguous() && out.dim() == 2 && out.size(1) == x.size(1));
   TORCH_CHECK(inv_pos.is_contiguous() && inv_pos.scalar_type() == at::kInt && inv_pos.numel() == x.size(0) * topk);
   if (scales.has_value()) {
@@ -231,6 +233,7 @@ void moe_gather(Tensor& out, const Tensor& x, const Tensor& sorted_ids, const Te
 void moe_combine(Tensor& out, const Tensor& y, const Tensor& weights, const Tensor& inv_pos,
                  const optional<Tensor>& shared, const optional<Tensor>& expert_ids, const optional<Tensor>& through,
                  int64_t identity_from) {
+  on_device_of(y, {&out, &weights, &inv_pos}, {&shared, &expert_ids, &through});
   TORCH_CHECK(y.is_contiguous() && out.is_contiguous() && weights.scalar_type() == at::kFloat);
   if (through.has_value())
     TORCH_CHECK(through->is_contiguous() && through->sizes() == out.sizes() && through->scalar_type() == y.scalar_type() &&

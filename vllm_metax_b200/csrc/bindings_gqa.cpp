@@ -23,7 +23,7 @@ void paged_attention_decode(Tensor& out, const Tensor& q, const Tensor& k_cache,
                             const optional<Tensor>& sigmoid_shift, bool stream, const optional<Tensor>& scratch) {
   TORCH_CHECK(q.dim() == 3 && q.stride(2) == 1 && q.stride(1) == q.size(2), "q must be [T, Hq, D] with packed heads");
   on_device_of(q, {&out, &k_cache, &v_cache, &block_table, &seq_lens},
-               {&kv_scales, &query_start_loc, &sinks, &lse_out, &workspace, &alibi_slopes, &distance_bias, &gate, &sigmoid_shift});
+               {&kv_scales, &query_start_loc, &sinks, &lse_out, &workspace, &alibi_slopes, &distance_bias, &gate, &sigmoid_shift, &scratch});
   const PagedViews pv = paged_views(k_cache, v_cache);
   TORCH_CHECK(block_table.scalar_type() == at::kInt && seq_lens.scalar_type() == at::kInt);
   b200::DecodeParams p{};
