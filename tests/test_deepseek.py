@@ -330,24 +330,64 @@ def test_mla_rope_insert_and_keys(dtype, T, H, absorbed, pitch):
     ops.check_kernel_status(0)
 
 
-def test_mla_layer_with_gradients_cpu():
-    """The layer in grad mode: outputs as without, and the gradient of the queries (a finite difference along one direction)."""
-    from vllm_metax_b200.attention.metadata import AttentionMetadata, ForwardContext, set_forward_context
+def _mla_decode_layer(nope, dtype, device, g):
+    """A latent layer, its step of three decode rows, and what stands in front of the attention: queries, the latent product and
+    its norm, the rotation."""
+    from types import SimpleNamespace
+
+    from vllm_metax_b200.attention.metadata import AttentionMetadata, ForwardContext
+    from vllm_metax_b200.layers.basic import RMSNorm
     from vllm_metax_b200.layers.mla import MLAAttention
 
-    g = torch.Generator().manual_seed(3)
-    at = MLAAttention(2, 0.1, 32, 64, 32, 512, 0, torch.float32)
-    at.set_kv_b(torch.randn(2 * 64, 512, generator=g) * 0.05)
-    q, kv_c, k_pe = (torch.randn(*s, generator=g) for s in ((3, 2, 96), (3, 512), (3, 64)))
-    cache = torch.randn(4, 16, 576, generator=g)
-    ints = lambda *x: torch.tensor(x, dtype=torch.int32)
+    at = MLAAttention(2, 0.1, nope, 64, 32, 512, 0, dtype).to(device)
+    at.set_kv_b((torch.randn(2 * (nope + 32), 512, generator=g) * 0.05).to(device))
+    norm = RMSNorm(512, 1e-6, dtype).to(device)
+    put = lambda t: t.to(dtype).to(device)
+    q, kv, cache = (put(torch.randn(*s, generator=g)) for s in ((3, 2, nope + 64), (3, 576), (4, 16, 576)))
+    rope = SimpleNamespace(is_neox=False, cos_sin_cache=torch.randn(16, 64, generator=g).to(device))
+    ints = lambda *x: torch.tensor(x, dtype=torch.int32, device=device)
     md = AttentionMetadata(num_tokens=3, num_reqs=3, num_decodes=3, num_decode_tokens=3, query_start_loc=ints(0, 1, 2, 3),
                            seq_lens=ints(5, 6, 7), block_table=ints(0, 1, 2)[:, None].contiguous(),
-                           slot_mapping=torch.tensor([4, 21, 38]), max_query_len=1, max_seq_len=16, block_size=16,
+                           slot_mapping=torch.tensor([4, 21, 38], device=device), max_query_len=1, max_seq_len=16, block_size=16,
                            prefill_query_start_loc=ints(0), max_prefill_query_len=0)
+    pos = torch.tensor([4, 5, 6], device=device)
+    return at, norm, rope, q, kv, pos, ForwardContext(md, [{"mla": cache}], pos)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nope", [32, 12, 20])
+def test_mla_layer_of_any_query_width(nope):
+    """Query rows that do not start on 16 bytes take the separate operations in front of the attention, as they did; the results
+    of both ways agree with the layer on the CPU."""
+    from vllm_metax_b200.attention.metadata import set_forward_context
+
+    results = []
+    for device in ("cpu", "cuda"):
+        at, norm, rope, q, kv, pos, ctx = _mla_decode_layer(nope, torch.bfloat16, device, torch.Generator().manual_seed(nope))
+        with torch.no_grad(), set_forward_context(ctx):
+            done = at.rope_insert(pos, q, kv, norm, rope, False)
+            assert (done is not None) == (device == "cuda" and nope == 32)
+            if done is None:
+                kv_c, k_pe, q_pe = norm(kv[:, :512].contiguous()), kv[:, 512:].contiguous(), q[..., nope:].reshape(3, -1).contiguous()
+                ops.rotary_embedding(pos, q_pe, k_pe, 64, rope.cos_sin_cache, False)
+                q, qa = torch.cat([q[..., :nope], q_pe.view(3, 2, 64)], -1), None
+            else:
+                kv_c, k_pe, qa = done
+            results.append(at(q, kv_c, k_pe, None, None, qa).float().cpu())
+    # roundings to bf16 of queries, weights, latent sums and the result (2^-9 each) on values of size 1
+    torch.testing.assert_close(results[1], results[0], rtol=2.0 ** -5, atol=2.0 ** -5 * float(results[0].abs().max()))
+
+
+def test_mla_layer_with_gradients_cpu():
+    """The layer in grad mode: outputs as without, and the gradient of the queries (a finite difference along one direction)."""
+    from vllm_metax_b200.attention.metadata import ForwardContext, set_forward_context
+
+    g = torch.Generator().manual_seed(3)
+    at, _, _, q, kv, pos, ctx = _mla_decode_layer(32, torch.float32, "cpu", g)
+    kv_c, k_pe, cache = kv[:, :512].contiguous(), kv[:, 512:].contiguous(), ctx.kv_caches[0]["mla"]
 
     def run(x):
-        with set_forward_context(ForwardContext(md, [{"mla": cache.clone()}], torch.tensor([4, 5, 6]))):
+        with set_forward_context(ForwardContext(ctx.attn_metadata, [{"mla": cache.clone()}], pos)):
             return at(x, kv_c, k_pe)
 
     with torch.no_grad():

@@ -73,11 +73,14 @@ class MLAAttention(nn.Module):
     def rope_insert(self, positions, q, kv, norm, rope, sparse: bool):
         """Everything between the projections and the attention in one launch: ``q [T, H, nope+rope]`` rotated in place,
         ``kv [T, 576]`` (latent, shared key part) normed, rotated and written to the cache.  Returns ``(kv_c, k_pe, qa)`` for
-        ``forward``, or None where another path applies (other caches, context parallel steps, CPU)."""
+        ``forward``, or None where another path applies (other caches or alignments, context parallel steps, gradients, CPU)."""
         ctx = get_forward_context()
         md, cache = ctx.attn_metadata, ctx.kv_caches[self.layer_idx]["mla"]
+        rows = lambda x, pitch: x.stride(-1) == 1 and pitch % 8 == 0 and x.data_ptr() % 16 == 0          # (on 16 bytes)
         if not q.is_cuda or cache.dtype != q.dtype or q.dtype == torch.float32 or rope.is_neox \
-                or "pcp_slots_all" in md.extra or "dcp_ctx_lens" in md.extra or kv.stride(0) % 8 or kv.data_ptr() % 16:
+                or "pcp_slots_all" in md.extra or "dcp_ctx_lens" in md.extra or not rows(kv, kv.stride(0)) \
+                or not rows(q, q.shape[2]) or not q.is_contiguous() or not rows(cache, 8) or norm.weight.dtype != q.dtype \
+                or (torch.is_grad_enabled() and (q.requires_grad or kv.requires_grad)):
             return None
         T, H = q.shape[0], self.num_heads
         pure = md.extra.get("prefill_no_context", False) and not sparse
