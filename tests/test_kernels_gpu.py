@@ -675,3 +675,18 @@ def test_decode_of_wide_heads_in_large_groups(dtype, Hq, Hkv, dqk, dv):
             out.fill_(float("nan"))
             graph.replay()
             assert check()
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("N,K", [(8, 8), (1024, 1016), (1032, 1016), (4096, 4096), (4104, 4096), (4096, 4104), (8192, 1024),
+                                 (8192, 8192), (8200, 8192)])
+def test_few_tokens_around_the_choice_of_kernel(M, N, K):
+    """Sizes on either side of where the products of one to four tokens change kernels, and a contraction that ends inside a
+    warp's piece: sums of products exact in fp32, rounded once."""
+    g = torch.Generator(device=DEV).manual_seed(N + M)
+    a = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(N, K, generator=g, device=DEV) / K ** 0.5).bfloat16()
+    b, r = (torch.randn(*s, generator=g, device=DEV).bfloat16() for s in ((N,), (M, N)))
+    want = a.double() @ w.double().T
+    torch.testing.assert_close(ops.gemm(a, w).double(), want, rtol=2.0 ** -8, atol=1e-5)
+    torch.testing.assert_close(ops.gemm(a, w, bias=b, residual=r).double(), want + b.double() + r.double(), rtol=2.0 ** -8, atol=1e-5)

@@ -74,9 +74,14 @@ void gemm(Tensor& out, const Tensor& a, const Tensor& w, const optional<Tensor>&
                          dtype16(a), 0, cur_stream()) == 0)
       return;
   }
-  // up to four tokens: the weight as a stream over its rows.  The head of a model (whole tiles for every SM many times over)
-  // streams as fast on the tensor-core kernel.
-  if (force_bn == 0 && M <= 4 && epi <= 1) {
+  // Up to four tokens: the weight as a stream over its rows.  The multiply-adds of each token begin to count for two from some 60
+  // million entries on (4096 x 14336 31 / 29 us on the kernels below / here, 28672 x 4096 50 / 52), and for three and four, whose
+  // rows are on their way four at a time, much earlier and the more the shorter a row is (four tokens: 4096 x 4096 16.6 / 14.3,
+  // 1024 x 2048 11.5 / 5.6, but 8192 x 1024 14.6 / 17.3, 12288 x 2048 21 / 27, 28672 x 4096 50 / 75).  The head of a model
+  // (whole tiles for every SM many times over) streams as fast on the tensor-core kernel.
+  const int64_t entries = (int64_t)N * K;
+  const bool few = M == 1 || (M == 2 && entries <= (1 << 26)) || (M <= 4 && entries <= (1 << 24) && (N <= K || N <= 1024));
+  if (force_bn == 0 && few && epi <= 1) {
     static int sms_of[64] = {};
     int& sms = sms_of[a.get_device() & 63];
     if (sms == 0) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a.get_device());

@@ -5,10 +5,10 @@
 // A CTA owns an equal, contiguous share of the rows; its warps divide K among them, 16 bytes a lane, so that whatever N and K
 // are every SM streams the same number of bytes and a row's sum is finished inside one CTA: no partial tiles in memory, no second
 // pass, no ring or tensor memory to set up.  Eight rows (four, for three or four tokens) are on their way per warp at a time; the first rows come to L2 while the
-// kernel before still runs.  Bound by the weight's bytes; with more than four tokens the multiply-adds (one per token and entry,
-// on the CUDA cores) begin to, and the tensor-core kernels take over.
-// M = 1, bf16, N x K, stream-K on CTA pairs / here, us: 6144 x 4096 17.4 / 10.6, 28672 x 4096 (gated) 45 / 40, 4096 x 14336
-// 28.5 / 24, 4096 x 4096 14.5 / 16, of which half runs beside the kernel in front.
+// kernel before still runs.  Bound by the weight's bytes with one token; with more the multiply-adds (one per token and entry, on
+// the CUDA cores) begin to count, and the tensor-core kernels take over where bindings_core.cpp says.
+// M = 1, bf16, N x K, stream-K on CTA pairs / here behind a small kernel of a graph, us: 6144 x 4096 20 / 12, 28672 x 4096 (gated)
+// 50 / 39, 4096 x 14336 32 / 24, 4096 x 4096 16.5 / 9.3, 2048 x 2048 12 / 5.5; M = 4: 4096 x 4096 16.6 / 14.3.
 #include "common.cuh"
 #include "f32x2.cuh"
 #include "ops.h"
