@@ -228,6 +228,14 @@ def test_fp8_block_scaled_mm_shapes(M, N, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(400, 1536, 7168), (400, 2112, 7168), (129, 4096, 7168), (1, 128, 4864), (1, 128, 4736), (256, 24576, 256),
+                                   (1100, 4608, 128), (1100, 4352, 128)])
+def test_fp8_block_scaled_mm_around_the_choice_of_kernel(M, N, K):
+    """Sizes on either side of where K is cut among CTAs and of where tiles are wide, as above."""
+    test_fp8_block_scaled_mm_shapes(M, N, K)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("T,topk,E,N,K", [(5, 2, 4, 256, 256), (64, 8, 64, 512, 1024), (700, 3, 5, 2304, 512)])
 def test_fp8_grouped_mm_without_padding(T, topk, E, N, K):
     """Experts' rows at the start of their blocks: one, a few, all of a block; padding rows hold NaN and touch nothing."""

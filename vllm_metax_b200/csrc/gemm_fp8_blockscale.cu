@@ -12,7 +12,7 @@
 // Tile 128 x 256, or 128 x 128 where N has few tiles; TMA ring of 128-byte-swizzled [rows x 128 B] tiles.
 //
 // Dense tiles go down M first within groups of kGroupM row blocks, so that the CTAs of a wave share weights and A stays in L2.
-// With few tiles (decode rows, narrow products) the (tile, k block) space is cut into one contiguous range per CTA (stream-K):
+// Where whole tiles leave SMs idle for long the (tile, k block) space is cut into one contiguous range per CTA (stream-K):
 // a CTA whose range covers part of a tile leaves an fp32 partial in a slot of its own, and the one that arrives last at the tile
 // adds them in CTA order.  Nobody waits.  Where K is cut follows the number of rows: results that must not depend on the batch take
 // whole tiles, whose sums run through K in one order whatever the tile.
@@ -352,13 +352,17 @@ static void launch_f8(const void* A, int lda, const void* W, int E, const F8Para
   kern<<<grid, kF8Threads, F8Smem<BN>::kDyn, stream>>>(tmA, tmW, p);
 }
 
-// Stream-K pays where whole tiles would leave SMs idle for much of the time: below two tiles of 128 x 128 per SM, and with at
-// least 4 k blocks per CTA.  Returns the CTAs, or 0.
+// Ranges instead of whole tiles cost some 10 us: their counters' memset, the parts' way through memory, the last arriver's sums.
+// A k block of a tile takes 0.3 to 0.5 us, so they pay where they make a CTA's longest share at least kF8Saved blocks shorter (with
+// at least 4 blocks per CTA; and with two tiles per SM or more, tiles of twice the width are the better way).  us, whole tiles / ranges and the blocks saved: 1 x 7168 x 18432 60 / 41 (90), 64 x 2112 x 7168
+// 27.9 / 24.8 (50), 400 x 1536 x 7168 29.1 / 27.5 (38), 129 x 4096 x 7168 28.7 / 29.0 (32), 1000 x 2112 x 7168 32 / 41 (5),
+// 64 x 7168 x 2048 12.8 / 20.7 (10).  Returns the CTAs, or 0.
+constexpr int kF8Saved = 34;
 static int f8_streamk_ctas(int M, int N, int K, int sms) {
-  const int64_t tiles = (int64_t)ceil_div(M, kF8BM) * ceil_div(N, 128), units = tiles * ceil_div(K, kF8BK);
-  if (tiles >= 2 * sms || tiles == sms) return 0;
+  const int64_t tiles = (int64_t)ceil_div(M, kF8BM) * ceil_div(N, 128), num_k = ceil_div(K, kF8BK), units = tiles * num_k;
   const int64_t ctas = units / 4 < sms ? units / 4 : sms;
-  return ctas > tiles || tiles > sms ? (int)ctas : 0;
+  const int64_t longest = (tiles + sms - 1) / sms * num_k;
+  return ctas > 0 && tiles < 2 * sms && longest * ctas - units >= kF8Saved * ctas ? (int)ctas : 0;
 }
 
 void gemm_fp8_scratch(int M, int N, int K, int sms, int64_t* floats, int64_t* counters) {
@@ -373,9 +377,11 @@ static void run_f8(const void* A, int lda, const void* W, int E, const F8Params&
     launch_f8<T, 128, kF8StreamK>(A, lda, W, E, p, f8_streamk_ctas(p.M, p.N, p.K, sms), stream);
     return;
   }
-  // 128 x 256 halves what a block reads of A per product and its tensor-core time is shared-memory bound at 128 x 128; it
-  // needs enough tiles
-  const bool wide = p.N % 256 == 0 && (int64_t)ceil_div(p.M, kF8BM) * (p.N / 256) >= sms;
+  // 128 x 256 halves what a block reads of A per product, and its tensor-core time is shared-memory bound at 128 x 128: a tile
+  // takes 1.55 times as long as one of 128.  It needs enough tiles, and a last wave that does not give that back (two waves or
+  // three, 256 x 24576 x 1536: 30 us, 28 us in the narrow tiles; three or five, 1500 x 7168 x 16384: 245 us, 269 us)
+  const int64_t tw = (int64_t)ceil_div(p.M, kF8BM) * (p.N / 256), tn = (int64_t)ceil_div(p.M, kF8BM) * ceil_div(p.N, 128);
+  const bool wide = p.N % 256 == 0 && tw >= sms && (grouped || ceil_div(tw, sms) * 31 <= ceil_div(tn, sms) * 20);
   const int64_t tiles = (int64_t)ceil_div(p.M, kF8BM) * ceil_div(p.N, wide ? 256 : 128);
   const int grid = tiles < sms ? (int)tiles : sms;
   if (grouped) {
