@@ -690,3 +690,16 @@ def test_few_tokens_around_the_choice_of_kernel(M, N, K):
     want = a.double() @ w.double().T
     torch.testing.assert_close(ops.gemm(a, w).double(), want, rtol=2.0 ** -8, atol=1e-5)
     torch.testing.assert_close(ops.gemm(a, w, bias=b, residual=r).double(), want + b.double() + r.double(), rtol=2.0 ** -8, atol=1e-5)
+
+
+@pytest.mark.parametrize("M", [1, 32, 33, 64, 65])
+@pytest.mark.parametrize("N,K", [(8, 32), (512, 4096), (520, 4096), (64, 16384), (64, 16416), (64, 32768), (16, 65536)])
+def test_narrow_products_around_the_choice_of_kernel(M, N, K):
+    """Sizes on either side of where narrow products of a decode batch change kernels: one rounding behind fp32 sums."""
+    g = torch.Generator(device=DEV).manual_seed(N + M)
+    a = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(N, K, generator=g, device=DEV) / K ** 0.5).bfloat16()
+    b = torch.randn(N, generator=g, device=DEV).bfloat16()
+    want = a.double() @ w.double().T
+    torch.testing.assert_close(ops.gemm(a, w).double(), want, rtol=2.0 ** -8, atol=2e-5)
+    torch.testing.assert_close(ops.gemm(a, w, bias=b).double(), want + b.double(), rtol=2.0 ** -8, atol=2e-5)

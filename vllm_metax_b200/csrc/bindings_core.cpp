@@ -66,8 +66,10 @@ void gemm(Tensor& out, const Tensor& a, const Tensor& w, const optional<Tensor>&
   }
   // A router, or another narrow product of a decode batch: the stream-K kernel's fixed costs are most of its 13 us there
   // (64 x 128 x 2048: 8.9 us here).  From a few MB of weights on it streams them faster, and re-reading the tokens for every 8
-  // columns, as this kernel does, begins to count.
-  if (force_bn == 0 && M <= 64 && N <= 512 && (int64_t)N * K <= (1 << 21) && epi == 0 && !residual.has_value() && K % 32 == 0) {
+  // columns, as this kernel does, begins to count; so it does for more than 32 tokens against a few very long rows, which
+  // eight CTAs at most share (64 x 64 x 32768: 37.6 / 43 us; x 16384: faster here).
+  if (force_bn == 0 && M <= 64 && N <= 512 && (int64_t)N * K <= (1 << 21) && (M <= 32 || K <= 16384) && epi == 0 &&
+      !residual.has_value() && K % 32 == 0) {
     const auto wide = [](const void* at) { return (reinterpret_cast<uintptr_t>(at) & 15) == 0; };
     if (wide(a.data_ptr()) && wide(w.data_ptr()) &&
         b200::small_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), ptr(bias), M, N, K, a.stride(0), w.stride(0), out.stride(0),
