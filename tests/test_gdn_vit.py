@@ -361,3 +361,26 @@ def test_gdn_tokens_in_front_of_a_bad_one(dtype, bad, at):
     g2[at, 2] = bad
     for got, same in ((run(k2, v, g), [0, 1]), (run(k, v, g2), [0, 1, 3])):
         assert torch.equal(got[:at], want[:at]) and torch.equal(got[31:], want[31:]) and torch.equal(got[:, same], want[:, same])
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("lens", [(1,) * 90 + (40,), (7, 8, 5, 6) * 20, (3, 0, 5) * 30, (2,) * 4, (5, 6, 7, 8), (1, 1, 1, 26), (8,) * 80,
+                                  (0, 33) + (5,) * 80 + (17, 6)])
+@pytest.mark.parametrize("known", [False, True])
+def test_gdn_short_sequences_beside_long_ones(dtype, lens, known):
+    """Sequences of 5 to 8 tokens, around where they change from a token at a time to chunks or groups; few and many of them, alone
+    and beside longer ones, with the longest length known or not.  Outputs rounded once, fp32 state within 1e-5."""
+    from vllm_metax_b200.ops.gdn import gated_delta_rule
+
+    q, k, v, g, beta, qsl, _, _, _ = _gdn_case(dtype, seed=len(lens), lens=lens)
+    gen = torch.Generator().manual_seed(9)
+    state = torch.randn(len(lens) + 1, 4, 128, 128, generator=gen) * 0.1
+    idx = torch.randperm(len(lens) + 1, generator=gen)[:len(lens)].to(torch.int32)
+    has = (torch.rand(len(lens), generator=gen) < 0.7).to(torch.int32)
+    want, s_want = _gdn_f64(q, k, v, g, beta, lens, state, idx, has)
+    s_got = state.cuda()
+    got = gated_delta_rule(*(t.cuda() for t in (q, k, v, g, beta, qsl)), s_got, idx.cuda(), has.cuda(), max_len=max(lens) if known else 0)
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    torch.testing.assert_close(got.cpu().double(), want, rtol=eps, atol=1e-5)
+    torch.testing.assert_close(s_got.cpu().double(), s_want, rtol=1e-5, atol=1e-5)

@@ -704,9 +704,9 @@ void v4_gather_dequant(Tensor& dst, const Tensor& cache, const Tensor& slots, in
 }
 
 // q, k [T, Hq, 128], v [T, Hv, 128], g / beta f32 [T, Hv], state f32 [slots, Hv, 128, 128] (in / out)
-void gdn_run(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& query_start_loc,
+int64_t gdn_run(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& query_start_loc,
              const optional<Tensor>& state_idx, const optional<Tensor>& has_initial, double scale, bool l2norm, bool by_token,
-             b200::GdnParams& p) {
+             int64_t max_len, b200::GdnParams& p) {
   on_device_of(q, {&out, &state, &k, &v, &query_start_loc}, {&state_idx, &has_initial});
   TORCH_CHECK(q.dim() == 3 && k.dim() == 3 && v.dim() == 3 && q.stride(2) == 1 && k.stride(2) == 1 && v.stride(2) == 1);
   TORCH_CHECK(q.stride(1) == q.size(2) && k.stride(1) == k.size(2) && v.stride(1) == v.size(2) && k.sizes() == q.sizes());
@@ -727,7 +727,11 @@ void gdn_run(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const
   p.tokens = T; p.q_stride = q.stride(0); p.k_stride = k.stride(0); p.v_stride = v.stride(0);
   p.batch = (int)B; p.hq = (int)hq; p.hv = (int)hv; p.l2norm = l2norm; p.scale = (float)scale;
   Tensor scratch;
-  p.step = by_token || T <= B;                        // (a step of decode rows only, or one order of sums for all rows)
+  // A token at a time: one order of sums for all rows was asked for, or all sequences are short (as far as is known); beside longer
+  // ones, the short ones where they are so many that their chunks would not fit beside those of the long ones.
+  const int sms = device_sms(q), shorter = b200::gdn_short_len(B * hv, dtype16(q), sms);
+  p.step = by_token || T <= B || (max_len > 0 ? max_len <= shorter : T <= shorter * B);
+  p.short_len = B * hv >= 2 * sms ? shorter : 0;
   if (!p.step) {
     scratch = at::empty({b200::gdn_scratch_bytes(T, (int)B, (int)hq, (int)hv, dtype16(q))}, q.options().dtype(at::kByte));
     p.lengths = reinterpret_cast<const b200::GdnLengths*>(scratch.data_ptr());
@@ -735,6 +739,7 @@ void gdn_run(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const
   }
   const int rc = b200::gdn_recurrent(p, (int)q.size(2), (int)v.size(2), dtype16(q), cur_stream());
   TORCH_CHECK(rc == 0, "gdn_recurrent: head sizes must be 128 and value heads a multiple of q/k heads");
+  return p.step ? 1 : p.short_len > 0 ? 3 : 2;        // (launches)
 }
 void sigmoid_dot_scale(Tensor& out, const Tensor& x, const Tensor& w, const Tensor& y) {
   on_device_of(x, {&out, &w, &y}, {});
@@ -746,21 +751,21 @@ void sigmoid_dot_scale(Tensor& out, const Tensor& x, const Tensor& w, const Tens
                                          (int)y.size(1), x.stride(0), y.stride(0), dtype16(x), cur_stream());
   TORCH_CHECK(rc == 0, "sigmoid_dot_scale: rows must be 16-byte aligned");
 }
-void gdn_recurrent(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g,
-                   const Tensor& beta, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
-                   const optional<Tensor>& has_initial, double scale, bool l2norm, bool by_token) {
+int64_t gdn_recurrent(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g,
+                      const Tensor& beta, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
+                      const optional<Tensor>& has_initial, double scale, bool l2norm, bool by_token, int64_t max_len) {
   on_device_of(q, {&g, &beta});
   const int64_t n = v.numel() / (v.dim() == 3 && v.size(2) > 0 ? v.size(2) : 1);
   TORCH_CHECK(g.is_contiguous() && beta.is_contiguous() && g.scalar_type() == at::kFloat && beta.scalar_type() == at::kFloat &&
               g.numel() == n && beta.numel() == n);
   b200::GdnParams p{};
   p.g = g.data_ptr<float>(); p.beta = beta.data_ptr<float>();
-  gdn_run(out, state, q, k, v, query_start_loc, state_idx, has_initial, scale, l2norm, by_token, p);
+  return gdn_run(out, state, q, k, v, query_start_loc, state_idx, has_initial, scale, l2norm, by_token, max_len, p);
 }
 // the same with g = -exp(a_log) softplus(a + dt_bias) and beta = sigmoid(b) of ba [T, Hq, 2 Hv / Hq] = (b.., a..) per key head
-void gdn_recurrent_ba(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& ba,
+int64_t gdn_recurrent_ba(Tensor& out, Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& ba,
                       const Tensor& a_log, const Tensor& dt_bias, const Tensor& query_start_loc, const optional<Tensor>& state_idx,
-                      const optional<Tensor>& has_initial, double scale, bool l2norm, bool by_token) {
+                      const optional<Tensor>& has_initial, double scale, bool l2norm, bool by_token, int64_t max_len) {
   on_device_of(q, {&ba, &a_log, &dt_bias});
   TORCH_CHECK(v.dim() == 3 && ba.dim() == 2 && ba.stride(1) == 1 && ba.size(0) == v.size(0) && ba.size(1) == 2 * v.size(1) &&
               ba.scalar_type() == v.scalar_type());
@@ -769,7 +774,7 @@ void gdn_recurrent_ba(Tensor& out, Tensor& state, const Tensor& q, const Tensor&
   b200::GdnParams p{};
   p.ba = ba.data_ptr(); p.ba_stride = ba.stride(0);
   p.a_log = a_log.data_ptr<float>(); p.dt_bias = dt_bias.data_ptr<float>();
-  gdn_run(out, state, q, k, v, query_start_loc, state_idx, has_initial, scale, l2norm, by_token, p);
+  return gdn_run(out, state, q, k, v, query_start_loc, state_idx, has_initial, scale, l2norm, by_token, max_len, p);
 }
 // out [T, H * D] = norm(o) * silu(z), or o * sigmoid(z) without w; z [T, groups, at least rep * D]: head h in group h / rep
 void gated_head_norm(Tensor& out, const Tensor& o, const Tensor& z, const optional<Tensor>& w, int64_t dim, double eps) {
@@ -1038,10 +1043,10 @@ TORCH_LIBRARY_FRAGMENT(b200, m) {
   m.def("v4_gather_dequant(Tensor(a!) dst, Tensor cache, Tensor slots, int block_size) -> ()", &v4_gather_dequant);
   m.def("mla_rope_insert(Tensor(a!) q, Tensor(b!) qa, Tensor(c!) kv_c, Tensor(d!) k_pe, Tensor(e!) cache, Tensor kv, Tensor norm_w, Tensor positions, Tensor cos_sin, Tensor slots, float eps) -> ()", &mla_rope_insert);
   m.def("mla_expand_keys(Tensor(a!) out, Tensor kv, Tensor k_pe, int nope) -> ()", &mla_expand_keys);
-  m.def("gdn_recurrent_ba(Tensor(a!) out, Tensor(b!) state, Tensor q, Tensor k, Tensor v, Tensor ba, Tensor a_log, Tensor dt_bias, Tensor query_start_loc, Tensor? state_idx, Tensor? has_initial, float scale, bool l2norm, bool by_token=False) -> ()", &gdn_recurrent_ba);
+  m.def("gdn_recurrent_ba(Tensor(a!) out, Tensor(b!) state, Tensor q, Tensor k, Tensor v, Tensor ba, Tensor a_log, Tensor dt_bias, Tensor query_start_loc, Tensor? state_idx, Tensor? has_initial, float scale, bool l2norm, bool by_token=False, int max_len=0) -> int", &gdn_recurrent_ba);
   m.def("gated_head_norm(Tensor(a!) out, Tensor o, Tensor z, Tensor? w, int dim, float eps) -> ()", &gated_head_norm);
   m.def("sigmoid_dot_scale(Tensor(a!) out, Tensor x, Tensor w, Tensor y) -> ()", &sigmoid_dot_scale);
-  m.def("gdn_recurrent(Tensor(a!) out, Tensor(b!) state, Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, Tensor query_start_loc, Tensor? state_idx, Tensor? has_initial, float scale, bool l2norm, bool by_token=False) -> ()", &gdn_recurrent);
+  m.def("gdn_recurrent(Tensor(a!) out, Tensor(b!) state, Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, Tensor query_start_loc, Tensor? state_idx, Tensor? has_initial, float scale, bool l2norm, bool by_token=False, int max_len=0) -> int", &gdn_recurrent);
   m.def("tq_slot_bytes(int kbits, int vbits) -> int", &tq_slot_bytes);
   m.def("tq_store(Tensor(a!) cache, Tensor k, Tensor v, Tensor slot_mapping, int kbits, int vbits, bool nc) -> ()", &tq_store);
   m.def("tq_dequant(Tensor(a!) k_out, Tensor(b!) v_out, Tensor cache, Tensor slots, int kbits, int vbits, bool nc) -> ()", &tq_dequant);

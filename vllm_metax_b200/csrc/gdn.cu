@@ -5,8 +5,8 @@
 //   S  <- S + k_t u^T
 //   o_t = S^T (scale * q_t)
 //
-// bf16 prompts go by chunks of 16 tokens on the tensor cores (further down); decode steps a token at a time (gdn_step_kernel),
-// and so does everything where results must not depend on what else is in a step or on where a prompt is cut;
+// bf16 prompts go by chunks of 16 tokens on the tensor cores (further down); decode rows and other short sequences a token at a
+// time (gdn_step_kernel), and so does everything where results must not depend on what else is in a step or on where a prompt is cut;
 // fp16 prompts by groups of G = 4 on the fp32 units, as follows.  With S as it is before the group, G_t the sum of g over the group's
 // tokens up to t and D_tj = exp(G_t - G_j) (never above 1):
 //
@@ -144,7 +144,7 @@ gdn_kernel(const GdnParams p) {
   constexpr int KQ = NS * (kD / 8) / kThreads;
   const int b = blockIdx.z, h = blockIdx.y, hk = h / (p.hv / p.hq), col0 = blockIdx.x * kCols;
   const int64_t t0 = p.query_start_loc[b], t1 = p.query_start_loc[b + 1];
-  if (t1 <= t0) return;
+  if ((int)t1 - (int)t0 <= p.short_len) return;
   __shared__ __align__(16) float s_k[NB][NS][kD], s_q[NB][NS][kD];
   __shared__ __align__(16) T s_v[NB][NS][kCols], s_o[NB][NS][kCols];
   __shared__ __align__(16) float s_c[NB][NS][12];              // beta|k|^-1 e^G, beta, q e^G, update's factor; L x 3, e^G_last; M x 4
@@ -397,12 +397,17 @@ gdn_kernel(const GdnParams p) {
 constexpr int kC = 16;                     // tokens of a chunk
 constexpr int kChunkFloats = 2 * kC * kC + 5 * kC;   // T, M; factors a, beta, c, w; e^G of the last token
 
+__device__ __forceinline__ int gdn_chunks(const GdnParams& p, int b) {
+  const int n = p.query_start_loc[b + 1] - p.query_start_loc[b];
+  return n > p.short_len ? (n + kC - 1) / kC : 0;
+}
+
 // The chunk of index `at` in the order of the sequences: its sequence and first token, or false behind the last.  A whole warp.
-__device__ __forceinline__ bool gdn_locate(const int* qsl, int batch, int at, int lane, int& seq, int& first, int& end) {
+__device__ __forceinline__ bool gdn_locate(const GdnParams& p, int at, int lane, int& seq, int& first, int& end) {
   int before = 0;
-  for (int b0 = 0; b0 < batch; b0 += 32) {
+  for (int b0 = 0; b0 < p.batch; b0 += 32) {
     const int b = b0 + lane;
-    const int n = b < batch ? (qsl[b + 1] - qsl[b] + kC - 1) / kC : 0;
+    const int n = b < p.batch ? gdn_chunks(p, b) : 0;
     int inc = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -414,8 +419,8 @@ __device__ __forceinline__ bool gdn_locate(const int* qsl, int batch, int at, in
       const int src = __ffs(hit) - 1;
       const int start = before + __shfl_sync(0xffffffffu, inc - n, src);
       seq = b0 + src;
-      first = qsl[seq] + (at - start) * kC;
-      end = qsl[seq + 1];
+      first = p.query_start_loc[seq] + (at - start) * kC;
+      end = p.query_start_loc[seq + 1];
       return true;
     }
     before += __shfl_sync(0xffffffffu, inc, 31);
@@ -454,7 +459,7 @@ gdn_chunk_prepare_kernel(const GdnParams p) {
   __shared__ float s_kk[kC][kC], s_qk[kC][kC], s_ik[kC], s_iq[kC], s_l[4][kC][kC + 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, hk = blockIdx.y;
   int seq, first, end;
-  if (!gdn_locate(p.query_start_loc, p.batch, blockIdx.x, lane, seq, first, end)) return;
+  if (!gdn_locate(p, blockIdx.x, lane, seq, first, end)) return;
   const int n = min(kC, end - first);
   gdn_copy_rows<VEC>(s_k, reinterpret_cast<const T*>(p.k) + first * p.k_stride + hk * kD, p.k_stride, n, tid, 128);
   gdn_copy_rows<VEC>(s_q, reinterpret_cast<const T*>(p.q) + first * p.q_stride + hk * kD, p.q_stride, n, tid, 128);
@@ -583,9 +588,9 @@ gdn_chunk_kernel(const GdnParams p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tl = lane & 3;
   const int b = blockIdx.z, h = blockIdx.y, hk = h / (p.hv / p.hq), col0 = blockIdx.x * CV + warp * kWarpCols;
   const int t0 = p.query_start_loc[b], t1 = p.query_start_loc[b + 1];
-  if (t1 <= t0) return;
+  if (t1 <= t0 + p.short_len) return;
   int chunk = 0;                                    // index of the sequence's first chunk
-  for (int i = lane; i < b; i += 32) chunk += (p.query_start_loc[i + 1] - p.query_start_loc[i] + kC - 1) / kC;
+  for (int i = lane; i < b; i += 32) chunk += gdn_chunks(p, i);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) chunk += __shfl_xor_sync(0xffffffffu, chunk, o);
   const int slot = p.state_idx ? p.state_idx[b] : -1;
@@ -733,7 +738,7 @@ gdn_chunk_kernel(const GdnParams p) {
   }
 }
 
-// Decode rows: one CTA = one (sequence, value head), tokens one at a time.  A warp holds 16 rows of S, a lane 4 columns of them, so
+// Short sequences: one CTA = one (sequence, value head), tokens one at a time.  A warp holds 16 rows of S, a lane 4 columns of them, so
 // that a warp reads and writes whole rows of 512 bytes, all before the first product; the warps' sums meet in shared memory.
 template <typename T>
 __global__ void __launch_bounds__(256, 2)
@@ -742,7 +747,7 @@ gdn_step_kernel(const GdnParams p) {
   pdl_wait();
   const int b = blockIdx.x, h = blockIdx.y, hk = h / (p.hv / p.hq), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t t0 = p.query_start_loc[b], t1 = p.query_start_loc[b + 1];
-  if (t1 <= t0) return;
+  if (t1 <= t0 || (!p.step && t1 - t0 > p.short_len)) return;
   __shared__ __align__(16) float s_sum[2][2][8][kD];           // (two sets: a token is one barrier)
   const int slot = p.state_idx ? p.state_idx[b] : -1;
   const bool init = slot >= 0 && (p.has_initial == nullptr || p.has_initial[b] != 0);
@@ -817,10 +822,8 @@ void launch(const GdnParams& p, cudaStream_t stream) {
   auto wide = [](const void* at, int64_t stride) { return (reinterpret_cast<uintptr_t>(at) & 15) == 0 && stride % 8 == 0; };
   const bool vec = wide(p.q, p.q_stride) && wide(p.k, p.k_stride) && wide(p.v, p.v_stride);
   const dim3 grid(kD / kCols, p.hv, p.batch);
-  if (p.step) {
-    pdl_run(gdn_step_kernel<T>, dim3(p.batch, p.hv), 256, 0, stream, p);
-    return;
-  }
+  if (p.step || p.short_len > 0) pdl_run(gdn_step_kernel<T>, dim3(p.batch, p.hv), 256, 0, stream, p);
+  if (p.step) return;
   if constexpr (std::is_same<T, __nv_bfloat16>::value) {
     const dim3 chunks((unsigned)gdn_max_chunks(p.tokens, p.batch), p.hq), parts(kD / (kWarpCols * kChunkWarps), p.hv, p.batch);
     if (vec) {
@@ -903,6 +906,12 @@ int gated_head_norm(void* out, const void* o, const void* z, const void* w, int6
 int64_t gdn_scratch_bytes(int64_t tokens, int batch, int hq, int hv, int dtype) {
   return dtype == 0 ? gdn_max_chunks(tokens, batch) * hv * kChunkFloats * (int64_t)sizeof(float) : tokens * hq * (int64_t)sizeof(GdnLengths);
 }
+
+// Tokens up to which a sequence is faster a token at a time than in a chunk of 16 (or groups of four): a CTA's chain is a token's
+// 1.4 us there and some 13 us for a chunk, behind the launch in front.  us by tokens / by chunks, 64 sequences of 32 heads, bf16:
+// 2 tokens 66 / 101, 4 tokens 91 / 102, 5 tokens 103 / 103, 8 tokens 141 / 104; 4 sequences: 6 tokens 12.5 / 15.7, 8 tokens
+// 14.4 / 15.5; fp16, by tokens / by groups, 64 sequences: 6 tokens 115 / 143, 8 tokens 140 / 145.
+int gdn_short_len(int64_t sequences_by_heads, int dtype, int sms) { return dtype != 0 || sequences_by_heads <= sms ? 7 : 5; }
 
 // Returns 0, or 1 when the head sizes are not 128 / the head counts do not divide.
 int gdn_recurrent(const GdnParams& p, int dk, int dv, int dtype, cudaStream_t stream) {

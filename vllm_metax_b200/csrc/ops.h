@@ -372,12 +372,14 @@ struct GdnParams {
   const int *query_start_loc, *state_idx, *has_initial;
   const GdnLengths* lengths; // scratch of gdn_scratch_bytes(): fp16,
   const float* chunks;       //   bf16
-  int step;                  // a token at a time, no scratch
+  int step;                  // a token at a time for all sequences, no scratch
+  int short_len;             // else: a token at a time for sequences of up to this many tokens
   int64_t tokens, q_stride, k_stride, v_stride, ba_stride;
   int batch, hq, hv, l2norm;
   float scale;
 };
 int64_t gdn_scratch_bytes(int64_t tokens, int batch, int hq, int hv, int dtype);
+int gdn_short_len(int64_t sequences_by_heads, int dtype, int sms);
 int gdn_recurrent(const GdnParams& p, int dk, int dv, int dtype, cudaStream_t stream);
 // out[t, h] = (unit_rms(o[t, h]) * w) * silu(z[t, h / rep, h % rep]), or o * sigmoid(z) without w; 0, 1: head size, 2: alignment
 int gated_head_norm(void* out, const void* o, const void* z, const void* w, int64_t tokens, int heads, int dim, int rep,

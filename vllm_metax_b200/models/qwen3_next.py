@@ -113,7 +113,7 @@ class GatedDeltaNet(nn.Module):
                                   heads=(self.nk_l, self.dk, self.rep * self.dv))
         q, k, v = mixed.split([self.key_l, self.key_l, self.val_l], -1)
         o = gdn.gated_delta_rule_ba(q.view(T, self.nk_l, self.dk), k.view(T, self.nk_l, self.dk), v.view(T, self.nv_l, self.dv),
-                                    ba, self.A_log, self.dt_bias, qsl, self.ssm_state, idx, init)
+                                    ba, self.A_log, self.dt_bias, qsl, self.ssm_state, idx, init, max_len=md.max_query_len)
         z = qkvz.view(T, self.nk_l, -1)[..., 2 * self.dk + self.rep * self.dv:]
         o = gdn.gated_head_norm(o.reshape(T, self.val_l), z, self.norm.weight, self.dv, self.norm.eps)
         return self.out_proj(o)

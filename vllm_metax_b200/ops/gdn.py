@@ -121,8 +121,9 @@ def gated_delta_rule_chunked(q, k, v, g, beta, query_start_loc, state=None, stat
 
 
 def gated_delta_rule(q, k, v, g, beta, query_start_loc, state=None, state_indices=None, has_initial_state=None,
-                     scale: Optional[float] = None, l2norm: bool = True):
-    """Output ``[T, Hv, 128]``; ``state`` is updated in place.  ``B200_GDN_CHUNKED=1`` sends batches that contain a
+                     scale: Optional[float] = None, l2norm: bool = True, max_len: int = 0):
+    """Output ``[T, Hv, 128]``; ``state`` is updated in place.  ``max_len``: tokens of the longest sequence, where the host
+    knows it (chooses kernels only).  ``B200_GDN_CHUNKED=1`` sends batches that contain a
     prompt chunk of ``B200_GDN_CHUNKED_MIN_TOKENS`` tokens or more through the chunked form instead of the recurrent
     kernel."""
     from .. import envs
@@ -142,17 +143,16 @@ def gated_delta_rule(q, k, v, g, beta, query_start_loc, state=None, state_indice
         state = torch.zeros(1, Hv, 128, 128, dtype=torch.float32, device=q.device)
         state_indices = None
     out = torch.empty_like(v)
-    ops._launches += 2 if q.shape[0] > query_start_loc.numel() - 1 and not ops.batch_invariant() else 1
-    torch.ops.b200.gdn_recurrent(
+    ops._launches += torch.ops.b200.gdn_recurrent(
         out, state, q, k, v, g.float().contiguous(), beta.float().contiguous(), query_start_loc.int().contiguous(),
         None if state_indices is None else state_indices.int().contiguous(),
         None if has_initial_state is None else has_initial_state.int().contiguous(),
-        q.shape[-1] ** -0.5 if scale is None else scale, l2norm, ops.batch_invariant())
+        q.shape[-1] ** -0.5 if scale is None else scale, l2norm, ops.batch_invariant(), max_len)
     return out
 
 
 def gated_delta_rule_ba(q, k, v, ba, a_log, dt_bias, query_start_loc, state=None, state_indices=None, has_initial_state=None,
-                        scale: Optional[float] = None, l2norm: bool = True):
+                        scale: Optional[float] = None, l2norm: bool = True, max_len: int = 0):
     """:func:`gated_delta_rule` with ``g = -exp(a_log) softplus(a + dt_bias)`` and ``beta = sigmoid(b)`` of the projection
     ``ba [T, Hq * 2 rep]``, which holds per key head ``rep = Hv / Hq`` numbers b and as many a; formed in the kernel."""
     from .. import envs
@@ -162,17 +162,16 @@ def gated_delta_rule_ba(q, k, v, ba, a_log, dt_bias, query_start_loc, state=None
         b, a = ba.reshape(T, Hq, 2 * (Hv // Hq)).chunk(2, -1)
         beta = torch.sigmoid(b.reshape(T, Hv).float())
         g = -torch.exp(a_log) * torch.nn.functional.softplus(a.reshape(T, Hv).float() + dt_bias)
-        return gated_delta_rule(q, k, v, g, beta, query_start_loc, state, state_indices, has_initial_state, scale, l2norm)
+        return gated_delta_rule(q, k, v, g, beta, query_start_loc, state, state_indices, has_initial_state, scale, l2norm, max_len)
     from .. import _custom_ops as ops
 
     ops.load_native()
     out = torch.empty(v.shape, dtype=v.dtype, device=v.device)
-    ops._launches += 2 if T > query_start_loc.numel() - 1 and not ops.batch_invariant() else 1
-    torch.ops.b200.gdn_recurrent_ba(
+    ops._launches += torch.ops.b200.gdn_recurrent_ba(
         out, state, q, k, v, ba, a_log, dt_bias, query_start_loc.int().contiguous(),
         None if state_indices is None else state_indices.int().contiguous(),
         None if has_initial_state is None else has_initial_state.int().contiguous(),
-        q.shape[-1] ** -0.5 if scale is None else scale, l2norm, ops.batch_invariant())
+        q.shape[-1] ** -0.5 if scale is None else scale, l2norm, ops.batch_invariant(), max_len)
     return out
 
 
