@@ -285,3 +285,16 @@ def test_tensors_of_another_device_are_refused():
                     op(*args[:i], a.cpu(), *args[i + 1:])
     torch.cuda.synchronize()
     ops.check_kernel_status(0)
+
+
+def test_choice_of_tiles_for_256_wide_heads():
+    """The rule at sizes that were timed on both kernels: (tokens, sequences, longest portion, heads, key heads, longest length)
+    and whether the 128-row tiles were the faster ones."""
+    for args, faster in [((2, 1, 2, 16, 2, 2), True), ((100, 1, 100, 16, 2, 100), True), ((4, 1, 4, 16, 2, 8196), False),
+                         ((64, 1, 64, 16, 2, 8256), False), ((16, 1, 16, 8, 1, 30016), False), ((4096, 8, 512, 16, 2, 512), True),
+                         ((1000, 1, 1000, 16, 2, 5000), True), ((210, 30, 7, 16, 2, 507), True), ((128, 64, 2, 16, 2, 1002), False),
+                         ((210, 30, 7, 8, 1, 507), False), ((1000, 1, 1000, 8, 1, 5000), True), ((1000, 1, 1000, 4, 1, 5000), False),
+                         ((210, 30, 7, 16, 16, 507), False), ((128, 64, 2, 16, 16, 1002), False), ((4096, 8, 512, 16, 16, 512), True),
+                         ((1000, 1, 1000, 16, 16, 5000), True), ((3949, 4, 2048, 16, 2, 2048), True), ((3949, 4, 2048, 16, 2, 0), True),
+                         ((64, 1, 64, 16, 2, 0), False)]:
+        assert ops.prefill_tiles_of_128_pay(*args) == faster, args

@@ -530,6 +530,19 @@ def distance_bias_tiles(bias, group: int):
     return (bias[:, d] * 1.4426950408889634).view(H // gp, gp, L + 254).transpose(1, 2).contiguous()
 
 
+def prefill_tiles_of_128_pay(tokens: int, batch: int, max_q_len: int, q_heads: int, kv_heads: int, max_seq_len: int, sms: int = 148) -> bool:
+    """256-wide heads: whether the one-tile tcgen05 kernel (128 rows a CTA) is faster than 16-row tiles of the decode kernel.  Both
+    keep one CTA per SM, and a CTA's time is its chain over the keys, 69 ns each there and 33 ns here: with few rows, as in a short
+    portion of a prompt behind a long context, both kernels are one wave and the small tiles win.  us, 16-row tiles / tcgen05: 64
+    tokens behind 8192, 16 heads over 2 287 / 583; 64 x 2 behind 1000 56 / 94; 1000 behind 4000, 4 over 1 340 / 360, 8 over 1 653 /
+    361; 8 x 512, 16 over 2 676 / 124.  Up to some 110 keys the tcgen05 kernel wins all the same (launch and prologue 14 us, 18 us)."""
+    g = q_heads // kv_heads
+    gp = g if 128 % g == 0 else 1
+    tiles = lambda rows, per, heads: heads * min(batch * -(-max_q_len * rows // per), max(batch, -(-tokens * rows // per) + batch // 2))
+    small, large = (-(-n // sms) for n in (tiles(g, 16, kv_heads), tiles(gp, 128, q_heads // gp)))
+    return (2.1 * large - small) * (max_seq_len or 1 << 30) <= 120
+
+
 def paged_attention_prefill(q, kv_cache, block_table, seq_lens, query_start_loc, scale, *, out=None, kv_scales=None,
                             max_q_len: int = 0, window: int = -1, softcap: float = 0.0, sinks=None, lse_out=None,
                             k_scale=1.0, v_scale=1.0, causal=True, max_seq_len: int = 0, alibi_slopes=None,
@@ -545,7 +558,9 @@ def paged_attention_prefill(q, kv_cache, block_table, seq_lens, query_start_loc,
         # weights rounded to 16 bits: callers that ask for it keep the other)
         plain256 = lse_out is None and k.shape[-1] == v.shape[-1] == 256 and distance_bias is None and gate is None and out_scale == 1.0 \
             and chunk == 0 and sigmoid_shift is None and out.is_contiguous() and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 \
-            and (128 % k.shape[1] == 0 or k.shape[1] % 128 == 0) and k.shape[1] % 16 == 0
+            and (128 % k.shape[1] == 0 or k.shape[1] % 128 == 0) and k.shape[1] % 16 == 0 \
+            and prefill_tiles_of_128_pay(q.shape[0], B, max_q_len or q.shape[0], q.shape[1], k.shape[2],
+                                         min(max_seq_len or 1 << 30, window + 128) if window > 0 else max_seq_len)
         if k.dtype == q.dtype and q.dtype != torch.float32 and kv_scales is None \
                 and (k.shape[-1] <= 192 and v.shape[-1] <= 128 or plain256):
             if distance_bias is not None and bias_tiles is None:
