@@ -401,3 +401,37 @@ def test_mla_layer_with_gradients_cpu():
         f = lambda e: float(run(q + e * d).double().square().sum())
         # (central differences of steps h: relative errors of h^2 and of 2^-24 / h)
         assert abs((f(1e-2) - f(-1e-2)) / 2e-2 - float((q.grad * d).sum())) < 1e-2 * float((q.grad.norm() * d.norm()))
+
+
+def test_choice_of_the_latent_attention_kernel():
+    """The rule at sizes that were timed on both kernels, from 128 to 32768 rows each: (tokens, heads) where the tcgen05 kernel was
+    the faster one at most lengths, and lengths that are short anyway."""
+    for tokens, heads, pays in [(1, 128, False), (4, 128, False), (8, 128, False), (16, 128, True), (64, 128, True), (256, 128, True),
+                                (1024, 128, True), (8, 96, False), (16, 96, True), (16, 64, False), (32, 64, True), (128, 64, True),
+                                (256, 64, False), (64, 32, False), (64, 16, False)]:
+        assert ops.mla_tcgen05_pays(tokens, heads) == pays and ops.mla_tcgen05_pays(tokens, heads, 4096) == pays
+        assert not ops.mla_tcgen05_pays(tokens, heads, 128)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H", [64, 128, 200])
+@pytest.mark.parametrize("lens", [[128] * 128, [1, 128, 64, 3, 97] * 50, [129] * 80, [32] * 300, [4000] + [5] * 90, [100] * 5])
+def test_mla_tcgen05_ranges(H, lens):
+    """Tokens too short to be cut, in ranges that end where tokens do, around the length where cutting begins, and empty ranges;
+    against the CPU's statement in fp32."""
+    g = torch.Generator().manual_seed(H + len(lens))
+    bs = 32
+    nb = [-(-n // bs) for n in lens]
+    table, perm, at = torch.zeros(len(lens), max(nb), dtype=torch.int32), torch.randperm(sum(nb), generator=g), 0
+    for i, n in enumerate(nb):
+        table[i, :n] = perm[at: at + n]
+        at += n
+    q, cache = torch.randn(len(lens), H, 576, generator=g).bfloat16(), torch.randn(sum(nb), bs, 576, generator=g).bfloat16()
+    sl, lse = torch.tensor(lens, dtype=torch.int32), torch.empty(H, len(lens), device="cuda")
+    got = [ops.mla_decode(q.cuda(), cache.cuda(), table.cuda(), sl.cuda(), 0.05, impl=2, lse_out=lse).float().cpu() for _ in range(2)]
+    want, want_lse = ref.mla_decode(q.float(), cache.float(), table, sl, 0.05)
+    assert torch.equal(got[0], got[1])
+    # weights rounded to bf16 (2^-9 each) against rows of size 1, the result once more
+    torch.testing.assert_close(got[0], want, rtol=2.0 ** -7, atol=2.0 ** -8)
+    torch.testing.assert_close(lse.cpu(), want_lse, rtol=1e-4, atol=2e-3)
+    ops.check_kernel_status(0)

@@ -1058,20 +1058,31 @@ def mla_decode_num_splits(tokens: int, heads: int, kv: int, window: int = 0, fp8
     return 1 if ctas >= 148 else max(1, min((296 + ctas - 1) // ctas, kv // 256, 16))
 
 
+def mla_tcgen05_pays(tokens: int, heads: int, max_seq_len: int = 0) -> bool:
+    """Whether the tcgen05 kernel is the faster one for dense 16-bit latent attention, whatever the lengths are.  It wants 128 heads
+    for its rows and enough tokens for its CTAs, which take a tile of 32 after the other.  us, mma.sync with splits / tcgen05, 512
+    and 8192 cached rows each: 128 heads, 4 tokens 26 / 37, 78 / 84; 8 tokens 30 / 37, 148 / 90; 16 tokens 53 / 39, 307 / 135; 64
+    heads, 16 tokens 31 / 37, 155 / 133; 32 tokens 54 / 37, 308 / 215; 128 tokens of 512 146 / 82, 256 tokens of 128 43 / 65, of 512
+    129 / 138, of 2048 440 / 401.  Up to 128 rows each it gains too little to matter."""
+    if heads < 64 or 0 < max_seq_len <= 128:
+        return False
+    return tokens >= 16 if heads >= 96 else 32 <= tokens < 256
+
+
 def mla_decode(q, mla_cache, block_table, seq_lens, scale, *, query_start_loc=None, topk_indices=None, out=None,
                lse_out=None, num_splits: int = 0, max_seq_len: int = 0, impl: int = 0, window: int = 0,
                kv_rank: int = 512, workspace=None):
     """Absorbed MLA over the latent cache (dense, or sparse with ``topk_indices [T, topk]``).
     ``q [T, H, 576]`` -> ``[T, H, 512]``.  ``impl``: 0 = choose, 1 = mma.sync kernel, 2 = tcgen05 kernel (dense 16-bit
     caches; csrc/mla_decode_tcgen05.cu, which divides the work itself whatever ``num_splits``) or fail.  "Choose" takes the tcgen05
-    kernel for 64 heads per rank or more, unless results must not depend on the batch or ``B200_MLA_TCGEN05=0``.  Other sizes: cache rows ``[kv_rank latent | rotated part | padding]``, queries of the same
+    kernel where ``mla_tcgen05_pays``, unless results must not depend on the batch or ``B200_MLA_TCGEN05=0``.  Other sizes: cache rows ``[kv_rank latent | rotated part | padding]``, queries of the same
     row length, output ``[T, H, kv_rank]``.  ``window`` > 0: only the last ``window`` visible positions.  ``workspace``: for
     the partial results of splits, where the caller owns it (fp32)."""
     if _use_cuda(q):
         T, H, _ = q.shape
         if q.dtype == torch.float32 or kv_rank > 512:      # CUDA-core kernel: one pass
             num_splits = 1
-        if impl == 0 and (not envs.B200_MLA_TCGEN05 or batch_invariant()):
+        if impl == 0 and (not envs.B200_MLA_TCGEN05 or batch_invariant() or not mla_tcgen05_pays(T, H, max_seq_len)):
             impl = 1
         out = torch.empty(T, H, kv_rank, dtype=q.dtype, device=q.device) if out is None else out
         if num_splits <= 0 and batch_invariant():

@@ -57,6 +57,7 @@ constexpr int kTcQBytes = (kTcKC - kTcQT) * kTcQChunk;   // 49152
 constexpr int kTcTileBytes = kTcKC * kTcKChunk;  // 36864
 constexpr int kTcStages = 4;
 constexpr int kTcMaxTokens = 1024;
+constexpr int kTcShort = 4;                      // tiles of tokens that are not cut
 constexpr int kTcSlot = kTcHalf * kTcBM + 2 * kTcBM;     // floats of a part: [64][128] float4, 128 maxima, 128 denominators
 constexpr float kTcLazy = 8.f;                   // log2 of the growth of a row maximum that forces a rescale
 
@@ -107,7 +108,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint64_t* met = o_done + 2;          // the softmax warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::kNumBars);
   int* s_pre = reinterpret_cast<int*>(smem + L::kPrefix);
-  __shared__ int s_sum[6], s_done[2];
+  __shared__ int s_sum[6], s_max[6], s_done[2];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int hf = blockIdx.x;                                  // latent half of the output
@@ -159,21 +160,26 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   // ---- tiles in front of every token (a token that sees nothing has one, all masked)
   {
     const int per = (T_ + 191) / 192;
-    int sum = 0, seq;
+    int sum = 0, seq, most = 0;
     for (int i = 0; i < per; ++i) {
       const int t = (int)threadIdx.x * per + i;
       if (t >= T_) break;
       const int n = max(1, (visible(t, seq) + kTcBN - 1) / kTcBN);
       s_pre[t + 1] = n;
       sum += n;
+      most = max(most, n);
     }
     int inc = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int v = __shfl_up_sync(0xffffffffu, inc, o);
       if (lane >= o) inc += v;
+      most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
     }
-    if (lane == 31) s_sum[warp] = inc;
+    if (lane == 31) {
+      s_sum[warp] = inc;
+      s_max[warp] = most;
+    }
     __syncthreads();
     int before = inc - sum;
     for (int w = 0; w < warp; ++w) before += s_sum[w];
@@ -195,12 +201,24 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int groups = (int)min(min((long long)gridDim.z, units),
                               (long long)T_ * max(1, (int)sqrtf(0.5f * (float)units / (float)T_)));
   const int grp = blockIdx.z;
-  const int u0 = grp < groups ? (int)(units * grp / groups) : 0, u1 = grp < groups ? (int)(units * (grp + 1) / groups) : 0;
-  int tok0 = 0;
-  for (int hi = T_ - 1; tok0 < hi;) {                         // the last token that starts at or before u0
-    const int mid = (tok0 + hi + 1) >> 1;
-    if (s_pre[mid] <= u0) tok0 = mid; else hi = mid - 1;
-  }
+  auto find = [&](int at) -> int {                            // the last token that starts at or before tile `at`
+    int t = 0;
+    for (int hi = T_ - 1; t < hi;) {
+      const int mid = (t + hi + 1) >> 1;
+      if (s_pre[mid] <= at) t = mid; else hi = mid - 1;
+    }
+    return t;
+  };
+  // ends of ranges; where all tokens are short, the nearer end of the token there: adding up parts would cost more than it saves
+  const int longest = max(max(max(s_max[0], s_max[1]), max(s_max[2], s_max[3])), max(s_max[4], s_max[5]));
+  auto border = [&](int c) -> int {
+    const int at = (int)(units * c / groups);
+    if (longest > kTcShort || c >= groups) return at;
+    const int t = find(at);
+    return at - s_pre[t] <= s_pre[t + 1] - at ? s_pre[t] : s_pre[t + 1];
+  };
+  const int u0 = grp < groups ? border(grp) : 0, u1 = grp < groups ? border(grp + 1) : 0;
+  const int tok0 = find(u0);
 
   if (warp == 4) {
     // ------------------------------------------------------------ TMA producer

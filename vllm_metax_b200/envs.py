@@ -64,7 +64,8 @@ environment_variables: dict[str, Callable[[], Any]] = {
     # (ops/gdn.py:gated_delta_rule_chunked, PyTorch products) instead of the recurrent kernel.  0 = always recurrent.
     "B200_GDN_CHUNKED": _flag("B200_GDN_CHUNKED", "0"),
     "B200_GDN_CHUNKED_MIN_TOKENS": _int("B200_GDN_CHUNKED_MIN_TOKENS", 256),
-    # Absorbed-MLA decode on tcgen05 (csrc/mla_decode_tcgen05.cu) for dense 16-bit caches from 64 heads per rank up;
+    # Absorbed-MLA decode on tcgen05 (csrc/mla_decode_tcgen05.cu) for dense 16-bit caches where it pays: 16 query tokens and
+    # more of 96 heads per rank and more, 32 to 255 of 64 heads;
     # 0 = the mma.sync kernel unless a call asks for the tcgen05 one.
     "B200_MLA_TCGEN05": _flag("B200_MLA_TCGEN05", "1"),
     # Prepare step k + 1 on the host (schedule, staging buffers) while the device runs step k; 0 = strictly in turn.
