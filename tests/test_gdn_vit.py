@@ -384,3 +384,26 @@ def test_gdn_short_sequences_beside_long_ones(dtype, lens, known):
     eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     torch.testing.assert_close(got.cpu().double(), want, rtol=eps, atol=1e-5)
     torch.testing.assert_close(s_got.cpu().double(), s_want, rtol=1e-5, atol=1e-5)
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,C", [(64, 8192), (65, 8192), (80, 8192), (81, 8192), (160, 4096), (161, 4096), (513, 8192), (1, 8)])
+@pytest.mark.parametrize("K", [2, 4])
+def test_convolution_around_the_choice_of_kernel(dtype, T, C, K):
+    """Steps on either side of where threads take several channels and tokens, sequences of one token and of many, with and without
+    a carry: products of 16-bit numbers summed in fp32 in the order of the taps, one rounding (and the silu's exponential)."""
+    from vllm_metax_b200.ops import gdn
+
+    g = torch.Generator().manual_seed(T)
+    lens = [1] * min(T, 40) + ([T - 40] if T > 40 else [])
+    B = len(lens)
+    x, w = torch.randn(T, C, generator=g).to(dtype), torch.randn(C, K, generator=g).to(dtype)
+    state = torch.randn(B + 1, K - 1, C, generator=g).to(dtype)
+    qsl = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32)
+    idx, has = torch.randperm(B + 1, generator=g)[:B].to(torch.int32), (torch.rand(B, generator=g) < 0.6).to(torch.int32)
+    s1, s2 = state.clone(), state.cuda()
+    want = gdn.causal_conv1d_ref(x, w, None, s1, qsl, idx, has)
+    got = gdn.causal_conv1d(*(t.cuda() for t in (x, w)), None, s2, qsl.cuda(), idx.cuda(), has.cuda())
+    assert torch.equal(s2.cpu(), s1)
+    torch.testing.assert_close(got.cpu(), want, rtol=2.0 ** (-7 if dtype == torch.bfloat16 else -9), atol=1e-3)

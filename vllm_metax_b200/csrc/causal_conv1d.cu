@@ -8,10 +8,12 @@
 // state[slot, K-1, C] (oldest first) and is rewritten by a second kernel once the outputs are done, so a decode step
 // (one token) and a prefill chunk (thousands) go through the same two launches.
 //
-// Forward kernel: a thread takes 8 channels (16 bytes) of up to kTok tokens; their rows and the K-1 before them are read first,
-// all at once; bound by that traffic.  Rows whose channel count, pitch or base does not allow
-// 16-byte reads, and fp32, go through the kernel with a channel per thread.  kTok: 8 where the tokens fill the GPU that way,
-// 4 or 1 for fewer.  3949 tokens, 8192 channels: 144 us with a channel per thread, 61 us with 8.
+// Forward kernel: a thread takes 8 channels (16 bytes) of 4 or, where the tokens fill the GPU that way, 8 tokens; their rows and
+// the K-1 before them are read first, all at once; bound by that traffic.  Rows whose channel count, pitch or base does not allow
+// 16-byte reads, and fp32, go through the kernel with a channel per thread, and so do steps of few tokens: with kVecWork outputs
+// and less there are too few threads of 8 for their reads to be hidden.  us, a channel per thread / 8 channels, both launches:
+// 64 tokens, 8192 channels 14.9 / 15.9; 64, 4096 10.6 / 12.2; 200, 1024 11.2 / 12.5; 200, 4096 16.0 / 14.7; 500, 4096 18.9 / 14.3;
+// 3949, 8192 182 / 64.
 // The channels may be gathered from rows that hold several heads' q, k, v and gates in turn (`map`): the projection of a
 // gated-delta-rule layer is read where it is.
 #include <cuda_bf16.h>
@@ -51,7 +53,7 @@ __device__ __forceinline__ int sequence_of(const int* __restrict__ qsl, int batc
   return lo;
 }
 
-constexpr int kMaxK = 8;
+constexpr int kMaxK = 8, kVecWork = 640 * 1024;
 
 template <typename T>
 __device__ __forceinline__ float ld(const T* p) { return (float)*p; }
@@ -214,14 +216,13 @@ void launch(void* out, const void* x, int64_t x_stride, const void* w, const voi
       (T*)out, (const T*)x, x_stride, (const T*)w, (const T*)bias, (const T*)state, qsl, state_idx, has_init, batch, tokens, \
       channels, silu, map)
 #define CONV_TOK(TAPS)                                                                                             \
-  if (tokens <= 64) CONV_VEC(1, TAPS);                                                                             \
-  else if ((int64_t)tokens * channels <= (1 << 22)) CONV_VEC(4, TAPS);                                             \
+  if ((int64_t)tokens * channels <= (1 << 22)) CONV_VEC(4, TAPS);                                                  \
   else CONV_VEC(8, TAPS)
   bool vec = false;
   if constexpr (sizeof(T) == 2) {
     auto wide = [](const void* at) { return (reinterpret_cast<uintptr_t>(at) & 15) == 0; };
     vec = channels % 8 == 0 && x_stride % 8 == 0 && map.dk % 8 == 0 && map.dv % 8 == 0 && map.group % 8 == 0 && wide(x) &&
-          wide(out) && wide(bias) && wide(state) && K >= 2 && K <= 4;
+          wide(out) && wide(bias) && wide(state) && K >= 2 && K <= 4 && (int64_t)tokens * channels > kVecWork;
     if (vec) {
       if (K == 2) { CONV_TOK(2); }
       else if (K == 3) { CONV_TOK(3); }
