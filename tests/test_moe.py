@@ -289,3 +289,23 @@ def test_gate_behind_a_product_in_a_graph(dtype, T, N, K, kernel_status_ok):
             want = step().clone()
             graph.replay()
             assert torch.equal(out, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,topk,E,N,K,epi", [(255, 2, 4, 256, 128, 0), (256, 2, 4, 256, 128, 1), (257, 2, 4, 1024, 192, 0), (1500, 3, 5, 300, 72, 0),
+                                              (900, 2, 2, 512, 128, 1)])
+def test_grouped_products_of_full_blocks(T, topk, E, N, K, epi):
+    """Around the mean of 128 rows per expert from which whole blocks are read, with experts that get far fewer: padding rows hold NaN
+    and touch nothing, the others equal those of the call that takes every row."""
+    g = torch.Generator().manual_seed(T)
+    ids = torch.stack([torch.multinomial(torch.arange(1, E + 1).float() ** 2, topk, generator=g) for _ in range(T)]).to(torch.int32).cuda()
+    sorted_ids, be, total, inv = ops.moe_align_block_size(ids, 128, E, want_inverse=True)
+    real = sorted_ids < ids.numel()
+    x = torch.randn(T, K, generator=g).bfloat16().cuda()
+    a = ops.moe_scatter(x, inv, sorted_ids, total, topk)
+    a[~real] = float("nan")
+    w = torch.randn(E, N, K, generator=g).bfloat16().cuda()
+    got = ops.gemm_grouped(a, w, be, total, epi, None, sorted_ids, ids.numel())
+    want = ops.gemm_grouped(torch.where(real[:, None], a, torch.zeros_like(a)), w, be, total, epi)
+    assert torch.equal(got[real], want[real]) and bool(torch.isfinite(got[real]).all())
+    ops.check_kernel_status(0)
