@@ -309,3 +309,19 @@ def test_grouped_products_of_full_blocks(T, topk, E, N, K, epi):
     want = ops.gemm_grouped(torch.where(real[:, None], a, torch.zeros_like(a)), w, be, total, epi)
     assert torch.equal(got[real], want[real]) and bool(torch.isfinite(got[real]).all())
     ops.check_kernel_status(0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,topk,hidden", [(4095, 2, 4096), (4096, 2, 4096), (4097, 5, 2056), (5000, 1, 264)])
+def test_combined_rows_of_many_tokens(tokens, topk, hidden):
+    """Around the number of tokens from which a CTA walks its whole row: sums in fp32 in the order of the pairs, rounded once."""
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    y = torch.randn(tokens * topk, hidden, generator=g, device="cuda").bfloat16()
+    w = torch.rand(tokens, topk, generator=g, device="cuda")
+    inv = torch.randperm(tokens * topk, generator=g, device="cuda").to(torch.int32)
+    inv[::11] = -1
+    shared = torch.randn(tokens, hidden, generator=g, device="cuda").bfloat16()
+    acc, iv = shared.float(), inv.view(tokens, topk).long()
+    for k in range(topk):
+        acc = torch.where((iv[:, k] >= 0)[:, None], acc + w[:, k: k + 1] * y[iv[:, k].clamp_min(0)].float(), acc)
+    torch.testing.assert_close(ops.moe_combine(y, w, inv, tokens, shared).float(), acc, rtol=2.0 ** -7, atol=1e-5)

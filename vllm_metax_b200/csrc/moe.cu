@@ -483,42 +483,43 @@ __device__ __forceinline__ const T* combine_row(const T* y, const T* through, co
 }
 
 // out[t] = sum_k w[t,k] * row of pair (t, k)  (+ shared[t]).  CTA (t, j): a 16-byte vector of the row a thread; the places of
-// four pairs and then their rows are read before the sums, so that a thread waits four times and not sixteen for 8 pairs: 64
-// rows of 7168 take 4.5 us where one pair after the other and a CTA per row took 22.  Prompts are bound by the rows' bytes.
-template <typename T>
+// P = four pairs (two, where there are no more) and then their rows are read before the sums, so that a thread waits four times and not sixteen for 8 pairs: 64
+// rows of 7168 take 4.5 us where one pair after the other and a CTA per row took 22.  Prompts are bound by the rows' bytes; from
+// 4096 tokens on a CTA walks its whole row (8192 rows of 4096 from 2 pairs each: 58 us with two CTAs a row, 50 us with one).
+template <typename T, int P>
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(T* __restrict__ out, const T* __restrict__ y, const float* __restrict__ weights,
                    const int* __restrict__ inv_pos, const T* __restrict__ shared, const int* __restrict__ expert_ids,
                    const T* __restrict__ through, int identity_from, int topk, int hidden) {
   const size_t t = blockIdx.x;
-  const int v = blockIdx.y * blockDim.x + threadIdx.x;
-  if (v >= hidden / 8) return;
-  float acc[8];
+  for (int v = blockIdx.y * blockDim.x + threadIdx.x; v < hidden / 8; v += gridDim.y * blockDim.x) {
+    float acc[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-  if (shared) unpack8<T>(reinterpret_cast<const uint4*>(shared + t * hidden)[v], acc);
-  for (int k0 = 0; k0 < topk; k0 += 4) {
-    const T* row[4];
-    uint4 r[4];
-    float w[4];
+    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+    if (shared) unpack8<T>(reinterpret_cast<const uint4*>(shared + t * hidden)[v], acc);
+    for (int k0 = 0; k0 < topk; k0 += P) {
+      const T* row[P];
+      uint4 r[P];
+      float w[P];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      row[k] = k0 + k < topk ? combine_row(y, through, expert_ids, identity_from, inv_pos, t * topk + k0 + k, t, hidden) : nullptr;
-      w[k] = k0 + k < topk ? weights[t * topk + k0 + k] : 0.f;
+      for (int k = 0; k < P; ++k) {
+        row[k] = k0 + k < topk ? combine_row(y, through, expert_ids, identity_from, inv_pos, t * topk + k0 + k, t, hidden) : nullptr;
+        w[k] = k0 + k < topk ? weights[t * topk + k0 + k] : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < P; ++k)
+        if (row[k] != nullptr) r[k] = reinterpret_cast<const uint4*>(row[k])[v];
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        if (row[k] == nullptr) continue;
+        float f[8];
+        unpack8<T>(r[k], f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] += w[k] * f[i];
+      }
     }
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (row[k] != nullptr) r[k] = reinterpret_cast<const uint4*>(row[k])[v];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (row[k] == nullptr) continue;
-      float f[8];
-      unpack8<T>(r[k], f);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] += w[k] * f[i];
-    }
+    reinterpret_cast<uint4*>(out + t * hidden)[v] = pack8<T>(acc);
   }
-  reinterpret_cast<uint4*>(out + t * hidden)[v] = pack8<T>(acc);
 }
 
 // Rows of fp32, or of a width that 16-byte vectors do not divide: one element per thread and trip.
@@ -661,9 +662,12 @@ void moe_combine(void* out, const void* y, const float* weights, const int* inv_
     return;
   }
   const int vecs = hidden / 8, th = vecs < 256 ? (vecs < 32 ? 32 : vecs) : 256;
-  const dim3 grid(tokens, ceil_div(vecs, th));
-  if (dtype == 0) COMBINE(moe_combine_kernel, __nv_bfloat16, grid, th);
-  else COMBINE(moe_combine_kernel, __half, grid, th);
+  const dim3 grid(tokens, tokens < 4096 ? ceil_div(vecs, th) : 1);
+#define COMBINE_ROWS(T, P) moe_combine_kernel<T, P><<<grid, th, 0, stream>>>((T*)out, (const T*)y, weights, inv_pos, (const T*)shared, \
+                                                                            expert_ids, (const T*)through, identity_from, topk, hidden)
+  if (dtype == 0) { if (topk <= 2) COMBINE_ROWS(__nv_bfloat16, 2); else COMBINE_ROWS(__nv_bfloat16, 4); }
+  else { if (topk <= 2) COMBINE_ROWS(__half, 2); else COMBINE_ROWS(__half, 4); }
+#undef COMBINE_ROWS
 #undef COMBINE
 }
 
