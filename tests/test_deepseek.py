@@ -261,37 +261,56 @@ def test_deepseek_graph_under_another_architecture_name_cpu():
 
 
 def test_mla_tcgen05_tiling_arithmetic_cpu():
-    """The index arithmetic of csrc/mla_decode_tcgen05.cu restated: for every visible length, split count and page
-    size the kernel serves, the 32-token tiles of all splits cover the visible positions exactly once, no tile
-    straddles a page, every tile holds at least one visible position, and TMA coordinates stay 16-byte aligned."""
+    """The index arithmetic of csrc/mla_decode_tcgen05.cu restated: for ragged tokens and any number of groups, the groups' ranges
+    cover the 32-token tiles of every token's visible rows exactly once, tokens are not cut where all are short, the groups that the
+    kernel takes for the owners of a token's parts are those that have some, a group leaves at most two parts, no tile straddles a
+    page, and shared and tensor memory suffice."""
+    import math
     import random
 
-    BN = 32
+    BN, SHORT = 32, 4
     rng = random.Random(0)
-    for _ in range(2000):
-        block_size = rng.choice([32, 64, 128, 256])
-        max_blocks = rng.randint(1, 40)
-        lim = min(rng.randint(-3, max_blocks * block_size + 40), max_blocks * block_size)      # the kernel clamps to the table
-        splits = rng.randint(1, 9)
-        tiles_total = (lim + BN - 1) // BN if lim > 0 else 0
-        per = (tiles_total + splits - 1) // splits
-        seen = []
-        for s in range(splits):
-            begin = s * per
-            n = max(0, min(tiles_total, begin + per) - begin)
-            for j in range(n):
-                tok0 = (begin + j) * BN
-                page_index, off = tok0 // block_size, tok0 % block_size
-                assert page_index < max_blocks and off + BN <= block_size          # inside the table, inside one page
-                assert tok0 < lim                                                  # at least one visible position
-                seen.extend(range(tok0, min(tok0 + BN, lim)))
-        assert seen == list(range(max(lim, 0)))
+    for _ in range(400):
+        block_size, max_blocks = rng.choice([32, 64, 128, 256]), rng.randint(1, 40)
+        top = rng.choice([100, 128, 129, 4000])
+        lims = [min(rng.randint(-3, top), max_blocks * block_size) for _ in range(rng.randint(1, 90))]      # clamped to the table
+        T, ctas = len(lims), rng.randint(1, 80)
+        n = [max(1, -(-max(v, 0) // BN)) for v in lims]
+        pre = [0]
+        for x in n:
+            pre.append(pre[-1] + x)
+        units = pre[-1]
+        groups = min(ctas, units, T * max(1, int(math.sqrt(0.5 * units / T))))
+
+        def border(c):
+            at = units * c // groups
+            if max(n) > SHORT or c >= groups:
+                return at
+            t = max(k for k in range(T) if pre[k] <= at)
+            return pre[t] if at - pre[t] <= pre[t + 1] - at else pre[t + 1]
+
+        ends = [border(c) for c in range(groups + 1)]
+        assert ends[0] == 0 and ends[-1] == units and all(a <= b for a, b in zip(ends, ends[1:]))
+        for t in range(T):
+            owners = [c for c in range(groups) if ends[c] < pre[t + 1] and ends[c + 1] > pre[t]]
+            if max(n) <= SHORT:
+                assert len(owners) == 1
+            elif len(owners) > 1:
+                assert owners == list(range((pre[t] * groups + groups - 1) // units, (pre[t + 1] * groups - 1) // units + 1))
+            for j in range(n[t]):
+                page, off = j * BN // block_size, j * BN % block_size
+                assert off + BN <= block_size and (page < max_blocks and j * BN < lims[t] or lims[t] <= 0)
+        for c in range(groups):
+            cut = [t for t in range(T) if max(ends[c], pre[t]) < min(ends[c + 1], pre[t + 1]) and
+                   (ends[c] > pre[t] or ends[c + 1] < pre[t + 1])]
+            assert len(cut) <= 2
     # TMA: innermost coordinate c * 64 elements of 2 bytes = multiples of 128 bytes; boxes of 64 elements = 128 bytes
     assert all((c * 64 * 2) % 16 == 0 for c in range(9)) and (64 * 2) % 16 == 0 and (576 * 2) % 16 == 0
-    # shared memory: Q tile + two cache stages + barriers fit the 227 KB limit with the 1024-byte alignment slack
-    assert 128 * 576 * 2 + 2 * 32 * 576 * 2 + 10 * 8 + 16 + 1024 <= 232448
-    # tensor memory: two score buffers of 32 fp32 columns and 256 output columns fit 512 columns
-    assert 2 * 32 + 256 <= 512
+    # shared memory: three query chunks, four cache stages, barriers and the prefix of 1024 tokens fit the 227 KB limit with the
+    # 1024-byte alignment slack
+    assert 3 * 128 * 128 + 4 * 32 * 576 * 2 + 18 * 8 + 16 + 1025 * 4 + 1024 <= 232448
+    # tensor memory: two score buffers of 32 fp32 columns, 256 output columns and 384 query entries as pairs fill 512 columns
+    assert 2 * 32 + 256 + 384 // 2 == 512
 
 
 @pytest.mark.gpu

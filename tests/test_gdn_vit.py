@@ -407,3 +407,18 @@ def test_convolution_around_the_choice_of_kernel(dtype, T, C, K):
     got = gdn.causal_conv1d(*(t.cuda() for t in (x, w)), None, s2, qsl.cuda(), idx.cuda(), has.cuda())
     assert torch.equal(s2.cpu(), s1)
     torch.testing.assert_close(got.cpu(), want, rtol=2.0 ** (-7 if dtype == torch.bfloat16 else -9), atol=1e-3)
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gdn_of_a_long_prompt(dtype):
+    """2048 tokens of one sequence, where errors of the recurrence would add up: outputs rounded once, and the fp32 state within 1e-5
+    (its entries decay, so that an error of 2^-24 per token does not grow)."""
+    from vllm_metax_b200.ops.gdn import gated_delta_rule
+
+    q, k, v, g, beta, qsl, state, idx, has = _gdn_case(dtype, seed=21, lens=(2048, 1, 700))
+    want, s_want = _gdn_f64(q, k, v, g, beta, (2048, 1, 700), state, idx, has)
+    s_got = state.cuda()
+    got = gated_delta_rule(*(t.cuda() for t in (q, k, v, g, beta, qsl)), s_got, idx.cuda(), has.cuda())
+    torch.testing.assert_close(got.cpu().double(), want, rtol=2.0 ** (-8 if dtype == torch.bfloat16 else -11), atol=1e-5)
+    torch.testing.assert_close(s_got.cpu().double(), s_want, rtol=1e-5, atol=1e-5)

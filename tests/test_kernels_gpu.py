@@ -592,7 +592,7 @@ def test_prefill_of_256_wide_heads(bs, Hq, Hkv, kw, kernel_status_ok):
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M", [1, 2, 3, 4])
-@pytest.mark.parametrize("N,K", [(640, 2048), (6144, 4096), (1001, 1000), (28672, 512), (576, 14336)])
+@pytest.mark.parametrize("N,K", [(640, 2048), (6144, 4096), (1000, 1000), (1008, 1000), (28672, 512), (576, 14336)])
 def test_few_tokens_against_a_weight(dtype, M, N, K, kernel_status_ok):
     """Rows that do not fill a CTA's eight, a contraction that ends inside a warp's piece, bias, residual and gated rows: sums of
     products exact in fp32, rounded once (gated: the two factors first)."""
@@ -603,9 +603,8 @@ def test_few_tokens_against_a_weight(dtype, M, N, K, kernel_status_ok):
     r = torch.randn(M, N, generator=g).to(dtype).cuda()
     eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     want = a.double() @ w.double().T
-    if N % 8 == 0:
-        torch.testing.assert_close(ops.gemm(a, w).double(), want, rtol=eps, atol=1e-5)
-        torch.testing.assert_close(ops.gemm(a, w, bias=b, residual=r).double(), want + b.double() + r.double(), rtol=eps, atol=1e-5)
+    torch.testing.assert_close(ops.gemm(a, w).double(), want, rtol=eps, atol=1e-5)
+    torch.testing.assert_close(ops.gemm(a, w, bias=b, residual=r).double(), want + b.double() + r.double(), rtol=eps, atol=1e-5)
     if N % 16 == 0:
         f = lambda x: x.to(dtype).double()
         gate, up = f(want[:, 0::2]), f(want[:, 1::2])
@@ -703,3 +702,20 @@ def test_narrow_products_around_the_choice_of_kernel(M, N, K):
     want = a.double() @ w.double().T
     torch.testing.assert_close(ops.gemm(a, w).double(), want, rtol=2.0 ** -8, atol=2e-5)
     torch.testing.assert_close(ops.gemm(a, w, bias=b).double(), want + b.double(), rtol=2.0 ** -8, atol=2e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("Hq,Hkv,D,int8", [(32, 8, 128, False), (16, 8, 64, False), (8, 1, 128, False), (4, 4, 256, False), (16, 2, 128, True),
+                                           (24, 2, 128, True)])
+@pytest.mark.parametrize("lens", [[128] * 32, [150, 64, 1, 192] * 20, [192, 193] * 40, [700] * 30 + [650], [3000, 10, 5] * 3, [64] * 300,
+                                  [2000], [1, 4000], [1024, 64, 700, 320, 900, 0, 128, 200]])
+def test_decode_ranges(dtype, Hq, Hkv, D, int8, lens):
+    """The ways in which the CTAs share out the sequences: a part of one each, a whole one each, ranges that end where short
+    sequences do and ranges that end anywhere; both 16-bit types, int8 rows widened to either; a kept scratch is zero again."""
+    q, cache, scales, table, sl, want, bound = _decode_case(Hq, Hkv, D, D, lens, dtype, int8)
+    cd = cache.cuda() if int8 else _decode_views(cache.cuda(), 64, Hkv, D, D)
+    scratch = ops.decode_scratch(Hq, Hkv, D, "cuda")
+    got = [ops.paged_attention_decode(q.cuda(), cd, table.cuda(), sl.cuda(), D ** -0.5, max_seq_len=max(lens), scratch=scratch,
+                                      kv_scales=None if scales is None else scales.cuda()).float().cpu() for _ in range(2)]
+    assert torch.equal(got[0], got[1]) and not bool(scratch[:16384].any())
+    assert bool(((got[0] - want).abs() <= bound).all()), float((got[0] - want).abs().max())

@@ -1,10 +1,9 @@
 """The tcgen05 absorbed-MLA decode kernel (csrc/mla_decode_tcgen05.cu) against the fp32 oracle.
 
-The cases run in a child process: the file sorts last and the kernel is opt-in (``impl=2`` /
-``B200_MLA_TCGEN05=1``), so whatever it does stays outside the process that runs the rest of the suite.  Cases: one and
-two head tiles, fewer heads than a tile, lengths that end inside a tile / a page, several tokens per request, splits
-that own no tile, page sizes 32 and 64, bf16 and fp16, and a score scale at which row maxima keep growing (the
-accumulator rescale path).
+The cases run in a child process, which pins the kernel (``impl=2``).  Cases: one and two head tiles, fewer heads than a
+tile, lengths that end inside a tile / a page, several tokens per request, few tokens that many CTAs share and many that
+they have several of each, page sizes 32 and 64, bf16 and fp16, and a score scale at which row maxima keep growing (the
+accumulator rescale path).  The kernel divides the work itself: a split count makes no difference.
 """
 import json
 import os
@@ -37,8 +36,8 @@ def _mla_case(lens, qlens, H, bs, dtype, seed=0):
     return q, cache, bt, torch.tensor(lens, dtype=torch.int32), qsl
 
 
-CASES = [(H, splits, bs, scale, dt)
-         for H in (128, 16, 200) for splits in (1, 3)
+CASES = [(H, copies, bs, scale, dt)
+         for H in (128, 16, 200) for copies in (1, 12)
          for bs, scale, dt in ((64, 0.1, "bfloat16"), (32, 1.5, "bfloat16"), (64, 0.1, "float16"))]
 
 
@@ -48,17 +47,19 @@ def _child() -> None:
 
     ops.load_native()
     out = []
-    for H, splits, bs, scale, dt in CASES:
+    for H, copies, bs, scale, dt in CASES:
         dtype = getattr(torch, dt)
-        q, cache, bt, sl, qsl = _mla_case([70, 300, 17, 1000, 33], [1, 3, 1, 2, 1], H, bs, dtype, seed=5)
+        q, cache, bt, sl, qsl = _mla_case([70, 300, 17, 1000, 33] * copies, [1, 3, 1, 2, 1] * copies, H, bs, dtype, seed=5)
         lse = torch.empty(H, q.shape[0], device="cuda")
         got = ops.mla_decode(q.cuda(), cache.cuda(), bt.cuda(), sl.cuda(), scale, query_start_loc=qsl.cuda(),
-                             lse_out=lse, num_splits=splits, impl=2)
+                             lse_out=lse, impl=2)
+        again = ops.mla_decode(q.cuda(), cache.cuda(), bt.cuda(), sl.cuda(), scale, query_start_loc=qsl.cuda(), num_splits=3, impl=2)
         torch.cuda.synchronize()
+        assert torch.equal(again, got)
         want, wlse = ref.mla_decode(q.float(), cache.float(), bt, sl, scale, query_start_loc=qsl)
         a, b = got.float().cpu().flatten(), want.flatten()
         cos = 1 - float(torch.dot(a, b) / (a.norm() * b.norm()))
-        out.append({"case": [H, splits, bs, scale, dt], "finite": bool(torch.isfinite(a).all()), "cos_diff": cos,
+        out.append({"case": [H, copies, bs, scale, dt], "finite": bool(torch.isfinite(a).all()), "cos_diff": cos,
                     "lse_max_diff": float((lse.cpu() - wlse).abs().max())})
     print("RESULT " + json.dumps({"cases": out, "status": ops.kernel_status()}))
 

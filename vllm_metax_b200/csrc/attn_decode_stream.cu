@@ -1,7 +1,8 @@
 // Paged GQA decode attention, one token per sequence, with the KV stream shared out evenly whatever the lengths are.
 //
-// The sequences' tokens, in units of 64, form one list; the CTAs of a key head (as many as fit on the GPU at once) take equal
-// contiguous ranges of it, and neighbouring CTAs the same range of neighbouring heads, whose rows lie side by side in a page.  A
+// The sequences' tokens, in units of 64, form one list, with two units more for the end of each (without these, a step's many short
+// rows, such as those that pad a captured one, came to one CTA); the CTAs of a key head (as many as fit on the GPU at once) take
+// equal contiguous ranges of it, and neighbouring CTAs the same range of neighbouring heads, whose rows lie side by side in a page.  A
 // range may end inside a sequence: such a part leaves its state (sums, maximum, denominator) in a slot, and the CTA that arrives
 // last at the sequence adds the parts up when it is through with its range, all its warps at once.  Nobody waits.  A CTA copies
 // without a break from its first unit to its last: the ring of tiles runs on over the ends of sequences, the page of a tile is
@@ -16,13 +17,16 @@
 // on - and value columns likewise (lane g the 16 bytes from 16 g on), so fragments are 16-byte loads and byte permutations; the
 // integers are exact in either 16-bit type.
 //
-// What bounds it: the KV bytes.  One CTA per (sequence, head) and tiles converted through shared memory / now, us:
+// What bounds it: the KV bytes; with few or ragged rows the ends of ranges and of sequences.  One CTA per (sequence, head) and
+// tiles converted through shared memory / now, us:
 //   256 rows of 1088 tokens, 32 heads over 8, bf16      234 / 190   (its bytes at copy bandwidth: 177)
 //   16 rows, 64 heads over 8, int8                       472 / 208   (91)
 //   64 rows, 32 heads over 4, bf16                        51 / 35
 //   64 rows of 2 key heads of 256, bf16                   81 / 56
-//   40 rows of 42 thousand tokens in all, 32 over 8       50 / 55     (27; ends of ranges and of sequences count)
-//   1 row                                                 10 / 11
+//   40 rows of 42 thousand tokens in all and 8 that pad, 32 over 8   54 / 47   (58 before ends counted in the ranges)
+//   100 rows of 37 thousand tokens and 12 that pad        58 / 49   (65)
+//   1 row of 900                                          13 / 13
+//   32 rows of 128, 32 over 8                             12 / 17   (a sequence's parts; such steps are where it loses)
 // Covers the same calls as attn_decode.cu (see there for the reference's).
 #include <type_traits>
 #include "attn_decode.cuh"
@@ -34,6 +38,7 @@ namespace b200 {
 namespace {
 
 constexpr int kWarps = 4, kThreads = 128, kTile = 16, kStages = 3, kMaxBatch = 1024, kMaxSmem = 227 * 1024;
+constexpr int kEnd = 2;                                                   // what a sequence's end costs a CTA, in units
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 
 template <int D, int KIND, int ROWS>
@@ -92,14 +97,14 @@ paged_decode_stream_kernel(const DecodeParams p, int batch, float* parts, int* c
     tile_lo = first_key(kv_len, p.window, p.chunk) / kTile;
     return max(1, ((kv_len + kTile - 1) / kTile - tile_lo + kWarps - 1) / kWarps);
   };
-  // ---- units in front of every sequence
+  // ---- what is in front of every sequence: units, and kEnd for the end of each
   {
     const int per = (batch + kThreads - 1) / kThreads;
     int sum = 0, x, y;
     for (int i = 0; i < per; ++i) {
       const int b = tid * per + i;
       if (b >= batch) break;
-      const int n = extent(b, x, y);
+      const int n = extent(b, x, y) + kEnd;
       s_pre[b + 1] = n;
       sum += n;
     }
@@ -122,17 +127,27 @@ paged_decode_stream_kernel(const DecodeParams p, int batch, float* parts, int* c
     if (tid == 0) s_pre[0] = 0;
     __syncthreads();
   }
-  const long long units = s_pre[batch];
+  const long long space = s_pre[batch];
   // every range holds a unit; and a sequence's parts, which one CTA adds up, are no more than pays beside its units
+  const long long units = space - (long long)kEnd * batch;
   const int groups = (int)min(min((long long)(gridDim.x / p.num_kv_heads), units),
                               (long long)batch * max(1, (int)sqrtf(4.f * (float)units / (float)batch)));
   if (grp >= groups) return;
-  const int u0 = (int)(units * grp / groups), u1 = (int)(units * (grp + 1) / groups);
-  int b = 0;
-  for (int hi = batch - 1; b < hi;) {                                     // the last sequence that starts at or before u0
-    const int mid = (b + hi + 1) >> 1;
-    if (s_pre[mid] <= u0) b = mid; else hi = mid - 1;
-  }
+  // where range c begins: a unit of sequence `seq`, in units and ends from the first one on
+  auto border = [&](int c, int& seq) -> int {
+    const int at = (int)(space * c / groups);
+    int lo = 0;
+    for (int hi = batch; lo < hi;) {                                      // the last sequence that starts at or before `at`
+      const int mid = (lo + hi + 1) >> 1;
+      if (s_pre[mid] <= at) lo = mid; else hi = mid - 1;
+    }
+    seq = lo;
+    if (lo == batch || at < s_pre[lo + 1] - kEnd) return at;
+    return s_pre[seq = lo + 1];                                           // (within its end: the next one)
+  };
+  int b, b_end;
+  const int u0 = border(grp, b), u1 = border(grp + 1, b_end);
+  if (u0 >= u1) return;
 
   uint8_t* ring = smem + S::kRing + warp * kStages * S::kStage;
   // queries of sequence `seq` into buffer `qb`: 16-byte chunks, swizzled for ldmatrix (16-bit caches) or as they are
@@ -147,7 +162,7 @@ paged_decode_stream_kernel(const DecodeParams p, int batch, float* parts, int* c
   };
 
   // ---- what is copied next: tile `warp` of unit iu of sequence ib
-  int ib = b, iu = u0 - s_pre[b], in, ilen, itile_lo, ileft = u1 - u0, ipage = -1;
+  int ib = b, iu = u0 - s_pre[b], in, ilen, itile_lo, ileft = u1 - u0 - kEnd * (b_end - b), ipage = -1;
   in = extent(ib, ilen, itile_lo);
   auto look_up = [&]() {
     const int tok0 = (itile_lo + iu * kWarps + warp) * kTile;
@@ -318,8 +333,8 @@ paged_decode_stream_kernel(const DecodeParams p, int batch, float* parts, int* c
   };
   // the CTAs that hold a sequence's units, and where a CTA leaves its part of one: a range that starts inside the sequence, or not
   auto sharers = [&](int seq, int& c0, int& c1) {
-    c0 = (int)(((long long)s_pre[seq] * groups + groups - 1) / units);
-    c1 = (int)(((long long)s_pre[seq + 1] * groups - 1) / units);
+    c0 = (int)(((long long)s_pre[seq] * groups + groups - 1) / space);
+    c1 = (int)(((long long)(s_pre[seq + 1] - kEnd) * groups - 1) / space);
   };
   constexpr int kSlot = S::kState / 4;
   auto slot = [&](int c, bool tail) { return parts + (((int64_t)c * p.num_kv_heads + hk) * 2 + (tail ? 0 : 1)) * kSlot; };
@@ -337,7 +352,7 @@ paged_decode_stream_kernel(const DecodeParams p, int batch, float* parts, int* c
     // ---- one sequence's share of this CTA: units u .. seg_end
     int kv_len, tile_lo;
     extent(b, kv_len, tile_lo);
-    const int first = s_pre[b], behind = s_pre[b + 1], seg_end = min(u1, behind), seg0 = u;
+    const int first = s_pre[b], behind = s_pre[b + 1] - kEnd, seg_end = min(u1, behind), seg0 = u;
     const int lo_pos = first_key(kv_len, p.window, p.chunk);
     clear();
     uint32_t qf[D / 16][4];
@@ -358,7 +373,7 @@ paged_decode_stream_kernel(const DecodeParams p, int batch, float* parts, int* c
     }
     for (; u < seg_end; ++u) {
       issue((stage + kStages - 1) % kStages);
-      if (u == seg0 && seg_end < u1) copy_q(b + 1, qb ^ 1);
+      if (u == seg0 && seg_end + kEnd < u1) copy_q(b + 1, qb ^ 1);
       cp_async_commit();
       cp_async_wait<kStages - 1>();
       __syncwarp();
@@ -497,6 +512,7 @@ paged_decode_stream_kernel(const DecodeParams p, int batch, float* parts, int* c
         reinterpret_cast<float4*>(mine)[i] = reinterpret_cast<const float4*>(merge[0])[i];
       if (tail) left0 = b; else left1 = b;
     }
+    if (u == behind) u += kEnd;
     ++b;
     qb ^= 1;
   }
@@ -521,7 +537,7 @@ paged_decode_stream_kernel(const DecodeParams p, int batch, float* parts, int* c
     __threadfence();
     int c0, c1;
     sharers(seq, c0, c1);
-    write(seq, c1 - c0 + 1, slot(c0 + 1, true), (int64_t)p.num_kv_heads * 2 * kSlot, slot(c0, units * c0 / groups > s_pre[seq]));
+    write(seq, c1 - c0 + 1, slot(c0 + 1, true), (int64_t)p.num_kv_heads * 2 * kSlot, slot(c0, space * c0 / groups > s_pre[seq]));
   }
 }
 
@@ -568,9 +584,14 @@ cudaError_t dispatch(const DecodeParams& p, int kind, int batch, int sms, float*
 }  // namespace
 
 // Whether the kernel serves a step of `batch` sequences of one token each.  16 rows of heads wider than 128 would take 240 KB of
-// shared memory, of which a CTA may have 227: these stay in attn_decode.cu.
-bool decode_stream_serves(const DecodeParams& p, int kv_kind, int batch) {
-  const int head = p.dqk > p.dv ? p.dqk : p.dv;
+// shared memory, of which a CTA may have 227: these stay in attn_decode.cu.  So do most other steps with more than 8 heads per key
+// head, which need that kernel's 16 rows anyway: its CTAs, cut into splits for few sequences, fall behind only where they leave an
+// uneven last wave, and for int8 rows also when there are many.  us there / here, even rows: 48 heads over 4, 16 rows of 1024 29 /
+// 25, 64 rows 39 / 54; int8, 32 heads over 2: 8 rows of 4096 26 / 30, 64 rows 132 / 80, 128 rows of 1024 53 / 56, 256 rows 103 / 86.
+bool decode_stream_serves(const DecodeParams& p, int kv_kind, int batch, int sms) {
+  const int head = p.dqk > p.dv ? p.dqk : p.dv, ctas = batch * p.num_kv_heads;
+  if (p.num_q_heads > 8 * p.num_kv_heads && (ctas < 64 || (kv_kind == 0 ? head <= 64 || ctas >= sms : ctas >= sms && ctas < 2 * sms)))
+    return false;
   if (batch <= 0 || batch > kMaxBatch || p.num_q_heads > 16 * p.num_kv_heads || batch * p.num_kv_heads > kDecodeCounters ||
       p.block_size % kTile != 0 || smem_of(p.num_q_heads / p.num_kv_heads, head, kv_kind, batch) > kMaxSmem)
     return false;

@@ -74,10 +74,8 @@ void paged_attention_decode(Tensor& out, const Tensor& q, const Tensor& k_cache,
   if (kind == 0)
     TORCH_CHECK(k_cache.scalar_type() == q.scalar_type() && pv.page_stride % 8 == 0 && q.stride(0) % 8 == 0 && aligned(q) &&
                 aligned(k_cache) && aligned(v_cache), "paged attention: rows must start on 16 bytes");
-  if (stream && !query_start_loc.has_value() && max_q_len == 1 && batch == T && b200::decode_stream_serves(p, kind, (int)batch)) {
-    static int sms_of[64] = {};
-    int& sms = sms_of[q.get_device() & 63];
-    if (sms == 0) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, q.get_device());
+  const int sms = device_sms(q);
+  if (stream && !query_start_loc.has_value() && max_q_len == 1 && batch == T && b200::decode_stream_serves(p, kind, (int)batch, sms)) {
     int64_t floats = 0;
     b200::decode_stream_scratch(p, kind, dtype16(q), (int)batch, sms, &floats);
     // the caller's, zero in front, or one of this call alone

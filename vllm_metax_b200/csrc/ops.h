@@ -177,7 +177,7 @@ void act_and_mul_quant(void* out_q, float* scale_out, const float* scale_in, con
                        float p0, float p1, int group, int ue8m0, const int* sorted_ids, int numel, int dtype,
                        cudaStream_t stream);
 // ---- attention
-bool decode_stream_serves(const DecodeParams& p, int kv_kind, int batch);
+bool decode_stream_serves(const DecodeParams& p, int kv_kind, int batch, int sms);
 void decode_stream_scratch(const DecodeParams& p, int kv_kind, int dtype, int batch, int sms, int64_t* floats);
 cudaError_t decode_stream(const DecodeParams& p, int kv_kind, int dtype, int batch, int sms, float* parts, int* counters, bool early,
                           cudaStream_t stream);
