@@ -5,7 +5,8 @@
 //   S  <- S + k_t u^T
 //   o_t = S^T (scale * q_t)
 //
-// bf16 prompts go by chunks of 16 tokens on the tensor cores (further down); decode rows and other short sequences a token at a
+// bf16 prompts go by chunks of 16 tokens on the tensor cores (further down, the chunked form of Yang et al., "Gated Delta
+// Networks: Improving Mamba2 with Delta Rule", 2024); decode rows and other short sequences a token at a
 // time (gdn_step_kernel), and so does everything where results must not depend on what else is in a step or on where a prompt is cut;
 // fp16 prompts by groups of G = 4 on the fp32 units, as follows.  With S as it is before the group, G_t the sum of g over the group's
 // tokens up to t and D_tj = exp(G_t - G_j) (never above 1):

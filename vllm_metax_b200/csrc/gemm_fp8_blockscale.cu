@@ -19,8 +19,8 @@
 // Grouped mode: A is the expert-sorted padded activation matrix, W [E, N, K], w_scale
 // [E, N/128, K/128]; block_expert / total_padded as in gemm_grouped_tcgen05.cu.  With `sorted_ids`, rows of padding (at a block's
 // end) are neither read, folded nor written: with a handful of rows per expert they are most of a block.
-// us with 128 threads folding whole tiles of 128 x 128 / now: 64 x 2112 x 7168 26.8 / 12, 64 x 7168 x 16384 56.8 / 28,
-// 1836 x 36864 x 7168 794 / 560, 64 experts 4096 x 7168 for 64 x 8 rows 389 / 300, for 1836 x 8 rows 804 / 680.
+// us with 128 threads folding whole tiles of 128 x 128 / now, in a replayed graph: 64 x 2112 x 7168 28.9 / 24.8, 64 x 7168 x 16384
+// 61.5 / 41, 2048 x 36864 x 7168 907 / 606; 64 experts 4096 x 7168 for 64 x 8 rows 389 / 300, for 1836 x 8 rows 804 / 680.
 // Replaces cutlass_fp8_block_scaled_mm / deep_gemm fp8 grouped GEMMs
 // (vllm_metax/model_executor/layers/quantization/_cutlass_ops.py:23-38,
 // experts/batched_deep_gemm_moe.py:299-326).

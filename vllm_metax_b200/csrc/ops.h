@@ -575,9 +575,7 @@ int tq_decode(void* out, float* part_out, float* part_lse, const void* q, int64_
 // ---- comm_allreduce.cu
 int custom_allreduce(const CustomArParams& p, const void* in, void* out, int dtype, int mode, cudaStream_t stream);
 int reduce_rms(const ReduceRmsParams& p, int dtype, cudaStream_t stream);
-// ---- mla_decode.cu
-// impl: 0 = choose (tcgen05 kernel for dense 16-bit caches from 64 heads per rank up), 1 = mma.sync kernel,
-// 2 = tcgen05 kernel or fail.  Returns 0, or -1 when impl 2 was asked for and that kernel does not serve the call.
+// ---- mla_decode.cu (mma.sync).  Returns 0, or -1 for sizes that it does not serve.
 int mla_decode(const MlaDecodeParams& p, int fp8_records, int dtype, cudaStream_t stream);
 // ---- mla_decode_tcgen05.cu
 bool mla_decode_tc_serves(const MlaDecodeParams& p);

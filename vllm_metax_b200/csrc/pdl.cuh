@@ -10,7 +10,6 @@
 // pdl_trigger() lets the next kernel start as soon as every CTA of this one has got that far; it says nothing about results, for
 // which the next one waits.  Without a dependent launch both do nothing.
 #pragma once
-#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -18,11 +17,6 @@ namespace b200 {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-// A tile of a 2-D map into L2.
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
-}
 
 // Whether a launch into this stream may carry the attribute: it is being captured, and the one node in front is a kernel.
 inline bool pdl_allowed(cudaStream_t stream) {
